@@ -27,6 +27,7 @@
 #include "internal.h"
 
 int sw_init_tables();
+int surf_init_tables();
 
 namespace {
 
@@ -467,7 +468,7 @@ extern "C" int ima_gpu_create(int device, ima_ctx **out)
   cudaEventCreate(&c->t1);
   cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&c->pageable_access, cudaDevAttrPageableMemoryAccess, device);
-  if (sw_init_tables() != 0 || hky_init_tables() != 0) {
+  if (sw_init_tables() != 0 || hky_init_tables() != 0 || surf_init_tables() != 0) {
     delete c;
     return IMA_ERR_CUDA;
   }

@@ -233,11 +233,15 @@ __device__ void refine_loop(const SurfPrep &S, TcSmem &sh, int *gerr, int r, int
 // stride > 0: max-only pass over genealogy tiles 0, stride, 2 stride, ...
 // that only raises the per-point lower bounds S.best (no candidates, no
 // partials); stride == 0: the full pass over every tile, which reads S.best
-// and leaves it unchanged.
+// and leaves it unchanged.  dense, sparse (may be null: every point): the
+// full pass leaves the points with dense[p] = 1 to k_surf_dense, and skips
+// the tiles without others (sparse[tile] = 0).
 __global__ void __launch_bounds__(TC_THREADS, 1)
-    k_surf_tc(SurfPrep S, int npoints, int tiles_per_chunk, int stride, double2 *part, int *gerr)
+    k_surf_tc(SurfPrep S, int npoints, int tiles_per_chunk, int stride, const uint8_t *dense, const int *sparse,
+              double2 *part, int *gerr)
 {
   extern __shared__ __align__(1024) char smem[];
+  if (sparse && sparse[blockIdx.x] == 0) return;
   char *bufA = smem;
   char *bufB = smem + A_BYTES;
   TcSmem &sh = *reinterpret_cast<TcSmem *>(smem + A_BYTES + TC_STAGES * B_BYTES);
@@ -348,7 +352,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int cg = ew >> 2;             // genealogy columns [GROUP_COLS cg, +GROUP_COLS)
     const int pl = q * 32 + lane;       // point within the tile = TMEM lane
     const int p = ptile * TC_M + pl;
-    const bool live = p < npoints;
+    const bool live = p < npoints && !(dense && dense[p]);
     const float err = live ? BF16_SCREEN_ERR * S.mag[p] : 0.f;  // screen error bound
     const float off = err + SURF_MARGIN;
     // lb: a lower bound on the point's maximum -- the pre-pass bound raised
@@ -438,9 +442,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   }
   if (threadIdx.x < TC_M && !maxonly) {
     const int p = ptile * TC_M + threadIdx.x;
-    if (p < npoints) atomicMax(&S.xmax[p], sh.xmax[threadIdx.x]);
-    if (p < npoints)
-      part[(size_t)p * gridDim.y + blockIdx.y] =
+    const bool mine = p < npoints && !(dense && dense[p]);
+    if (mine) atomicMax(&S.xmax[p], sh.xmax[threadIdx.x]);
+    if (mine)
+      part[(size_t)p * SURF_MAX_CHUNKS + blockIdx.y] =
           make_double2(sh.ovf[threadIdx.x] ? -1.0 : fixw_to_double(sh.sum[threadIdx.x]),
                        fixw_to_double(sh.sum2[threadIdx.x]));
   }
@@ -450,11 +455,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 // a flagged chunk goes to the list of points to take again (flag[0] = list
 // length, flag[1..] = points; the list's order does not matter, each point
 // is taken on its own).
-__global__ void k_surf_tc_merge(SurfArgs a, SurfPrep S, const double2 *part, int nchunks, int *flag)
+__global__ void k_surf_tc_merge(SurfArgs a, SurfPrep S, const double2 *part, int nchunks, const uint8_t *dense,
+                                const int *counts, int dense_blocks, int *flag)
 {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= a.npoints) return;
-  const double2 *w = part + (size_t)p * nchunks;
+  const double2 *w = part + (size_t)p * SURF_MAX_CHUNKS;
+  int per;
+  if (dense && dense[p]) nchunks = surf_dense_chunks(counts[0], dense_blocks, a.G, &per);
   double s = 0.0, s2 = 0.0;
   int ovf = 0;
   for (int c = 0; c < nchunks; c++) {
@@ -600,10 +608,12 @@ size_t surface_tc_scratch_bytes(int G, int npoints)
 {
   // prepared operands | chunk sums (double2 per point and chunk) | the list
   // of points to retake (a count, then points) | their coordinates,
-  // references, densities, sample sizes and the retake's own list
+  // references, densities, sample sizes and the retake's own list | how each
+  // point is taken (SurfSplit: counts, list, flags)
   const size_t np = (size_t)npoints;
   return surf_prep_bytes(G, npoints) + np * SURF_MAX_CHUNKS * sizeof(double2) + 2 * (np + 1) * sizeof(int) +
-         np * (SURF_K / 2) * sizeof(double) + np * sizeof(unsigned) + 2 * np * sizeof(double) + 4096;
+         np * (SURF_K / 2) * sizeof(double) + np * sizeof(unsigned) + 2 * np * sizeof(double) +
+         (1 + np / TC_M + 1 + np) * sizeof(int) + np + 4096;
 }
 
 namespace {
@@ -640,22 +650,37 @@ int surf_tc_chunks(int ptiles, int ntiles, int nsm, int *per)
 }  // namespace
 
 // One evaluation of the points of `a` on prepared operands S: the optional
-// max-only pre-pass, the full pass and the merge; returns the kernels queued.
-static int tc_passes(const SurfArgs &a, const SurfPrep &S, double2 *part, int *flag, int *d_err, int nsm, bool pre,
-                     cudaStream_t st)
+// max-only pre-pass, the choice between the screen and the direct form per
+// point (D null: the screen for all), the full pass, the direct form and the
+// merge; returns the kernels queued.
+static int tc_passes(const SurfArgs &a, const SurfPrep &S, const SurfSplit *D, double2 *part, int *flag, int *d_err,
+                     int nsm, bool pre, cudaStream_t st)
 {
   const int ntiles = S.Gpad / TC_N;
   const int ptiles = (a.npoints + TC_M - 1) / TC_M;
   int per = 0, nk = 0;
   if (pre) {
     const int nch = surf_tc_chunks(ptiles, (ntiles + PRE_STRIDE - 1) / PRE_STRIDE, nsm, &per);
-    k_surf_tc<<<dim3(ptiles, nch), TC_THREADS, TC_SMEM, st>>>(S, a.npoints, per, PRE_STRIDE, part, d_err);
+    k_surf_tc<<<dim3(ptiles, nch), TC_THREADS, TC_SMEM, st>>>(S, a.npoints, per, PRE_STRIDE, nullptr, nullptr, part,
+                                                              d_err);
     nk++;
   }
+  const uint8_t *dense = nullptr;
+  const int *counts = nullptr;
+  int db = 0;
+  if (D) {
+    dense = D->dense;
+    counts = D->counts;
+    db = surf_dense_grid(a, nsm);
+    surf_split(S, a.npoints, *D, st);
+    surf_dense(a, S, *D, db, part, st);
+    nk += 2;
+  }
   const int nchunks = surf_tc_chunks(ptiles, ntiles, nsm, &per);
-  k_surf_tc<<<dim3(ptiles, nchunks), TC_THREADS, TC_SMEM, st>>>(S, a.npoints, per, 0, part, d_err);
+  k_surf_tc<<<dim3(ptiles, nchunks), TC_THREADS, TC_SMEM, st>>>(S, a.npoints, per, 0, dense,
+                                                                counts ? counts + 1 : nullptr, part, d_err);
   cudaMemsetAsync(flag, 0, sizeof(int), st);
-  k_surf_tc_merge<<<(a.npoints + 127) / 128, 128, 0, st>>>(a, S, part, nchunks, flag);
+  k_surf_tc_merge<<<(a.npoints + 127) / 128, 128, 0, st>>>(a, S, part, nchunks, dense, counts, db, flag);
   return nk + 2;
 }
 
@@ -678,6 +703,10 @@ int launch_surface_tc(const SurfArgs &a, void *scratch, size_t scratch_bytes, in
   double *qs = reinterpret_cast<double *>((reinterpret_cast<uintptr_t>(refs + np) + 255) & ~static_cast<uintptr_t>(255));
   double *es = qs + np;
   int *flag2 = reinterpret_cast<int *>(es + np);  // the retake's own list (always empty)
+  SurfSplit D;
+  D.counts = flag2 + np + 1;
+  D.list = D.counts + 2 + np / TC_M;
+  D.dense = reinterpret_cast<uint8_t *>(D.list + np);
   static_assert(A_BYTES + TC_STAGES * B_BYTES + sizeof(TcSmem) + 1024 <= TC_SMEM, "smem");
   cudaFuncSetAttribute(k_surf_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
   int nsm = 152;
@@ -691,7 +720,7 @@ int launch_surface_tc(const SurfArgs &a, void *scratch, size_t scratch_bytes, in
   // a max-only pre-pass over every PRE_STRIDE-th tile gives every point a
   // lower bound at (or near) its screened maximum before the full pass
   const bool pre = S.Gpad / TC_N >= 4 * PRE_STRIDE;
-  int nk = (rows_ready ? 0 : 1) + 2 + tc_passes(a, S, part, flag, d_err, nsm, pre, st);
+  int nk = (rows_ready ? 0 : 1) + 2 + tc_passes(a, S, &D, part, flag, d_err, nsm, pre, st);
   // points whose terms left the fixed-point range: a second evaluation of
   // just them, referenced to their exact maxima
   int nflag = 0;
@@ -710,7 +739,7 @@ int launch_surface_tc(const SurfArgs &a, void *scratch, size_t scratch_bytes, in
     double2 *part2 = reinterpret_cast<double2 *>(surf_prep_carve(&S2, base, a.G, nflag));
     surf_prep(b, S2, true, true, st);
     k_surf_tc_setref<<<(nflag + 127) / 128, 128, 0, st>>>(S2.best, S2.xmax, refs, nflag);
-    nk += 3 + tc_passes(b, S2, part2, flag2, d_err, nsm, false, st);
+    nk += 3 + tc_passes(b, S2, nullptr, part2, flag2, d_err, nsm, false, st);
     k_surf_tc_scatter<<<(nflag + 127) / 128, 128, 0, st>>>(flag, qs, es, a.q, a.ess);
     nk++;
   }

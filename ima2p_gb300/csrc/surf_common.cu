@@ -47,6 +47,11 @@ __global__ void k_prep_rows(SurfArgs a, SurfPrep S)
     }
     col[K] = (float)bias;
   }
+  // the genealogies floor(i G / n), i < n
+  const int n = min(SURF_SAMPLES, a.G);
+  const int i = (int)(((long long)g * n + a.G - 1) / a.G);
+  if (g < a.G && i < n && (int)((long long)i * a.G / n) == g)
+    for (int k = 0; k < SURF_KP; k++) S.samp[i * SURF_KP + k] = col[k];
   // the grid covers Gpad (a multiple of 256) exactly, so every warp is full
   const unsigned lane = threadIdx.x & 31;
   for (int k = 0; k < SURF_KP; k++) {
@@ -147,6 +152,7 @@ size_t surf_prep_bytes(int G, int npoints)
   b += align256(sizeof(unsigned) * npad);
   b += align256(sizeof(unsigned) * SURF_KP);
   b += align256(2 * sizeof(uint16_t) * SURF_KP * Gpad);
+  b += align256(sizeof(float) * SURF_KP * SURF_SAMPLES);
   b += align256(2 * sizeof(uint16_t) * SURF_KP * npad);
   return b;
 }
@@ -169,6 +175,7 @@ SurfPart *surf_prep_carve(SurfPrep *S, char *base, int G, int npoints)
   S->biasff = reinterpret_cast<float2 *>(take(sizeof(float2) * Gpad));
   S->colmax = reinterpret_cast<unsigned *>(take(sizeof(unsigned) * SURF_KP));
   S->sbf = reinterpret_cast<uint16_t *>(take(2 * sizeof(uint16_t) * SURF_KP * Gpad));
+  S->samp = reinterpret_cast<float *>(take(sizeof(float) * SURF_KP * SURF_SAMPLES));
   S->phiff = reinterpret_cast<float2 *>(take(sizeof(float2) * SURF_K * npad));
   S->phi32 = reinterpret_cast<float *>(take(sizeof(float) * SURF_KP * npad));
   S->mag = reinterpret_cast<float *>(take(sizeof(float) * npad));

@@ -13,12 +13,15 @@ constexpr int SURF_KP = 32;         // screened columns: the terms, the bias, ze
 constexpr int SURF_MAX_CHUNKS = 64;
 constexpr float SURF_MARGIN = 32.0f;  // nats below the running max that still count
 constexpr int SURF_SEED = 256;      // genealogies sampled per point for the seed maximum (FP32 screen)
+constexpr int SURF_SAMPLES = 256;   // evenly spaced genealogies whose terms decide how a point is taken
+constexpr int SURF_DENSE_TILE = 64; // genealogies per tile of the direct form
 constexpr int SURF_TC_M = 128;      // tensor-core screen: points per A tile
 constexpr int SURF_TC_N = 256;      // tensor-core screen: genealogies per B tile
 
 // Operands prepared once per evaluation (model type and points fixed).
 struct SurfPrep {
   int G, Gpad, K, np, nm;
+  float *samp;      // [SURF_SAMPLES][SURF_KP] columns of the sampled genealogies
   float *sT;        // [SURF_KP][Gpad] statistics (exact floats), column K = bias (rounded)
   float2 *biasff;   // [Gpad] bias as float-float
   float2 *phiff;    // [npoints][SURF_K] phi as float-float
@@ -158,3 +161,29 @@ SurfPart *surf_prep_carve(SurfPrep *S, char *base, int G, int npoints);
 void surf_prep(const SurfArgs &a, SurfPrep &S, bool bf16, bool rows_ready, cudaStream_t st);
 void surf_merge(const SurfArgs &a, const SurfPart *part, int nchunks, cudaStream_t st);
 void surf_seed(const SurfPrep &S, int npoints, int samples, cudaStream_t st);
+
+// How the points of an evaluation are taken (k_surf_dense.cu): dense[p] = 1
+// where every term is evaluated directly, the list of those points,
+// counts[0] = their number and counts[1 + t] = points of tensor-core tile t
+// left to the screen.
+struct SurfSplit {
+  uint8_t *dense;
+  int *list, *counts;
+};
+int surf_init_tables();
+void surf_split(const SurfPrep &S, int npoints, const SurfSplit &D, cudaStream_t st);
+int surf_dense_grid(const SurfArgs &a, int nsm);
+// the chunking of nd dense points over a grid of nb CTAs: about three equal
+// rounds of (32 points, chunk) units, at most SURF_MAX_CHUNKS chunks of whole
+// tiles; the merge recomputes it from the same two numbers
+__host__ __device__ inline int surf_dense_chunks(int nd, int nb, int G, int *per)
+{
+  const int ntiles = (G + SURF_DENSE_TILE - 1) / SURF_DENSE_TILE;
+  const int groups = (nd + 31) / 32;
+  int n = groups > 0 ? 3 * nb / groups : 1;
+  const int lim = ntiles < SURF_MAX_CHUNKS ? ntiles : SURF_MAX_CHUNKS;
+  n = n < 1 ? 1 : n > lim ? lim : n;
+  *per = (ntiles + n - 1) / n;
+  return (ntiles + *per - 1) / *per;
+}
+void surf_dense(const SurfArgs &a, const SurfPrep &S, const SurfSplit &D, int nb, double2 *part, cudaStream_t st);

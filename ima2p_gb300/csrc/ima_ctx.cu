@@ -468,7 +468,8 @@ extern "C" int ima_gpu_create(int device, ima_ctx **out)
   cudaEventCreate(&c->t1);
   cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&c->pageable_access, cudaDevAttrPageableMemoryAccess, device);
-  if (sw_init_tables() != 0 || hky_init_tables() != 0 || surf_init_tables() != 0) {
+  if (sw_init_tables() != 0 || hky_init_tables() != 0 || surf_init_tables() != 0 ||
+      margin_init_tables() != 0) {
     delete c;
     return IMA_ERR_CUDA;
   }
@@ -2450,7 +2451,32 @@ static int margin_run(ima_ctx *c, int n, const int32_t *param, const double *x, 
   if (expo_mean)
     for (int i = 0; i < c->snm; i++)
       if (!(expo_mean[i] > 0.0)) return c->fail(IMA_ERR_ARG, "exponential prior mean %d must be > 0", i);
-  const int nchunks = margin_chunks(rg ? rg->hi - rg->lo : c->sG, n);
+  // requests by parameter, each parameter's filling whole blocks
+  std::vector<int> count(npar, 0), at(npar, 0);
+  for (int k = 0; k < n; k++) count[param[k]]++;
+  const int lognx = margin_log_block(*std::max_element(count.begin(), count.end()));
+  const int nx = 1 << lognx;
+  int np = 0;
+  for (int q = 0; q < npar; q++) {
+    at[q] = np;
+    np += (count[q] + nx - 1) / nx * nx;
+  }
+  std::vector<int32_t> hp(np);
+  std::vector<double> hx(np), hout(np);
+  std::vector<int> slot(n);
+  for (int k = 0; k < n; k++) {
+    slot[k] = at[param[k]]++;
+    hp[slot[k]] = param[k];
+    hx[slot[k]] = x[k];
+  }
+  for (int q = 0; q < npar; q++)
+    for (; at[q] % nx; at[q]++) {
+      hp[at[q]] = q;
+      hx[at[q]] = hx[at[q] / nx * nx];
+    }
+  const int ncall = n;
+  n = np;
+  const int nchunks = margin_chunks(rg ? rg->hi - rg->lo : c->sG, n / nx);
   // one device block: param | x | means | out | partials
   const size_t bytes = 256 * 5 + (size_t)n * 4 + (size_t)n * 8 + 64 * 8 + (size_t)n * 8 + (size_t)n * nchunks * 8;
   if (bytes > c->mscratch_cap) {
@@ -2493,17 +2519,20 @@ static int margin_run(ima_ctx *c, int n, const int32_t *param, const double *x, 
   a.param = d_param;
   a.x = d_x;
   a.expo_mean = expo_mean ? d_mean : nullptr;
-  int r = c->cuda(cudaMemcpyAsync(d_param, param, (size_t)n * 4, cudaMemcpyHostToDevice, c->st), "marginal points");
-  r = r ? r : c->cuda(cudaMemcpyAsync(d_x, x, (size_t)n * 8, cudaMemcpyHostToDevice, c->st), "marginal points");
+  int r = c->cuda(cudaMemcpyAsync(d_param, hp.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->st), "marginal points");
+  r = r ? r : c->cuda(cudaMemcpyAsync(d_x, hx.data(), (size_t)n * 8, cudaMemcpyHostToDevice, c->st), "marginal points");
   if (expo_mean) r = r ? r : c->cuda(cudaMemcpyAsync(d_mean, expo_mean, (size_t)c->snm * 8, cudaMemcpyHostToDevice, c->st), "means");
   if (r) return r;
   int lr = 0;
-  c->launch(IMA_K_MARGIN, (double)c->sG * c->srowlen * 4, [&] { lr = launch_margin(a, d_part, nchunks, d_out, c->st); });
+  c->launch(IMA_K_MARGIN, (double)c->sG * c->srowlen * 4, [&] { lr = launch_margin(a, lognx, d_part, nchunks, d_out, c->st); });
   c->launches += 1;  // pass + merge
   if (lr) return c->fail(IMA_ERR_ARG, "marginal: unsupported shape (%d)", lr);
   r = c->cuda(cudaGetLastError(), "marginal launch");
-  r = r ? r : c->cuda(cudaMemcpyAsync(out, d_out, (size_t)n * 8, cudaMemcpyDeviceToHost, c->st), "marginal values");
-  return r ? r : c->cuda(cudaStreamSynchronize(c->st), "marginal");
+  r = r ? r : c->cuda(cudaMemcpyAsync(hout.data(), d_out, (size_t)n * 8, cudaMemcpyDeviceToHost, c->st), "marginal values");
+  r = r ? r : c->cuda(cudaStreamSynchronize(c->st), "marginal");
+  if (!r)
+    for (int k = 0; k < ncall; k++) out[k] = hout[slot[k]];
+  return r;
 }
 
 static int ensure_logfact(ima_ctx *c);

@@ -155,13 +155,17 @@ struct MarginArgs {
   double div;               // the sum is divided by this (G for margincalc)
   int ccp, fcp, hccp, mcp, fmp, qip, mip;  // gsampinf column offsets
   const float *rows;        // [G][rowlen]
+  // n requests in blocks of 2^lognx of one parameter each (a block's spare
+  // entries repeat its first)
   const int32_t *param;     // [n] parameter index (population sizes first)
   const double *x;          // [n]
   const double *expo_mean;  // [nm] or null
   double yadjust;
 };
-int margin_chunks(int G, int n);
-int launch_margin(const MarginArgs &a, double *part, int nchunks, double *out, cudaStream_t st);
+int margin_init_tables();
+int margin_log_block(int most);  // lognx for at most `most` requests of one parameter
+int margin_chunks(int G, int nblocks);
+int launch_margin(const MarginArgs &a, int lognx, double *part, int nchunks, double *out, cudaStream_t st);
 
 // 2NM densities (calc_popmig / calc_pop_expomig) at n requested points
 struct PopmigArgs {

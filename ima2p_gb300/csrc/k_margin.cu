@@ -11,72 +11,107 @@
 // range of genealogies, takes the theta term's cc as stored and divides by
 // the range's length (+1 when it starts at genealogy 0).
 //
-// One thread per requested (parameter, x) and genealogy chunk; tiles of whole
-// gsampinf rows are staged in shared memory with coalesced loads, and every
-// thread reads its parameter's three or four columns from there.  Partial sums
-// per chunk are added in chunk order by the merge kernel.
+// A term is c a(x) + f b(x) + base: c the count, f the rate and base
+// everything that does not depend on x, all of one genealogy.  A CTA takes
+// requests of one parameter, so a tile's (c, f, base) go to shared memory as
+// doubles once for all its requests, in units of ln 2, and a term costs two
+// FP64 FMAs (three under an exponential prior); 2^term is formed in fixed
+// point on the integer pipe and summed in 96-bit integers (fxexp.cuh).  GB300
+// issues about 1.6 FP64 operations or conversions per cycle and SM: the
+// former kernel (conversions, six operations and an FP64 exponential per
+// term) spent 20 cycles a term, 83 ms for 13,000 points x 100,000
+// genealogies; the FP64 and integer pipes are now about evenly loaded.
+//
+// Threads: `nx` requests by MG_BS / nx genealogy strides, nx the power of two
+// that holds the largest parameter's requests, so a search's few points
+// still use every lane.  Partial sums per chunk are added in chunk order by
+// the merge kernel.
 #include <cfloat>
 #include <cmath>
 
+#include "fxexp.cuh"
 #include "internal.h"
 
 namespace {
 
-constexpr int MG_BS = 128;   // requests per CTA
-constexpr int MG_TG = 64;    // genealogies per shared-memory tile
-constexpr int MG_MAXROW = 64;
+constexpr int MG_BS = 128;  // threads per CTA
+constexpr int MG_TG = 128;  // genealogies per shared-memory tile
 constexpr double LOG2 = 0.69314718055994530942;
+constexpr double LOG2E = 1.4426950408889634074;
+constexpr double FX_LIMIT = 1000.0;  // |term| in units of ln 2 below which the fixed-point form holds
+
+__constant__ uint64_t c_fxtab[FX_TAB];
 
 __device__ __forceinline__ double intround(float v)  // INTEGERROUND (imamp.hpp:180)
 {
   return v >= 0.f ? (double)(long long)((double)v + 0.5) : (double)(long long)((double)v - 0.5);
 }
 
-__global__ void __launch_bounds__(MG_BS) k_margin(MarginArgs a, int chunk, double *part)
+template <bool EXPO>
+__global__ void __launch_bounds__(MG_BS) k_margin(MarginArgs a, int lognx, int chunk, double *part)
 {
-  __shared__ float tile[MG_TG * MG_MAXROW];
-  const int k = blockIdx.x * MG_BS + threadIdx.x;
-  const bool live = k < a.n;
-  const int pi = live ? a.param[k] : 0;
-  const double x = live ? a.x[k] : 1.0;
+  __shared__ uint64_t tab[FX_TAB];
+  __shared__ double sc[MG_TG], sf[MG_TG], sb[MG_TG];
+  const int tid = threadIdx.x, nx = 1 << lognx;
+  const int k = blockIdx.x * nx + (tid & (nx - 1));  // this thread's request
+  const int sub = tid >> lognx, nsub = MG_BS >> lognx;
+  for (int i = tid; i < FX_TAB; i += MG_BS) tab[i] = c_fxtab[i];
+  const int pi = a.param[blockIdx.x * nx];
+  const double x = a.x[k];
   const bool theta = pi < a.np;
-  // per-request constants
-  const double lx = theta ? LOG2 - log(x) : log(x);
-  const double ix = 1.0 / x;
-  double cst = 0.0, slope = 0.0;
-  if (!theta && a.expo_mean) {
+  // the term's coefficients in units of ln 2
+  const double A = (theta ? LOG2 - log(x) : log(x)) * LOG2E;
+  const double B = (theta ? 1.0 / x : x) * LOG2E;
+  double cst = 0.0;
+  if (EXPO && !theta) {
     const double meani = 1.0 / a.expo_mean[pi - a.np];
-    cst = log(meani);
-    slope = meani;
+    cst = (log(meani) - x * meani) * LOG2E;
   }
-  int c0, c1, c2, c3;  // columns: (qi, cc, hcc, fc) or (mi, mc, fm, -)
-  if (theta) {
-    c0 = a.qip + pi; c1 = a.ccp + pi; c2 = a.hccp + pi; c3 = a.fcp + pi;
-  } else {
-    const int p = pi - a.np;
-    c0 = a.mip + p; c1 = a.mcp + p; c2 = a.fmp + p; c3 = c2;
-  }
+  const int p = pi - a.np;  // columns: (qi, cc, hcc, fc) or (mi, mc, fm)
+  const int c0 = theta ? a.qip + pi : a.mip + p, c1 = theta ? a.ccp + pi : a.mcp + p,
+            c2 = theta ? a.hccp + pi : a.fmp + p, c3 = theta ? a.fcp + pi : c2;
   const int g0 = a.g_lo + blockIdx.y * chunk, g1 = min(a.g_hi, g0 + chunk);
-  double sum = 0.0;
+  FxSum sum;
+  sum.init();
+  int since = 0;  // terms since the last flush
   for (int t0 = g0; t0 < g1; t0 += MG_TG) {
     const int nt = min(MG_TG, g1 - t0);
     __syncthreads();
-    const float *src = a.rows + (size_t)t0 * a.rowlen;  // nt whole rows are contiguous
-    for (int i = threadIdx.x; i < nt * a.rowlen; i += MG_BS) tile[i] = src[i];
+    if (tid < nt) {
+      const float *r = a.rows + (size_t)(t0 + tid) * a.rowlen;
+      const float r0 = r[c0], r1 = r[c1], r2 = r[c2], r3 = r[c3];
+      sc[tid] = theta && a.raw_cc ? (double)r1 : intround(r1);
+      sf[tid] = theta ? -2.0 * (double)r3 : -(double)r2;
+      sb[tid] = theta ? (-(double)r0 - (double)r2) * LOG2E : -(double)r0 * LOG2E;
+    }
     __syncthreads();
-    if (!live) continue;
-    for (int j = 0; j < nt; j++) {
-      const float *r = tile + j * a.rowlen;
-      double temp;
-      if (theta)
-        temp = -(double)r[c0] + (a.raw_cc ? (double)r[c1] : intround(r[c1])) * lx - (double)r[c2] -
-               2.0 * (double)r[c3] * ix;
-      else
-        temp = -(double)r[c0] + cst - x * slope + intround(r[c1]) * lx - (double)r[c2] * x;
-      sum += exp(temp);
+    for (int j = sub; j < nt; j += nsub) {
+      double v = __fma_rn(sc[j], A, __fma_rn(sf[j], B, sb[j]));
+      if (EXPO) v += cst;
+      if (fabs(v) < FX_LIMIT) {
+        int i;
+        const uint64_t m = fx_exp2(v, tab, &i);
+        sum.add(m, i);
+      } else {  // beyond it, infinite or NaN
+        sum.total += exp2(v);
+      }
+    }
+    since += (nt - sub + nsub - 1) / nsub;
+    if (since > 512 - MG_TG) {
+      sum.flush();
+      since = 0;
     }
   }
-  if (live) part[(size_t)k * gridDim.y + blockIdx.y] = sum;
+  sum.flush();
+  double s = sum.total;
+  if (nsub > 1) {  // the strides of a request, in order
+    __shared__ double red[MG_BS];
+    red[tid] = s;
+    __syncthreads();
+    if (sub == 0)
+      for (int w = 1; w < nsub; w++) s += red[(w << lognx) + tid];
+  }
+  if (sub == 0) part[(size_t)k * gridDim.y + blockIdx.y] = s;
 }
 
 __global__ void k_margin_merge(MarginArgs a, int nchunks, const double *part, double *out)
@@ -92,23 +127,39 @@ __global__ void k_margin_merge(MarginArgs a, int nchunks, const double *part, do
 
 }  // namespace
 
-int margin_chunks(int G, int n)
+int margin_init_tables()
 {
-  const int rblocks = (n + MG_BS - 1) / MG_BS;
-  int nchunks = (4 * 152 + rblocks - 1) / rblocks;  // about four waves of CTAs
-  const int maxc = (G + 4 * MG_TG - 1) / (4 * MG_TG);  // at least four tiles per chunk
+  uint64_t t[FX_TAB];
+  for (int j = 0; j < FX_TAB; j++) t[j] = (uint64_t)(exp2l((long double)j / FX_TAB) * 9223372036854775808.0L);
+  return cudaMemcpyToSymbol(c_fxtab, t, sizeof(t)) == cudaSuccess ? 0 : -1;
+}
+
+int margin_chunks(int G, int nblocks)
+{
+  // about sixteen waves of one CTA per SM (eight fit at a time)
+  int nchunks = (16 * 152 + nblocks - 1) / nblocks;
+  const int maxc = (G + 2 * MG_TG - 1) / (2 * MG_TG);  // at least two tiles per chunk
   if (nchunks > maxc) nchunks = maxc;
   return nchunks < 1 ? 1 : nchunks;
 }
 
-int launch_margin(const MarginArgs &a, double *part, int nchunks, double *out, cudaStream_t st)
+int margin_log_block(int most)
 {
-  if (a.rowlen > MG_MAXROW || a.n < 1) return 2;
+  int l = 0;
+  while ((1 << l) < most && (1 << l) < MG_BS) l++;
+  return l;
+}
+
+int launch_margin(const MarginArgs &a, int lognx, double *part, int nchunks, double *out, cudaStream_t st)
+{
+  if (a.n < 1) return 2;
   const int ng = a.g_hi - a.g_lo;
   if (ng < 1) return 2;
   const int chunk = ((ng + nchunks - 1) / nchunks + MG_TG - 1) / MG_TG * MG_TG;
   nchunks = (ng + chunk - 1) / chunk;
-  k_margin<<<dim3((a.n + MG_BS - 1) / MG_BS, nchunks), MG_BS, 0, st>>>(a, chunk, part);
+  const dim3 grid(a.n >> lognx, nchunks);
+  if (a.expo_mean) k_margin<true><<<grid, MG_BS, 0, st>>>(a, lognx, chunk, part);
+  else k_margin<false><<<grid, MG_BS, 0, st>>>(a, lognx, chunk, part);
   k_margin_merge<<<(a.n + 127) / 128, 128, 0, st>>>(a, nchunks, part, out);
   return 0;
 }

@@ -59,3 +59,29 @@ def test_margincalc_rejects_bad_points():
         ctx.margincalc([5], [1.0])
     with pytest.raises(api.ImaError):
         ctx.margincalc([0], [0.0])
+
+
+@pytest.mark.parametrize("G", [1, 127, 128, 129, 1000])
+@pytest.mark.parametrize("counts", [(1, 0, 0, 0, 0), (3, 1, 0, 2, 5), (127, 128, 129, 1, 0)])
+@pytest.mark.parametrize("expo", [False, True])
+def test_margincalc_blocks_and_tiles(G, counts, expo):
+    """Requests of several parameters in one call, around the 128 a block
+    holds, over genealogy counts around the 128 of a tile; half the rows have
+    prior integrals that put the terms beyond +-1000 ln 2 (the FP64 path), at
+    the RTOL of the module."""
+    rng = np.random.default_rng(G + 7 * sum(counts))
+    rows, _, off = synth.surface_stats(rng, G, 3, 2, 1)
+    shift = rng.choice([0.0, -690.0, 640.0], size=G)
+    if G == 1:
+        shift[:] = -690.0
+    rows[:, off["qi"]:off["qi"] + 3] += shift[:, None].astype(np.float32)
+    param = np.repeat(np.arange(5), counts)
+    x = np.where(param < 3, rng.uniform(0.5, 20.0, len(param)), rng.uniform(0.05, 2.0, len(param)))
+    order = rng.permutation(len(param))
+    param, x = param[order], x[order]
+    em = np.array([0.7, 1.3]) if expo else None
+    ctx = ctx_with([("sw", 2, 1)])
+    ctx.surface_load(rows, 3, 2, 2)
+    got = ctx.margincalc(param, x, expo_mean=em)
+    want = np.array([O.margincalc(rows, 3, 2, int(p), float(v), expo_mean=em) for p, v in zip(param, x)])
+    np.testing.assert_allclose(got, want, rtol=RTOL)

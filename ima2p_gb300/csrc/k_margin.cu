@@ -19,8 +19,10 @@
 // point on the integer pipe and summed in 96-bit integers (fxexp.cuh).  GB300
 // issues about 1.6 FP64 operations or conversions per cycle and SM: the
 // former kernel (conversions, six operations and an FP64 exponential per
-// term) spent 20 cycles a term, 83 ms for 13,000 points x 100,000
-// genealogies; the FP64 and integer pipes are now about evenly loaded.
+// term) spent 20 cycles a term, 83.5 ms for 13,000 points x 100,000
+// genealogies; now 6.8 ms, 5.2 of them the two FMAs of each term.  Adding the
+// doubles instead (a third FP64 operation) measured 14.6 ms against 11.9 for
+// the integer sums before the last two steps (integer compare, shorter tail).
 //
 // Threads: `nx` requests by MG_BS / nx genealogy strides, nx the power of two
 // that holds the largest parameter's requests, so a search's few points
@@ -38,7 +40,7 @@ constexpr int MG_BS = 128;  // threads per CTA
 constexpr int MG_TG = 128;  // genealogies per shared-memory tile
 constexpr double LOG2 = 0.69314718055994530942;
 constexpr double LOG2E = 1.4426950408889634074;
-constexpr double FX_LIMIT = 1000.0;  // |term| in units of ln 2 below which the fixed-point form holds
+constexpr int FX_LIMIT_HI = 0x408f4000;  // high word of 1000.0, the bound of the fixed-point form's argument
 
 __constant__ uint64_t c_fxtab[FX_TAB];
 
@@ -88,7 +90,8 @@ __global__ void __launch_bounds__(MG_BS) k_margin(MarginArgs a, int lognx, int c
     for (int j = sub; j < nt; j += nsub) {
       double v = __fma_rn(sc[j], A, __fma_rn(sf[j], B, sb[j]));
       if (EXPO) v += cst;
-      if (fabs(v) < FX_LIMIT) {
+      // |v| < 1000, compared as bits: a DSETP would be a third FP64 operation
+      if ((__double2hiint(v) & 0x7fffffff) < FX_LIMIT_HI) {
         int i;
         const uint64_t m = fx_exp2(v, tab, &i);
         sum.add(m, i);
@@ -136,8 +139,9 @@ int margin_init_tables()
 
 int margin_chunks(int G, int nblocks)
 {
-  // about sixteen waves of one CTA per SM (eight fit at a time)
-  int nchunks = (16 * 152 + nblocks - 1) / nblocks;
+  // about six waves of eight resident CTAs per SM: the last one is then a
+  // small share (two waves left a quarter of the kernel to its tail)
+  int nchunks = (48 * 152 + nblocks - 1) / nblocks;
   const int maxc = (G + 2 * MG_TG - 1) / (2 * MG_TG);  // at least two tiles per chunk
   if (nchunks > maxc) nchunks = maxc;
   return nchunks < 1 ? 1 : nchunks;

@@ -36,21 +36,26 @@ __host__ __device__ __forceinline__ uint64_t fx_mul64(uint64_t a, uint32_t b)
   return (uint64_t)(uint32_t)(a >> 32) * b + fx_mulhi((uint32_t)a, b);
 }
 
-// 2^a = m 2^(i - 63), m in [2^63, 2^64), for |a| < 1000.  a goes to fixed
-// point with 53 fraction bits (exact for |a| >= 1/2, within 2^-54 below).
-__host__ __device__ __forceinline__ uint64_t fx_exp2(double a, const uint64_t *tab, int *i)
+// a in fixed point with 53 fraction bits, |a| < 1000 (exact for |a| >= 1/2,
+// within 2^-54 below)
+__host__ __device__ __forceinline__ int64_t fx_fix(double a)
 {
   const uint64_t b = fx_bits(a);
   const int hi = (int)(b >> 32);
   const uint64_t man = (b << 11) | (1ull << 63);
   int sh = 1033 - ((hi >> 20) & 0x7ff);  // 10 - E
   sh = sh < 63 ? sh : 63;
-  uint64_t v = man >> sh;
-  if (hi < 0) v = 0ull - v;
+  const uint64_t v = man >> sh;
+  return (int64_t)(hi < 0 ? 0ull - v : v);
+}
+
+// 2^(v 2^-53) = m 2^(i - 63), m in [2^63, 2^64)
+__host__ __device__ __forceinline__ uint64_t fx_exp2(int64_t v, const uint64_t *tab, int *i)
+{
   const int vh = (int)(v >> 32);
   *i = vh >> 21;
   const uint64_t T = tab[(vh >> 12) & (FX_TAB - 1)];
-  const uint64_t rho = v << 20;  // the low 44 bits: rho in [0, 1), 2^64
+  const uint64_t rho = (uint64_t)v << 20;  // the low 44 bits: rho in [0, 1), 2^64
   const uint32_t r = (uint32_t)(rho >> 32), rl = (uint32_t)rho;
   const uint32_t g3 = FX_L3 + fx_mulhi(r, FX_L4);
   const uint64_t g2 = FX_L2 + ((uint64_t)fx_mulhi(r, g3) << 10);

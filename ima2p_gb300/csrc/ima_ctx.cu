@@ -469,7 +469,7 @@ extern "C" int ima_gpu_create(int device, ima_ctx **out)
   cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&c->pageable_access, cudaDevAttrPageableMemoryAccess, device);
   if (sw_init_tables() != 0 || hky_init_tables() != 0 || surf_init_tables() != 0 ||
-      margin_init_tables() != 0) {
+      margin_init_tables() != 0 || popmig_init_tables() != 0) {
     delete c;
     return IMA_ERR_CUDA;
   }
@@ -2555,13 +2555,38 @@ static int popmig_run(ima_ctx *c, int n, const int32_t *thetai, const int32_t *m
     if (mig_mean && !(mig_mean[i] > 0.0)) return c->fail(IMA_ERR_ARG, "exponential prior mean %d must be > 0", i);
   }
   if (int r0 = ensure_logfact(c)) return r0;
-  const int nchunks = popmig_chunks(rg ? rg->hi - rg->lo : c->sG, n);
-  std::vector<double> hq(n), hm(n), hmean(mig_mean ? n : 0);
-  for (int k = 0; k < n; k++) {
-    hq[k] = theta_max[thetai[k]];
-    hm[k] = mig_max[mi[k]];
-    if (mig_mean) hmean[k] = mig_mean[mi[k]];
+  // uniform prior: points by term, each term's filling whole blocks (spare
+  // entries repeat a block's first); exponential prior: as they come
+  std::vector<int> count((size_t)c->snp * c->snm, 0), at(count.size(), 0), slot(n);
+  auto term = [&](int k) { return thetai[k] * c->snm + mi[k]; };
+  for (int k = 0; k < n; k++) count[term(k)]++;
+  const int lognx = mig_mean ? 5 : popmig_log_block(*std::max_element(count.begin(), count.end()));
+  const int nx = 1 << lognx, ncall = n;
+  if (!mig_mean) {
+    n = 0;
+    for (size_t q = 0; q < count.size(); q++) {
+      at[q] = n;
+      n += (count[q] + nx - 1) / nx * nx;
+    }
   }
+  std::vector<int32_t> hth(n), hmi(n);
+  std::vector<double> hx(n), hout(n), hq(n), hm(n), hmean(mig_mean ? n : 0);
+  auto put = [&](int at_, int th, int m, double xv) {
+    hth[at_] = th;
+    hmi[at_] = m;
+    hx[at_] = xv;
+    hq[at_] = theta_max[th];
+    hm[at_] = mig_max[m];
+    if (mig_mean) hmean[at_] = mig_mean[m];
+  };
+  for (int k = 0; k < ncall; k++) {
+    slot[k] = mig_mean ? k : at[term(k)]++;
+    put(slot[k], thetai[k], mi[k], x[k]);
+  }
+  if (!mig_mean)
+    for (size_t q = 0; q < count.size(); q++)
+      for (; at[q] % nx; at[q]++) put(at[q], (int)q / c->snm, (int)q % c->snm, hx[at[q] / nx * nx]);
+  const int nchunks = popmig_chunks(rg ? rg->hi - rg->lo : c->sG, (n + nx - 1) / nx, mig_mean ? 1 : 0);
   // one device block: thetai | mi | x | qmax | mmax | mmean | out | error | partials
   const size_t bytes = 256 * 9 + (size_t)n * (4 + 4 + 8 * 5) + 8 + (size_t)n * nchunks * 16;
   if (bytes > c->mscratch_cap) {
@@ -2613,23 +2638,25 @@ static int popmig_run(ima_ctx *c, int n, const int32_t *thetai, const int32_t *m
   a.mmean = mig_mean ? d_mean : nullptr;
   a.logfact = c->d_logfact;
   a.err = d_err;
-  int r = c->cuda(cudaMemcpyAsync(d_th, thetai, (size_t)n * 4, cudaMemcpyHostToDevice, c->st), "2NM points");
-  r = r ? r : c->cuda(cudaMemcpyAsync(d_mi, mi, (size_t)n * 4, cudaMemcpyHostToDevice, c->st), "2NM points");
-  r = r ? r : c->cuda(cudaMemcpyAsync(d_x, x, (size_t)n * 8, cudaMemcpyHostToDevice, c->st), "2NM points");
+  int r = c->cuda(cudaMemcpyAsync(d_th, hth.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->st), "2NM points");
+  r = r ? r : c->cuda(cudaMemcpyAsync(d_mi, hmi.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->st), "2NM points");
+  r = r ? r : c->cuda(cudaMemcpyAsync(d_x, hx.data(), (size_t)n * 8, cudaMemcpyHostToDevice, c->st), "2NM points");
   r = r ? r : c->cuda(cudaMemcpyAsync(d_q, hq.data(), (size_t)n * 8, cudaMemcpyHostToDevice, c->st), "2NM priors");
   r = r ? r : c->cuda(cudaMemcpyAsync(d_m, hm.data(), (size_t)n * 8, cudaMemcpyHostToDevice, c->st), "2NM priors");
   if (mig_mean) r = r ? r : c->cuda(cudaMemcpyAsync(d_mean, hmean.data(), (size_t)n * 8, cudaMemcpyHostToDevice, c->st), "2NM priors");
   r = r ? r : c->cuda(cudaMemsetAsync(d_err, 0, 4, c->st), "2NM status");
   if (r) return r;
   int lr = 0;
-  c->launch(IMA_K_POPMIG, (double)c->sG * c->srowlen * 4, [&] { lr = launch_popmig(a, d_part, nchunks, d_out, c->st); });
+  c->launch(IMA_K_POPMIG, (double)c->sG * c->srowlen * 4, [&] { lr = launch_popmig(a, lognx, d_part, nchunks, d_out, c->st); });
   c->launches += 1;  // pass + merge
   if (lr) return c->fail(IMA_ERR_ARG, "2NM densities: unsupported shape (%d)", lr);
   int32_t err = 0;
   r = c->cuda(cudaGetLastError(), "2NM launch");
-  r = r ? r : c->cuda(cudaMemcpyAsync(out, d_out, (size_t)n * 8, cudaMemcpyDeviceToHost, c->st), "2NM values");
+  r = r ? r : c->cuda(cudaMemcpyAsync(hout.data(), d_out, (size_t)n * 8, cudaMemcpyDeviceToHost, c->st), "2NM values");
   r = r ? r : c->cuda(cudaMemcpyAsync(&err, d_err, 4, cudaMemcpyDeviceToHost, c->st), "2NM status");
   r = r ? r : c->cuda(cudaStreamSynchronize(c->st), "2NM");
+  if (!r)
+    for (int k = 0; k < ncall; k++) out[k] = hout[slot[k]];
   if (!r && err)
     return c->fail(IMA_ERR_DATA, "2NM density: %s", err == 5 ? "a count beyond the logfact table"
                                                              : "an incomplete gamma series or fraction did not converge");

@@ -179,8 +179,11 @@ struct PopmigArgs {
   const double *logfact;                   // [TW_LF_N]
   int32_t *err;                            // first failing series / fraction (0 = none)
 };
-int popmig_chunks(int G, int n);
-int launch_popmig(const PopmigArgs &a, double *part, int nchunks, double *out, cudaStream_t st);
+int popmig_init_tables();
+int popmig_log_block(int most);  // lognx for at most `most` points of one term
+int popmig_chunks(int G, int nblocks, int expo);
+// uniform prior: n points in blocks of 2^lognx of one term each
+int launch_popmig(const PopmigArgs &a, int lognx, double *part, int nchunks, double *out, cudaStream_t st);
 
 // findmarginpeaks' numeric core (margin_peaks.cu, host): the searches run
 // together, their function values evaluated in batches by `eval`

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(MG_BS) k_margin(MarginArgs a, int lognx, int c
       // |v| < 1000, compared as bits: a DSETP would be a third FP64 operation
       if ((__double2hiint(v) & 0x7fffffff) < FX_LIMIT_HI) {
         int i;
-        const uint64_t m = fx_exp2(v, tab, &i);
+        const uint64_t m = fx_exp2(fx_fix(v), tab, &i);
         sum.add(m, i);
       } else {  // beyond it, infinite or NaN
         sum.total += exp2(v);

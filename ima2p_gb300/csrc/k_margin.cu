@@ -132,9 +132,15 @@ __global__ void k_margin_merge(MarginArgs a, int nchunks, const double *part, do
 
 int margin_init_tables()
 {
-  uint64_t t[FX_TAB];
-  for (int j = 0; j < FX_TAB; j++) t[j] = (uint64_t)(exp2l((long double)j / FX_TAB) * 9223372036854775808.0L);
-  return cudaMemcpyToSymbol(c_fxtab, t, sizeof(t)) == cudaSuccess ? 0 : -1;
+  struct Tab {
+    uint64_t t[FX_TAB];
+  };
+  static const Tab tab = [] {  // once per process (long double is slow in software on aarch64)
+    Tab v;
+    for (int j = 0; j < FX_TAB; j++) v.t[j] = (uint64_t)(exp2l((long double)j / FX_TAB) * 9223372036854775808.0L);
+    return v;
+  }();
+  return cudaMemcpyToSymbol(c_fxtab, tab.t, sizeof(tab.t)) == cudaSuccess ? 0 : -1;
 }
 
 int margin_chunks(int G, int nblocks)

@@ -20,7 +20,8 @@
 // 1.6 million random terms its mean relative error is 1e-14, that of the FP64
 // form 9e-7 on the same terms (log(1 - P) loses what x2 - x1 needs).
 // Measured on 8 curves of 1,000 points over 10,000 genealogies: 121.6 ms
-// before.  k_popmig: a CTA is one warp of 32 points and one chunk, each lane
+// before, 21.4 with every piece of the term inlined twice (instruction cache
+// misses were half of the stalls), 13.2 now.  k_popmig: a CTA is one warp of 32 points and one chunk, each lane
 // walking the rows.
 // Each (point, chunk) partial has its own slot.  calc_popmig's sum
 // of exp(temp1 + temp2) (terms outside +-700 skipped) is kept per chunk;
@@ -141,16 +142,17 @@ __device__ __forceinline__ ff pf_value(ff x, bool series, int na, int n, const f
 {
   if (series) {
     ff t = ff_from(1.f);
+#pragma unroll 1
     for (int k = n; k >= 1; k--) t = pf_series_step(t, x, rcp[na + k]);
     return ff_mul(t, ffc(rcp[na]));
   }
   const ff b0 = ff_add_f(x, (float)(1 - na));
-  const float fa = (float)na;
   const float sc = __int_as_float((254 - ((__float_as_int(b0.hi + (float)n) >> 23) & 0xff)) << 23);
   const ff bn = ff_add_f(b0, (float)(2 * n));
   ff p1 = ff_make(bn.hi * sc, bn.lo * sc), p2 = ff_from(1.f);
+#pragma unroll 1
   for (int k = n - 1; k >= 0; k--) {
-    const ff q = pf_fraction_step(b0, k, fa, sc, p1, p2);
+    const ff q = pf_fraction_step(b0, (float)k, (float)na, sc, p1, p2);
     p2 = p1;
     p1 = q;
   }
@@ -180,7 +182,7 @@ __device__ __forceinline__ double pf_ln(double q, const FxLogTab &T)
   const uint64_t f = fx_log2(q, T, &e);
   return ((double)(e + 1) - (f ? (double)(0ull - f) * 5.421010862427522e-20 : 1.0)) * 0.69314718055994530942;
 }
-constexpr int DIFF_BITS = 7;
+constexpr double DIFF_MIN = 1.0 / 128;
 
 __global__ void __launch_bounds__(32 * PF_WARPS, 4) k_popmig_fast(PopmigArgs a, int lognx, int nblocks, int nchunks,
                                                                int chunk, double *part)
@@ -236,72 +238,100 @@ __global__ void __launch_bounds__(32 * PF_WARPS, 4) k_popmig_fast(PopmigArgs a, 
       if (na > 0 && fine) {
         const double z = __fma_rn(G.fm, x, G.fc);
         const ff zf = ff_split(z);
-        const ff x1 = ff_mul(zf, r1f), x2 = ff_mul(zf, r2f);
         const float fa = (float)na;
-        const bool s1 = __fsub_rn(x1.hi, fa + 1.f) + x1.lo < 0.f, s2 = __fsub_rn(x2.hi, fa + 1.f) + x2.lo < 0.f;
-        const int n1 = s1 ? pf_series_terms(fa, x1.hi) : pf_fraction_terms(fa, __fsub_rn(x1.hi, fa - 1.f) + x1.lo);
-        const int n2 = s2 ? pf_series_terms(fa, x2.hi) : pf_fraction_terms(fa, __fsub_rn(x2.hi, fa - 1.f) + x2.lo);
         const double K = __fma_rn(G.mc, lx, G.base);
-        const double e1 = __fma_rn(z, c1, __fma_rn(G.a, l1, K)), e2 = __fma_rn(z, c2, __fma_rn(G.a, l2, K));
-        if (n1 > 0 && n2 > 0 && (s1 || !s2) && pf_in(e1) && pf_in(e2)) {
-          const ff v1 = pf_value(x1, s1, na, n1, T.rcp), v2 = pf_value(x2, s2, na, n2, T.rcp);
-          const double d1 = (double)v1.hi + (double)v1.lo, d2 = (double)v2.hi + (double)v2.lo;
-          const int64_t f1 = fx_fix(e1), f2 = fx_fix(e2);
-          int i;
-          double d = 0.0, big = 0.0;
-          if (s1) {
-            // Gamma(a) z^-a = 2^w, which needs log z
-            const double kg = __fma_rn(G.mc, lx, G.baseg);
-            int e;
-            const uint64_t f = fx_log2(z, T.lg, &e);
-            const int ae = na * e;
-            if (pf_in(kg) && abs(ae) < 999) {
-              const int64_t la = ((int64_t)ae << 53) +
-                                 (int64_t)((((uint64_t)(uint32_t)na * (uint32_t)(f >> 32)) << 21) +
-                                           (((uint64_t)(uint32_t)na * (uint32_t)f) >> 11));
-              const int64_t fk = fx_fix(kg), w = fk - la;
-              if (pf_sub_in(fk, la) && pf_sub_in(f1, w) && pf_sub_in(f2, w)) {
-                uint64_t m = fx_exp2(w, T.ex, &i);
-                big = pf_double(m, i);
-                m = fx_exp2(f1 - w, T.ex, &i);
-                const double g1s = pf_double(m, i) * d1;
-                m = fx_exp2(f2 - w, T.ex, &i);
-                const double g2s = pf_double(m, i) * d2;
-                if (!s2) {
-                  d = (1.0 - g1s - g2s) * big;
-                } else {
-                  // both from series: the reference subtracts two logarithms
-                  // gln + log(1 - P), and where P is small their rounding (an
-                  // ulp of gln) is what its difference keeps; rounded alike here
-                  const double q1 = 1.0 - g1s, q2 = 1.0 - g2s;
-                  if (q1 > 0.0 && q2 > 0.0) {
-                    const double A = G.gln + pf_ln(q1, T.lg), B = G.gln + pf_ln(q2, T.lg);
-                    const double df = A - B;
-                    if (df > 0.0) {
-                      m = fx_exp2(fx_fix(df * PF_LOG2E), T.ex, &i);
-                      const double E = __longlong_as_double((long long)(((uint64_t)(i + 1022) << 52) + (m >> 11) +
-                                                                        ((m >> 10) & 1)));
-                      d = (E - 1.0) * q2 * big;
-                      if (E == 1.0) d = -1.0;  // the reference takes log(0): the FP64 form
-                      else D = pf_kept(d) ? d : D;
-                      big = 0.0;
-                    } else if (df == 0.0) {
-                      d = (g2s - g1s) * big;  // it turns to the lower functions, which separate them
-                      big *= g2s;
-                    }
-                  }
-                }
-              }
-            }
+        // x1 then x2 through the same instructions (the kernel's code would
+        // not fit the instruction cache twice): value, exponent, kind
+        double v[2];
+        int64_t f[2];
+        bool s[2], ok = true;
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) {
+          const ff xh = ff_mul(zf, h ? r2f : r1f);
+          const bool se = __fsub_rn(xh.hi, fa + 1.f) + xh.lo < 0.f;
+          const int n = se ? pf_series_terms(fa, xh.hi) : pf_fraction_terms(fa, __fsub_rn(xh.hi, fa - 1.f) + xh.lo);
+          const double e = __fma_rn(z, h ? c2 : c1, __fma_rn(G.a, h ? l2 : l1, K));
+          ok = ok && n > 0 && pf_in(e);
+          const ff vf = pf_value(xh, se, na, n, T.rcp);
+          const double vd = (double)vf.hi + (double)vf.lo;
+          const int64_t fe = fx_fix(e);
+          if (h == 0) {
+            v[0] = vd;
+            f[0] = fe;
+            s[0] = se;
           } else {
-            uint64_t m = fx_exp2(f1, T.ex, &i);
-            big = pf_double(m, i) * d1;
-            m = fx_exp2(f2, T.ex, &i);
-            d = big - pf_double(m, i) * d2;
+            v[1] = vd;
+            f[1] = fe;
+            s[1] = se;
           }
-          // the difference at least 2^-DIFF_BITS of its larger part: below,
-          // the rounding of the reference's logarithms shows
-          if (big > 0.0 && (__double2hiint(d) >> 20) > (__double2hiint(big) >> 20) - DIFF_BITS && pf_kept(d)) D = d;
+        }
+        ok = ok && (s[0] || !s[1]);
+        // everything relative to 2^w: Gamma(a) z^-a where x1 takes the series
+        // (which needs log z), else x1's own factor
+        int64_t w = f[0];
+        if (s[0]) {
+          const double kg = __fma_rn(G.mc, lx, G.baseg);
+          int e;
+          const uint64_t lf = fx_log2(z, T.lg, &e);
+          const int ae = na * e;
+          ok = ok && pf_in(kg) && abs(ae) < 999;
+          const int64_t la = ((int64_t)ae << 53) +
+                             (int64_t)((((uint64_t)(uint32_t)na * (uint32_t)(lf >> 32)) << 21) +
+                                       (((uint64_t)(uint32_t)na * (uint32_t)lf) >> 11));
+          const int64_t fk = fx_fix(kg);
+          ok = ok && pf_sub_in(fk, la);
+          w = fk - la;
+        }
+        ok = ok && pf_sub_in(f[0], w) && pf_sub_in(f[1], w);
+        if (ok) {
+          double g1s = 0.0, g2s = 0.0, big = 0.0;
+#pragma unroll 1
+          for (int h = 0; h < 3; h++) {
+            int i;
+            const uint64_t m = fx_exp2(h == 2 ? w : (h ? f[1] : f[0]) - w, T.ex, &i);
+            const double e = pf_double(m, i);
+            if (h == 0) g1s = e * v[0];
+            else if (h == 1) g2s = e * v[1];
+            else big = e;
+          }
+          double d = -1.0, rel;  // rel: the difference over its larger part
+          if (!s[0]) {
+            d = g1s - g2s;
+            rel = d > DIFF_MIN * g1s ? 1.0 : 0.0;
+            d *= big;
+          } else if (!s[1]) {
+            rel = 1.0 - g1s - g2s;
+            d = rel * big;
+          } else {
+            // both from series: the reference subtracts two logarithms gln +
+            // log(1 - P), and where P is small their rounding (an ulp of gln)
+            // is what its difference keeps; rounded alike here
+            rel = 1.0;
+            double A[2];
+            const double q2 = 1.0 - g2s;
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) {
+              const double q = h ? q2 : 1.0 - g1s;
+              rel = q > 0.0 ? rel : 0.0;
+              const double l = G.gln + pf_ln(q, T.lg);
+              if (h == 0) A[0] = l;
+              else A[1] = l;
+            }
+            const double df = A[0] - A[1];
+            if (df > 0.0) {
+              int i;
+              const uint64_t m = fx_exp2(fx_fix(df * PF_LOG2E), T.ex, &i);
+              const double E = __longlong_as_double((long long)(((uint64_t)(i + 1022) << 52) + (m >> 11) +
+                                                                ((m >> 10) & 1)));
+              d = (E - 1.0) * q2 * big;
+              if (E == 1.0) rel = 0.0;  // the reference takes log(0)
+            } else {
+              d = (g2s - g1s) * big;  // equal: it turns to the lower functions, which separate them
+              if (df < 0.0) rel = 0.0;
+            }
+          }
+          // below DIFF_MIN the rounding of the reference's logarithms shows
+          if (rel > DIFF_MIN && pf_kept(d)) D = d;
         }
       }
       sum += D >= 0.0 ? D
@@ -391,20 +421,29 @@ __global__ void k_popmig_merge(PopmigArgs a, int nchunks, const double *part, do
 
 }  // namespace
 
+// the tables, made once per process (long double is slow in software on aarch64)
+static const PfTables &pf_tables()
+{
+  static const PfTables t = [] {
+    PfTables v{};
+    for (int j = 0; j < FX_TAB; j++) {
+      v.ex[j] = (uint64_t)(exp2l((long double)j / FX_TAB) * 9223372036854775808.0L);
+      const uint64_t r = (4294967296ull * FX_TAB + FX_TAB + j - 1) / (FX_TAB + j);  // ceil
+      v.lg.r[j] = (uint32_t)(r - 1);
+      v.lg.l[j] = j ? (uint64_t)(-log2l((long double)r / 4294967296.0L) * 18446744073709551616.0L) : 0ull;
+    }
+    for (int k = 1; k < PF_RCP; k++) {
+      const long double w = 1.0L / k;
+      v.rcp[k] = make_float2((float)w, (float)(w - (long double)(float)w));
+    }
+    return v;
+  }();
+  return t;
+}
+
 int popmig_init_tables()
 {
-  static PfTables t;
-  for (int j = 0; j < FX_TAB; j++) {
-    t.ex[j] = (uint64_t)(exp2l((long double)j / FX_TAB) * 9223372036854775808.0L);
-    const uint64_t r = (4294967296ull * FX_TAB + FX_TAB + j - 1) / (FX_TAB + j);  // ceil
-    t.lg.r[j] = (uint32_t)(r - 1);
-    t.lg.l[j] = j ? (uint64_t)(-log2l((long double)r / 4294967296.0L) * 18446744073709551616.0L) : 0ull;
-  }
-  for (int k = 1; k < PF_RCP; k++) {
-    const long double v = 1.0L / k;
-    t.rcp[k] = make_float2((float)v, (float)(v - (long double)(float)v));
-  }
-  return cudaMemcpyToSymbol(d_pf, &t, sizeof(t)) == cudaSuccess ? 0 : -1;
+  return cudaMemcpyToSymbol(d_pf, &pf_tables(), sizeof(PfTables)) == cudaSuccess ? 0 : -1;
 }
 
 int popmig_log_block(int most)

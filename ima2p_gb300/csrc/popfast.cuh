@@ -58,7 +58,9 @@ __device__ __forceinline__ uint64_t fx_log2(double z, const FxLogTab &T, int *e)
 
 __device__ __forceinline__ float pf_rcp(float a)
 {
-  return __frcp_rn(a);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
 }
 
 // The number of terms of gser (utilities.cpp: del < sum EPS), 0 when too
@@ -97,16 +99,29 @@ __device__ __forceinline__ int pf_fraction_terms(float a, float b0)
 // One step of the series by Horner's rule: t <- 1 + t x / k
 __device__ __forceinline__ ff pf_series_step(ff t, ff x, float2 rk)
 {
-  return ff_add_f(ff_mul(ff_mul(t, x), ffc(rk)), 1.0f);
+  // t x and x / k unnormalised: the TwoSum with 1 is exact whatever their lo
+  const float q = __fmul_rn(x.hi, rk.x);
+  const float qe = __fmaf_rn(x.hi, rk.y, __fmaf_rn(x.lo, rk.x, __fmaf_rn(x.hi, rk.x, -q)));
+  const float u = __fmul_rn(t.hi, q);
+  const float ue = __fmaf_rn(t.hi, qe, __fmaf_rn(t.lo, q, __fmaf_rn(t.hi, q, -u)));
+  const ff s = two_sum(1.0f, u);
+  return fast_two_sum(s.hi, __fadd_rn(s.lo, ue));
 }
 
 // One step of the fraction's numerators: p_k = b_k p_(k+1) + a_(k+1) p_(k+2),
-// scaled by s (a power of two)
-__device__ __forceinline__ ff pf_fraction_step(ff b0, int k, float a, float s, ff p1, ff p2)
+// scaled by s (a power of two).  Beyond k = a the second term is negative, but
+// the fraction converges there without losing more than a few bits.
+__device__ __forceinline__ ff pf_fraction_step(ff b0, float k, float a, float s, ff p1, ff p2)
 {
-  const ff b = ff_add_f(b0, (float)(2 * k));
-  const float ak = (float)(k + 1) * (a - (float)(k + 1)) * (s * s);
-  return ff_add(ff_mul(ff_make(b.hi * s, b.lo * s), p1), ff_mul_f(p2, ak));
+  const ff b2 = two_sum(b0.hi, k + k);
+  const ff b = ff_make(b2.hi * s, (b2.lo + b0.lo) * s);
+  const float ak = (k + 1.f) * (a - (k + 1.f)) * (s * s);
+  // b p1 and ak p2 unnormalised, one TwoSum of their leading parts
+  const float u = __fmul_rn(b.hi, p1.hi), v = __fmul_rn(ak, p2.hi);
+  const float ue = __fmaf_rn(b.hi, p1.lo, __fmaf_rn(b.lo, p1.hi, __fmaf_rn(b.hi, p1.hi, -u)));
+  const float ve = __fmaf_rn(ak, p2.lo, __fmaf_rn(ak, p2.hi, -v));
+  const ff t = two_sum(u, v);
+  return fast_two_sum(t.hi, __fadd_rn(t.lo, __fadd_rn(ue, ve)));
 }
 
 }  // namespace

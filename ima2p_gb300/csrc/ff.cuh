@@ -6,6 +6,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstdint>
+
 struct ff {
   float hi, lo;
 };
@@ -44,6 +46,19 @@ __device__ __forceinline__ ff ff_add(ff a, ff b)
   ff u = fast_two_sum(s.hi, e);
   e = __fadd_rn(t.lo, u.lo);
   return fast_two_sum(u.hi, e);
+}
+
+// a non-negative double as float-float on the integer pipe (a conversion
+// would take an FP64 issue slot, 1/64 of the FP32 rate): the leading 24 bits
+// truncated and the other 29 rounded to 24.  Outside the range where both
+// parts are normal floats: converted.
+__device__ __forceinline__ ff ff_split(double z)
+{
+  const int hi = __double2hiint(z), lo = __double2loint(z);
+  const int e = (hi >> 20) - 896;  // the float's biased exponent
+  if (e < 60 || e > 254) return ff_make((float)z, (float)(z - (double)(float)z));
+  const float h = __int_as_float((e << 23) | (int)(((uint32_t)(hi & 0xfffff) << 3) | ((uint32_t)lo >> 29)));
+  return ff_make(h, (float)(lo & 0x1fffffff) * __int_as_float((e - 52) << 23));
 }
 
 __device__ __forceinline__ ff ff_neg(ff a) { return ff_make(-a.hi, -a.lo); }

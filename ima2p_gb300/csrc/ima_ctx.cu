@@ -60,6 +60,7 @@ struct Batch {
   int hky_variant = 0, sw_variant = 0;  // launch shapes (ima_gpu_batch_autotune)
   // MC3 sweep of the batch (ima_gpu_batch_sweep): its items and accept mask
   // on the device, and the graph of evaluation, commit and swaps
+  long long cls_gen = -1;  // ima_ctx::cls_gen when the pattern classes of its items were last brought up to date
   int32_t *d_items = nullptr;
   uint8_t *d_acc = nullptr;
   cudaGraphExec_t sgraph = nullptr;
@@ -259,6 +260,12 @@ struct ima_ctx {
   unsigned long long *d_ctr = nullptr;
   int32_t *d_is_site = nullptr;  // IS per-site mutation branches, valid while the topology is
   uint8_t *d_is_valid = nullptr;
+  // HKY pattern classes, allocated on first use; cls_gen counts the changes
+  // of topology, a batch remembers the count its items' classes match
+  uint2 *d_ctask = nullptr;
+  uint16_t *d_crep = nullptr;
+  int32_t *d_clev = nullptr;
+  long long cls_gen = 0;
   double *d_uni = nullptr;
   size_t uni_cap = 0;
 
@@ -387,6 +394,9 @@ struct ima_ctx {
     P.sumlogk = d_sumlogk;
     P.is_site = d_is_site;
     P.is_valid = d_is_valid;
+    P.ctask = d_ctask;
+    P.crep = d_crep;
+    P.clev = d_clev;
     P.pdg_new = d_pdg_new;
     P.part = d_part;
     P.partlo = d_partlo;
@@ -506,7 +516,8 @@ extern "C" void ima_gpu_destroy(ima_ctx *c)
                   c->d_mscratch, c->d_tw, c->d_logfact, c->d_twerr, c->d_twin, c->d_twout, c->d_tpbuf,
                   c->d_pop, c->d_moff, c->d_inode_off, c->d_gl, c->d_gt, c->d_moff_start, c->d_bcnt, c->d_bicnt,
                   c->d_mig_p, c->d_rsamp, c->d_mbase, c->d_mig_t, c->d_tvr, c->d_len_hold, c->d_rhlog,
-                  c->d_rh2, c->d_rsel, c->d_is_site, c->d_is_valid, c->d_lterm, c->d_ug};
+                  c->d_rh2, c->d_rsel, c->d_is_site, c->d_is_valid, c->d_lterm, c->d_ug,
+                  c->d_ctask, c->d_crep, c->d_clev};
   for (void *p : devs)
     if (p) cudaFree(p);
   void *hosts[] = {c->h_nodes, c->h_t64, c->h_sched, c->h_nlev, c->h_len, c->h_pi, c->h_al};
@@ -1394,7 +1405,8 @@ static int flush(ima_ctx *c)
   r = r ? r : c->cuda(cudaMemcpyAsync(c->d_len + lo, c->h_len + lo, (hi - lo + 1) * sizeof(double), cudaMemcpyHostToDevice, st), "length");
   r = r ? r : c->cuda(cudaMemcpyAsync(c->d_pi + 4 * (size_t)lo, c->h_pi + 4 * (size_t)lo, 4 * (hi - lo + 1) * sizeof(double), cudaMemcpyHostToDevice, st), "pi");
   if (a1 > a0) r = r ? r : c->cuda(cudaMemcpyAsync(c->d_al + a0, c->h_al + a0, (a1 - a0) * sizeof(int32_t), cudaMemcpyHostToDevice, st), "alleles");
-  // topologies may have changed: the IS site caches of the range are stale
+  // topologies may have changed: the caches of the range are stale
+  c->cls_gen++;
   r = r ? r : c->cuda(cudaMemsetAsync(c->d_is_valid + lo, 0, hi - lo + 1, st), "IS site cache");
   c->dirty_lo = INT32_MAX;
   c->dirty_hi = -1;
@@ -1437,6 +1449,36 @@ static int ensure_ff_hky(ima_ctx *c)
   return c->cuda(cudaMemsetAsync(c->d_partlo, 0, c->npart * sizeof(float4), c->st), "float-float partials");
 }
 
+static int ensure_classes_alloc(ima_ctx *c)
+{
+  if (c->d_ctask || c->npart == 0) return IMA_OK;
+  c->d_ctask = dev_alloc<uint2>(c->npart / 2, c->dev_bytes, c->st);
+  c->d_crep = dev_alloc<uint16_t>(c->npart / 2, c->dev_bytes, c->st);
+  c->d_clev = dev_alloc<int32_t>(c->nsched, c->dev_bytes, c->st);
+  if (!c->d_ctask || !c->d_crep || !c->d_clev) {
+    cudaFree(c->d_ctask);
+    cudaFree(c->d_crep);
+    cudaFree(c->d_clev);
+    c->d_ctask = nullptr;
+    c->d_crep = nullptr;
+    c->d_clev = nullptr;
+    return c->fail(IMA_ERR_NOMEM, "HKY pattern classes (%zu tasks) do not fit", c->npart / 2);
+  }
+  return IMA_OK;
+}
+
+// The pattern classes of a batch's HKY items, after its flush and before its
+// kernels (or their graph) run
+static int ensure_classes(ima_ctx *c, Batch &b)
+{
+  if (!b.nhky || b.prec == IMA_PREC_FP64 || b.cls_gen == c->cls_gen) return IMA_OK;
+  if (int r = ensure_classes_alloc(c)) return r;
+  launch_hky_classes(c->pools(), b.d_req + b.nis, b.nhky, b.maxn_hky, b.maxs_hky, c->st);
+  c->launches++;
+  b.cls_gen = c->cls_gen;
+  return c->cuda(cudaGetLastError(), "pattern classes");
+}
+
 static double hky_bytes(ima_ctx *c, const Batch &b);
 static double sw_bytes(ima_ctx *c, const Batch &b);
 
@@ -1472,6 +1514,7 @@ static int build_batch(ima_ctx *c, Batch &b, int n, const int32_t *ci, const int
     std::stable_sort(g[m].begin(), g[m].end(), [&](int a, int b) { return cost(a) > cost(b); });
   b.n = n;
   b.prec = prec;
+  b.cls_gen = -1;
   b.nis = (int)g[0].size();
   b.nhky = (int)g[1].size();
   b.nsw = (int)g[2].size();
@@ -1746,6 +1789,7 @@ extern "C" int ima_gpu_eval(ima_ctx *c, int n, const int32_t *ci, const int32_t 
   r = r ? r : flush(c);
   r = r ? r : (b.nis ? ensure_lengths(c) : IMA_OK);  // the infinite-sites likelihood reads them
   r = r ? r : init_sumlogk(c, b);
+  r = r ? r : ensure_classes(c, b);
   if (!r) enqueue(c, b);
   r = r ? r : c->cuda(cudaGetLastError(), "launch");
   r = r ? r : fetch(c, b, result, status);
@@ -1801,6 +1845,7 @@ extern "C" int ima_gpu_batch_run(ima_ctx *c, int batch, int use_graph)
   int r = flush(c);
   r = r ? r : (b.nis ? ensure_lengths(c) : IMA_OK);  // the infinite-sites likelihood reads them
   r = r ? r : init_sumlogk(c, b);
+  r = r ? r : ensure_classes(c, b);
   if (r) return r;
   if (!use_graph || c->profiling) {
     enqueue(c, b);
@@ -1836,6 +1881,7 @@ extern "C" int ima_gpu_batch_autotune(ima_ctx *c, int batch, int reps, int *hky_
   int r = flush(c);
   r = r ? r : (b.nis ? ensure_lengths(c) : IMA_OK);  // the infinite-sites likelihood reads them
   r = r ? r : init_sumlogk(c, b);
+  r = r ? r : ensure_classes(c, b);
   if (r) return r;
   if (reps < 1) reps = 1;
   if (b.prec != IMA_PREC_FP64 && (b.nhky || b.nsw)) {
@@ -1976,6 +2022,7 @@ extern "C" int ima_gpu_batch_sweep(ima_ctx *c, int batch, const uint8_t *accept,
   int r = flush(c);
   r = r ? r : (b.nis ? ensure_lengths(c) : IMA_OK);  // the infinite-sites likelihood reads them
   r = r ? r : init_sumlogk(c, b);
+  r = r ? r : ensure_classes(c, b);
   if (r) return r;
   if (!b.d_items) {
     std::vector<int32_t> items(b.n);
@@ -4479,6 +4526,10 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
           c->launch(IMA_K_UG, 0.0, [&] { launch_ug_sw(u_, sh); }, sh);
         } else {
           if (!u_.hky) cudaStreamWaitEvent(sh, evW[slot], 0);  // the IS likelihood reads the new lengths
+          if (u_.hky && precision != IMA_PREC_FP64) {  // the proposals changed the topologies
+            launch_hky_classes(c->pools(), b.d_req, b.nhky, b.maxn_hky, b.maxs_hky, sh);
+            c->launches++;
+          }
           enqueue(c, b, sh);
         }
         cudaEventRecord(evH[slot], sh);
@@ -4491,6 +4542,7 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
     }
   if (step > 0) cudaStreamWaitEvent(c->st, evD[(step - 1) % R], 0);  // st carries on after the last decision
   // the device's genealogies are newer than the mirror from here on
+  c->cls_gen++;
   for (int k = 0; k < nch; k++) {
     c->topo_lo = std::min(c->topo_lo, chains[k] * nl);
     c->topo_hi = std::max(c->topo_hi, chains[k] * nl + nl - 1);

@@ -71,7 +71,12 @@ struct Pools {
   double *sumlogk;          // IS per-locus constant
   int32_t *is_site;         // IS: per item and site, (mutation node << 8) | branch (0 first daughter,
                             // 1 second, 2 both at the root); node -1 none, -2 two
-  uint8_t *is_valid;        // IS: the item's site cache matches its topology
+  uint8_t *is_valid;        // the item's cache (IS: sites; HKY: pattern classes) matches its topology
+  // HKY pattern classes (k_hky_classes), per item at part_off / 2: tasks and
+  // representatives; task starts per level at sched_off
+  uint2 *ctask;
+  uint16_t *crep;
+  int32_t *clev;
   double *pdg_new;          // last evaluated log P(D|G) per item
   // HKY state
   float4 *part;             // FP32 partials (float-float form: the hi parts)
@@ -95,6 +100,9 @@ constexpr int HKY_FAST_VARIANTS = 6;  // float-float: 128 threads with registers
 constexpr int SW_FAST_VARIANTS = 3;   // one wave (5 or 6 CTAs per SM), 8 chain-loci per CTA
 void launch_hky_fast(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, int variant,
                      double *result, int32_t *status, cudaStream_t st);
+// the pattern classes of the requests' items whose cache is stale (before
+// launch_hky_fast and launch_hky_fp32, after every change of topology)
+void launch_hky_classes(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, cudaStream_t st);
 void launch_hky_fp32(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, int variant,
                      double *result, int32_t *status, cudaStream_t st);
 void launch_hky_fp64(const Pools &P, const ReqDev *reqs, int nreq, int maxn, double *result,

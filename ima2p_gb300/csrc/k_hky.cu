@@ -27,6 +27,7 @@
 // log L; the pairs bring that below 1e-8.
 // FP64 form: the reference's arithmetic -- partials divided by their maximum,
 // log(max) accumulated into an FP64 scale factor.
+#include <algorithm>
 #include <cmath>
 
 #include "ff.cuh"
@@ -34,7 +35,8 @@
 
 namespace {
 
-__constant__ FFConsts c_ffh;  // ln 2 and the log table (filled by hky_init_tables)
+__constant__ FFConsts c_ffh;     // ln 2 and the log table (filled by hky_init_tables)
+__device__ float2 d_exp64m1[64];  // 2^((j - 32) / 64) - 1 as float-float
 
 constexpr int HKY_BS = 128;
 constexpr double LN2 = 0.69314718055994530941723212146;
@@ -125,19 +127,65 @@ __device__ __forceinline__ void hky_apply(const HkyCoef &K, const float *pi, flo
   v[3] = fmaf(K.dY, L.w, tY);
 }
 
+// e^x and e^x - 1 of x <= 0 in float-float: x = k ln2 / 64 + r, |r| <= ln2 /
+// 128, y = 2^(j/64) e^r - 1 from its table t_j = 2^(j/64) - 1, j in [-32, 32)
+// (signed, so that a short branch has j = 0 and keeps its relative accuracy),
+// and m = e^r - 1: y = t + m + t m; then e^x = 2^e (1 + y).  About 75
+// instructions (ff_exp_expm1's four doublings take 110); relative errors
+// within 3e-14 of e^x - 1 and of e^x.
+constexpr float L64_A = 0.01082611083984375f;     // ln 2 / 64 = A + B + C: k A and k B exact for |k| < 2^13
+constexpr float L64_B = 4.3101608753204346e-06f;
+constexpr float L64_C = 3.695530104153022e-09f;
+__device__ __forceinline__ void hky_exp(ff x, const float2 *tab, ff *ex, ff *em1)
+{
+  if (x.hi < -86.0f) {
+    *ex = ff_from(0.0f);
+    *em1 = ff_from(-1.0f);
+    return;
+  }
+  const float z = __fmaf_rn(x.hi, 92.33248262f, 12582912.f);
+  const float kf = __fsub_rn(z, 12582912.f);
+  const int k = __float_as_int(z) - 0x4B400000;
+  const float c = __fmul_rn(-kf, L64_C);
+  ff r = two_sum(__fmaf_rn(-kf, L64_B, __fmaf_rn(-kf, L64_A, x.hi)), c);
+  r.lo = __fadd_rn(r.lo, __fadd_rn(x.lo, __fmaf_rn(-kf, L64_C, -c)));
+  const float h = r.hi;
+  // m = r (1 + r (1/2 + r (1/6 + r (1/24 + r / 120))))
+  const float g = __fmaf_rn(h, 1.f / 120, 1.f / 24);
+  const float s3 = __fmaf_rn(h, g, 0.16666667f), s3l = __fmaf_rn(h, g, 0.16666667f - s3) - 4.967054e-09f;
+  const float a1 = __fmul_rn(h, s3), a1e = __fmaf_rn(h, s3, -a1) + __fmaf_rn(h, s3l, r.lo * s3);
+  const ff s2 = fast_two_sum(0.5f, a1);
+  const float s2l = __fadd_rn(s2.lo, a1e);
+  const float a2 = __fmul_rn(h, s2.hi), a2e = __fmaf_rn(h, s2.hi, -a2) + __fmaf_rn(h, s2l, r.lo * s2.hi);
+  const ff s1 = fast_two_sum(1.0f, a2);
+  const ff m = ff_mul(r, ff_make(s1.hi, __fadd_rn(s1.lo, a2e)));
+  const int j = (k + 32) & 63, e = (k + 32 - j) >> 6;
+  const ff t = ffc(tab[j]);
+  const ff y = ff_add(ff_add(t, m), ff_mul(t, m));
+  const float p2 = __int_as_float((127 + e) << 23);
+  const ff one_y = ff_add_f(y, 1.0f);
+  *ex = ff_make(one_y.hi * p2, one_y.lo * p2);
+  *em1 = e == 0 ? y : ff_add_f(*ex, -1.0f);
+}
+
+// What the branches of a chain-locus share: A_c = 1 + Pi_c (kappa - 1),
+// 1 / Pi_c and 1 - Pi_c of the two classes.
+struct HkyShared {
+  float2 AR, AY, iR, iY, oR, oY;
+};
+
 // Float-float coefficients of one branch, K = {E1, b_R, b_Y, d_R, d_Y} as
 // (hi, lo) pairs: E1 = 1 - e^-b, E2_c = 1 - e^(-b A_c), d_c = e^(-b A_c)
 // taken directly (1 - E2_c would cancel on long branches).
-__device__ __forceinline__ void hky_coef_ff(const ff *pi, ff kpa, ff b, float *K)
+__device__ __forceinline__ void hky_coef_ff(const HkyShared &H, const float2 *tab, ff b, float *K)
 {
-  const ff PR = ff_add(pi[0], pi[2]), PY = ff_add(pi[1], pi[3]);
   ff e1, m1, eR, mR, eY, mY;
-  ff_exp_expm1(ff_neg(b), &e1, &m1);
-  ff_exp_expm1(ff_neg(ff_mul(b, ff_add_f(ff_mul(PR, kpa), 1.0f))), &eR, &mR);
-  ff_exp_expm1(ff_neg(ff_mul(b, ff_add_f(ff_mul(PY, kpa), 1.0f))), &eY, &mY);
+  hky_exp(ff_neg(b), tab, &e1, &m1);
+  hky_exp(ff_neg(ff_mul(b, ffc(H.AR))), tab, &eR, &mR);
+  hky_exp(ff_neg(ff_mul(b, ffc(H.AY))), tab, &eY, &mY);
   const ff E1 = ff_neg(m1), ER = ff_neg(mR), EY = ff_neg(mY);
-  const ff bR = ff_div(ff_sub(ER, ff_mul(E1, ff_add_f(ff_neg(PR), 1.0f))), PR);
-  const ff bY = ff_div(ff_sub(EY, ff_mul(E1, ff_add_f(ff_neg(PY), 1.0f))), PY);
+  const ff bR = ff_mul(ff_sub(ER, ff_mul(E1, ffc(H.oR))), ffc(H.iR));
+  const ff bY = ff_mul(ff_sub(EY, ff_mul(E1, ffc(H.oY))), ffc(H.iY));
   K[0] = E1.hi; K[1] = E1.lo;
   K[2] = bR.hi; K[3] = bR.lo;
   K[4] = bY.hi; K[5] = bY.lo;
@@ -158,14 +206,16 @@ __device__ __forceinline__ ff ff_fma_pos(ff a, ff b, ff c)
 struct HkyCoefFF {
   ff a, bR, bY, dR, dY;
 };
-__device__ __forceinline__ HkyCoefFF load_coef_ff(const float *Kp)
+__device__ __forceinline__ HkyCoefFF load_coef_ff(const float *Kp)  // 16-byte aligned
 {
+  const float4 a = reinterpret_cast<const float4 *>(Kp)[0], b = reinterpret_cast<const float4 *>(Kp)[1];
+  const float2 c = reinterpret_cast<const float2 *>(Kp)[4];
   HkyCoefFF K;
-  K.a = ff_make(Kp[0], Kp[1]);
-  K.bR = ff_make(Kp[2], Kp[3]);
-  K.bY = ff_make(Kp[4], Kp[5]);
-  K.dR = ff_make(Kp[6], Kp[7]);
-  K.dY = ff_make(Kp[8], Kp[9]);
+  K.a = ff_make(a.x, a.y);
+  K.bR = ff_make(a.z, a.w);
+  K.bY = ff_make(b.x, b.y);
+  K.dR = ff_make(b.z, b.w);
+  K.dY = ff_make(c.x, c.y);
   return K;
 }
 // P(b) applied to a tip observed in state st: column st of P(b)
@@ -213,17 +263,148 @@ __device__ __forceinline__ void hky_apply_ff(const HkyCoefFF &K, const ff *pi, c
 __device__ __forceinline__ ff ff_of(float2 v) { return ff_make(v.x, v.y); }
 
 // Shared-memory carve-up, identical on host (sizing) and device.
+// tip, inner: bytes of one branch's coefficients below a tip and below an
+// internal node; times: bytes of one node's time.
 struct HkyLayout {
-  size_t nd, fresh, order, total;
+  size_t inner, nd, times, fresh, order, lev, total;
 };
-__host__ __device__ inline HkyLayout hky_layout(int maxnl, size_t elem)
+__host__ __device__ inline HkyLayout hky_layout(int maxnl, size_t tip, size_t inner, size_t time)
 {
+  const size_t maxn = (size_t)(maxnl + 1) / 2;
   HkyLayout l;
-  l.nd = elem * 16 * (size_t)maxnl;
-  l.fresh = l.nd + sizeof(NodeRec) * (size_t)maxnl;
+  l.inner = tip * maxn;
+  l.nd = l.inner + inner * maxn;
+  l.times = l.nd + sizeof(NodeRec) * (size_t)maxnl;
+  l.fresh = l.times + time * (size_t)maxnl;
   l.order = (l.fresh + 3 * (size_t)maxnl + 15) & ~size_t(15);
-  l.total = (l.order + sizeof(int16_t) * (size_t)(maxnl + 3) + 15) & ~size_t(15);
+  l.lev = (l.order + sizeof(int16_t) * (size_t)(maxnl + 3) + 15) & ~size_t(15);
+  l.total = (l.lev + sizeof(int32_t) * (size_t)(maxnl / 2 + 2) + 15) & ~size_t(15);
   return l;
+}
+__host__ __device__ inline HkyLayout hky_layout64(int maxnl)  // k_hky_fp64: a 4 x 4 matrix per branch
+{
+  return hky_layout(maxnl, 16 * sizeof(double), 16 * sizeof(double), 0);
+}
+// k_hky_fast, in floats: a tip branch's 32 are padded so that lanes on
+// different branches of a level start in different banks
+__host__ __device__ constexpr int hky_tip_floats(bool ff) { return ff ? 36 : 8; }
+__host__ __device__ constexpr int hky_inner_floats(bool ff) { return ff ? 12 : 8; }
+__host__ __device__ inline HkyLayout hky_layout_fast(int maxnl, bool ff)
+{
+  return hky_layout(maxnl, 4 * hky_tip_floats(ff), 4 * hky_inner_floats(ff), sizeof(float2));
+}
+
+// ----------------------------------------------------- pattern classes
+// Below a node, site patterns that agree on its tips have the same partial.
+// A node's classes are numbered in the order of their first patterns, which
+// depends only on the tips below it, so that a clean node's stored partials
+// (one per class, at the class's number) stay addressable whatever happens
+// above.  k_hky_classes lists, per level, one task per class of each node: x =
+// (node - n) | class << 16, y = the index of either daughter's value (a tip's
+// state, or the class in the daughter), the internal daughter first.  The
+// root keeps every pattern, for the sum.  On sequences simulated on their
+// genealogies 8-20% of the (node, pattern) pairs remain, on random ones 30-40%.
+// Loci of more than CLS_MAXS patterns keep every pattern (CLS_MAXS bounds a
+// warp's hash table).
+constexpr int CLS_MAXS = 2048;
+constexpr int CLS_WARPS = 8;
+constexpr size_t CLS_SHARED = 32 * 1024;  // class numbers of all nodes and patterns kept in shared memory up to this
+constexpr uint32_t CLS_EMPTY = 0xffffffffu;
+
+__device__ __forceinline__ int2 hky_children(const NodeRec &nd, int n)
+{
+  return nd.up0 < n && nd.up1 >= n ? make_int2(nd.up1, nd.up0) : make_int2(nd.up0, nd.up1);
+}
+
+__global__ void __launch_bounds__(32 * CLS_WARPS) k_hky_classes(Pools P, const ReqDev *reqs, int maxnl, int logh, int cap)
+{
+  extern __shared__ __align__(16) char smem[];
+  const ReqDev R = reqs[blockIdx.x];
+  const int n = R.n, nl = 2 * n - 1, S = R.nsites, nint = n - 1;
+  if (S > CLS_MAXS || P.is_valid[R.item]) return;
+  const int H = 1 << logh;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  NodeRec *nd = reinterpret_cast<NodeRec *>(smem);
+  int16_t *order = reinterpret_cast<int16_t *>(nd + maxnl);
+  uint32_t *keys = reinterpret_cast<uint32_t *>(smem + ((sizeof(NodeRec) * maxnl + 2 * (maxnl + 3) + 15) & ~size_t(15))) +
+                   (size_t)warp * (H + H / 2);
+  uint16_t *vals = reinterpret_cast<uint16_t *>(keys + H);
+  __shared__ int count;  // tasks listed so far
+  for (int k = threadIdx.x; k < nl; k += 32 * CLS_WARPS) nd[k] = P.nodes[R.node_off + k];
+  for (int k = threadIdx.x; k < 2 * n; k += 32 * CLS_WARPS) order[k] = P.sched[R.sched_off + k];
+  if (threadIdx.x == 0) count = 0;
+  const int nlev = P.nlev[R.item];
+  const int16_t *lstart = order + nint;
+  const int8_t *seq = P.seq + R.seq_off;
+  // the classes of every node and pattern, read back by the parents
+  uint16_t *rep = nint * S <= cap ? reinterpret_cast<uint16_t *>(keys + (size_t)(CLS_WARPS - warp) * (H + H / 2))
+                                  : P.crep + R.part_off / 2;
+  uint2 *task = P.ctask + R.part_off / 2;
+  int32_t *clev = P.clev + R.sched_off;
+  __syncthreads();
+  for (int lv = 0; lv < nlev; lv++) {
+    if (threadIdx.x == 0) clev[lv] = count;
+    __syncthreads();
+    const int cnt = lstart[lv + 1] - lstart[lv];
+    for (int j = warp; j < cnt; j += CLS_WARPS) {
+      const int node = order[lstart[lv] + j];
+      const int2 c = hky_children(nd[node], n);
+      const bool root = nd[node].down < 0;  // its patterns are summed one by one
+      if (!root)
+        for (int h = lane; h < H; h += 32) keys[h] = CLS_EMPTY;
+      __syncwarp();
+      int ncls = 0;  // classes so far
+      for (int p0 = 0; p0 < S; p0 += 32) {
+        const int p = p0 + lane;
+        const bool in = p < S;
+        uint32_t ia = 0, ib = 0;
+        if (in) {
+          ia = c.x < n ? (uint32_t)seq[(size_t)c.x * S + p] : rep[(size_t)(c.x - n) * S + p];
+          ib = c.y < n ? (uint32_t)seq[(size_t)c.y * S + p] : rep[(size_t)(c.y - n) * S + p];
+        }
+        const uint32_t key = ia | ib << 16;
+        bool first = in;
+        unsigned f;
+        int r = p;
+        if (root) {
+          f = __ballot_sync(0xffffffffu, in);
+        } else {
+          const unsigned m = __match_any_sync(0xffffffffu, in ? key : CLS_EMPTY);
+          const int lead = __ffs(m) - 1;
+          first = false;
+          uint32_t h = 0;
+          if (in && lane == lead) {
+            // one lane per distinct key of these 32: find it or claim a slot
+            for (h = (key * 2654435761u) >> (32 - logh);; h = (h + 1) & (H - 1)) {
+              const uint32_t old = atomicCAS(&keys[h], CLS_EMPTY, key);
+              if (old == CLS_EMPTY) first = true;
+              else if (old == key) r = vals[h];
+              else continue;
+              break;
+            }
+          }
+          f = __ballot_sync(0xffffffffu, first);
+          if (first) {
+            r = ncls + __popc(f & ((1u << lane) - 1u));
+            vals[h] = (uint16_t)r;
+          }
+          ncls += __popc(f);
+          __syncwarp();
+          r = __shfl_sync(0xffffffffu, r, lead);
+          if (in) rep[(size_t)(node - n) * S + p] = (uint16_t)r;
+        }
+        int base = 0;
+        if (lane == 0) base = atomicAdd(&count, __popc(f));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (first) task[base + __popc(f & ((1u << lane) - 1u))] = make_uint2((uint32_t)(node - n) | (uint32_t)r << 16, key);
+      }
+    }
+    __syncthreads();  // the level's classes before its parents
+  }
+  if (threadIdx.x == 0) {
+    clev[nlev] = count;
+    P.is_valid[R.item] = 1;
+  }
 }
 
 // Per-CTA shared state common to both precisions.
@@ -301,42 +482,44 @@ __device__ __forceinline__ int expo_of(float m)  // floor(log2(m)) for normal m 
 template <bool FF, bool CACHE, int BS, int MINB>
 __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *reqs,
                                                      double *result, int32_t *status, int maxnl,
-                                                     int cache_S, int tip_cap)
+                                                     int cache_S, int task_cap)
 {
   extern __shared__ __align__(16) char smem[];
   // the request carries the item's offsets and sizes, so the tree loads
   // below wait on this one load only
   const ReqDev R = reqs[blockIdx.x];
   const int n = R.n, nl = 2 * n - 1, S = R.nsites, nint = n - 1;
-  // [maxnl][PMS]: 5 coefficients per branch (FF: pairs); FF tip branches
-  // hold instead the columns of P(b) for the four observed states, [4][4]
-  // pairs, so a tip daughter costs four loads
-  constexpr int PMS = FF ? 32 : 16;
-  const HkyLayout lay = hky_layout(maxnl, FF ? 2 * sizeof(float) : sizeof(float));
-  float *Pm = reinterpret_cast<float *>(smem);
+  // per branch 5 coefficients (FF: pairs); FF tip branches hold instead the
+  // columns of P(b) for the four observed states, [4][4] pairs, so a tip
+  // daughter costs two loads
+  constexpr int PT = hky_tip_floats(FF), PI = hky_inner_floats(FF);
+  const HkyLayout lay = hky_layout_fast(maxnl, FF);
+  float *Pt = reinterpret_cast<float *>(smem);                       // [tip][PT]
+  float *Pi = reinterpret_cast<float *>(smem + lay.inner) - n * PI;  // [internal node][PI]
+  float2 *stm = reinterpret_cast<float2 *>(smem + lay.times);        // node times
   Tree T;
   T.nd = reinterpret_cast<NodeRec *>(smem + lay.nd);
   T.fresh = reinterpret_cast<uint8_t *>(smem + lay.fresh);
   T.dirty = T.fresh + maxnl;
   T.slot = T.dirty + maxnl;
   T.order = reinterpret_cast<int16_t *>(smem + lay.order);
-  // the tips' states [n][S] when they fit in tip_cap bytes: the level loop
-  // then reads no global memory when the partials are cached too
-  int8_t *stip = reinterpret_cast<int8_t *>(smem + lay.total);
-  const size_t tipb = ((size_t)tip_cap + 15) & ~size_t(15);
-  const bool tips = n * S <= tip_cap;
-  float4 *cpart = reinterpret_cast<float4 *>(smem + lay.total + tipb);  // [nint][cache_S]
+  int32_t *lev = reinterpret_cast<int32_t *>(smem + lay.lev);
+  // the first task_cap tasks staged in shared memory
+  uint2 *stask = reinterpret_cast<uint2 *>(smem + lay.total);
+  float4 *cpart = reinterpret_cast<float4 *>(stask + task_cap);         // [nint][cache_S]
   float4 *cpartlo = cpart + (FF ? (size_t)(maxnl / 2) * cache_S : 0);   // FF: lo parts
   int32_t *cexp = reinterpret_cast<int32_t *>(cpartlo + (size_t)(maxnl / 2) * cache_S);
   __shared__ double red_d[BS / 32];
   __shared__ long long red_e[BS / 32];
   __shared__ float2 spi[4];   // pi (FP32: .x only)
-  __shared__ float2 smu, skpa;
+  __shared__ float2 smu, skpa, stab[FF ? 64 : 1];
+  __shared__ HkyShared sH;
 
   const int tid = threadIdx.x;
   const bool full = (R.e[0] == -1);
   for (int k = tid; k < nl; k += BS) {
     T.nd[k] = P.nodes[R.node_off + k];
+    stm[k] = P.tff[R.node_off + k];
     T.slot[k] = P.slot32[R.node_off + k];
     T.dirty[k] = 0;
     T.fresh[k] = full ? 1 : 0;
@@ -346,18 +529,42 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
   for (int k = tid; k < 2 * n; k += BS) T.order[k] = P.sched[R.sched_off + k];
   const int nlev = P.nlev[R.item];
   T.lstart = T.order + nint;
-  if (tips) {
-    const int8_t *sq = P.seq + R.seq_off;
-    for (int k = tid; k < n * S; k += BS) stip[k] = sq[k];
-  }
+  const bool cls = S <= CLS_MAXS;
+  const uint2 *task = P.ctask + R.part_off / 2;
+  const int staged = cls ? (int)min((long long)task_cap, (long long)nint * S) : 0;
+  for (int k = tid; k < staged; k += BS) stask[k] = task[k];
+  if (cls)
+    for (int k = tid; k < n; k += BS) lev[k] = P.clev[R.sched_off + k];  // nlev + 1 <= n of them are meant
   if (tid == 0) {
+    // mu = u / (totsites standfactor): 2 kappa (pA pG + pC pT) + 2 (pA + pG)
+    // (pC + pT), in float-float (in FP64 one thread's fifty operations held up
+    // the CTA for some 3,000 cycles)
     const double *pid = P.pi + 4 * (size_t)R.item;
-    const double mu = R.u / ((double)R.totsites * standfactor(pid, R.par));
-    const double kp = R.par - 1.0;
-    smu = make_float2((float)mu, (float)(mu - (double)(float)mu));
-    skpa = make_float2((float)kp, (float)(kp - (double)(float)kp));
-    for (int j = 0; j < 4; j++) spi[j] = make_float2((float)pid[j], (float)(pid[j] - (double)(float)pid[j]));
+    ff pj[4];
+    for (int j = 0; j < 4; j++) {
+      pj[j] = ff_split(pid[j]);
+      spi[j] = make_float2(pj[j].hi, pj[j].lo);
+    }
+    const ff kap = ff_split(R.par);
+    ff sf = ff_mul(kap, ff_add(ff_mul(pj[0], pj[2]), ff_mul(pj[1], pj[3])));
+    sf = ff_add(sf, ff_mul(ff_add(pj[0], pj[2]), ff_add(pj[1], pj[3])));
+    const ff mu = ff_div(ff_split(R.u), ff_mul(ff_make(2.f * sf.hi, 2.f * sf.lo), ff_split((double)R.totsites)));
+    smu = make_float2(mu.hi, mu.lo);
+  } else if (tid == 32) {
+    const double *pid = P.pi + 4 * (size_t)R.item;
+    const ff PR = ff_add(ff_split(pid[0]), ff_split(pid[2])), PY = ff_add(ff_split(pid[1]), ff_split(pid[3]));
+    const ff kp = ff_add_f(ff_split(R.par), -1.0f), one = ff_from(1.0f);
+    auto put = [](ff v) { return make_float2(v.hi, v.lo); };
+    skpa = put(kp);
+    sH.AR = put(ff_add_f(ff_mul(PR, kp), 1.0f));
+    sH.AY = put(ff_add_f(ff_mul(PY, kp), 1.0f));
+    sH.iR = put(ff_div(one, PR));
+    sH.iY = put(ff_div(one, PY));
+    sH.oR = put(ff_add_f(ff_neg(PR), 1.0f));
+    sH.oY = put(ff_add_f(ff_neg(PY), 1.0f));
   }
+  if (FF)
+    for (int k = tid; k < 64; k += BS) stab[k] = d_exp64m1[k];
   __syncthreads();
   if (!full && tid == 0) {  // the reference's propagation rule, bottom-up
     for (int q = 0; q < 4; q++)
@@ -370,20 +577,20 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
     }
   }
   if (!full) __syncthreads();
-  const float2 *tff = P.tff + R.node_off;
   for (int c = tid; c < nl; c += BS) {
     int d = T.nd[c].down;
     if (d < 0 || !T.fresh[d]) continue;
     if constexpr (FF) {
       const ff pif[4] = {ff_of(spi[0]), ff_of(spi[1]), ff_of(spi[2]), ff_of(spi[3])};
       const int u = T.nd[c].up0;
-      const ff tc = ff_of(tff[c]);
-      const ff br = (u < 0) ? tc : ff_sub(tc, ff_of(tff[u]));
+      const ff tc = ff_of(stm[c]);
+      const ff br = (u < 0) ? tc : ff_sub(tc, ff_of(stm[u]));
       float Kc[10];
-      hky_coef_ff(pif, ff_of(skpa), ff_mul(ff_of(smu), br), Kc);
-      float *dst = Pm + PMS * c;
+      hky_coef_ff(sH, stab, ff_mul(ff_of(smu), br), Kc);
+      float *dst = c < n ? Pt + PT * c : Pi + PI * c;
       if (c < n) {
-        const HkyCoefFF K = load_coef_ff(Kc);
+        const HkyCoefFF K = {ff_make(Kc[0], Kc[1]), ff_make(Kc[2], Kc[3]), ff_make(Kc[4], Kc[5]), ff_make(Kc[6], Kc[7]),
+                             ff_make(Kc[8], Kc[9])};
 #pragma unroll
         for (int st = 0; st < 4; st++) {
           ff v[4];
@@ -397,7 +604,7 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
       }
     } else {
       float pil[4] = {spi[0].x, spi[1].x, spi[2].x, spi[3].x};
-      hky_coef_fast(pil, skpa.x, smu.x * branch_ff(T.nd, tff, c), Pm + PMS * c);
+      hky_coef_fast(pil, skpa.x, smu.x * branch_ff(T.nd, stm, c), c < n ? Pt + PT * c : Pi + PI * c);
     }
   }
   __syncthreads();
@@ -408,28 +615,27 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
   int32_t *pexp = P.pexp + R.part_off;
   const int8_t *seq = P.seq + R.seq_off;
   const float pi4[4] = {spi[0].x, spi[1].x, spi[2].x, spi[3].x};
-  // warps take (node, 32-pattern chunk) pairs of a level in turn, so a warp
-  // works on one node at a time and its children's coefficients stay in
-  // registers; lanes are patterns
-  constexpr int NW = BS / 32;
-  const int warp = tid >> 5, lane = tid & 31;
-  const int nch = (S + 31) >> 5;
-  // a warp's task q = jj * nch + chunk advances by NW: by NW / nch nodes and
-  // NW % nch chunks (no division in the loop)
-  const int jstep = NW / nch, cstep = NW - jstep * nch;
-  const int j0 = warp / nch, c0 = warp - j0 * nch;
+  // a level's tasks (one per node and class, or per node and pattern) are
+  // independent; the threads take them in turn
   for (int lv = 0; lv < nlev; lv++) {
-    const int beg = T.lstart[lv], total = (T.lstart[lv + 1] - beg) * nch;
-    int jj = j0, ch = c0;
-    for (int q = warp; q < total; q += NW, jj += jstep, ch += cstep) {
-      if (ch >= nch) {
-        ch -= nch;
-        jj++;
+    const int beg = cls ? lev[lv] : 0, end = cls ? lev[lv + 1] : (T.lstart[lv + 1] - T.lstart[lv]) * S;
+    for (int q = beg + tid; q < end; q += BS) {
+      int node, i, ic[2];
+      if (cls) {
+        const uint2 t = q < staged ? stask[q] : task[q];
+        node = n + (int)(t.x & 0xffffu);
+        i = (int)(t.x >> 16);
+        ic[0] = (int)(t.y & 0xffffu);
+        ic[1] = (int)(t.y >> 16);
+      } else {
+        node = T.order[T.lstart[lv] + q / S];
+        i = q % S;
       }
-      const int i = ch * 32 + lane;
-      const int node = T.order[beg + jj];
-      if (!T.fresh[node] || i >= S) continue;
-      const int cc[2] = {T.nd[node].up0, T.nd[node].up1};
+      if (!T.fresh[node]) continue;
+      const int2 ch = hky_children(T.nd[node], n);
+      const int cc[2] = {ch.x, ch.y};
+      if (!cls)
+        for (int h = 0; h < 2; h++) ic[h] = cc[h] < n ? seq[(size_t)cc[h] * S + i] : i;
       int e = 0;
       float4 ov, ol = make_float4(0.f, 0.f, 0.f, 0.f);
       if constexpr (FF) {
@@ -439,24 +645,23 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
         for (int h = 0; h < 2; h++) {
           const int c = cc[h];
           if (c < n) {
-            const int st = tips ? stip[c * S + i] : seq[(size_t)c * S + i];
-            const float4 *col = reinterpret_cast<const float4 *>(Pm + PMS * c) + 2 * st;
+            const float4 *col = reinterpret_cast<const float4 *>(Pt + PT * c) + 2 * ic[h];
             const float4 a = col[0], b = col[1];
             v[h][0] = ff_make(a.x, a.y);
             v[h][1] = ff_make(a.z, a.w);
             v[h][2] = ff_make(b.x, b.y);
             v[h][3] = ff_make(b.z, b.w);
           } else {
-            const HkyCoefFF K = load_coef_ff(Pm + PMS * c);
+            const HkyCoefFF K = load_coef_ff(Pi + PI * c);
             float4 hi, lo;
             if (CACHE && T.fresh[c]) {
-              const size_t ci = (size_t)(c - n) * cache_S + i;
+              const size_t ci = (size_t)(c - n) * cache_S + ic[h];
               hi = cpart[ci];
               lo = cpartlo[ci];
               e += cexp[ci];
             } else {
               const int rs = T.fresh[c] ? 1 - T.slot[c] : T.slot[c];
-              const size_t idx = rs * slot_stride + (size_t)(c - n) * S + i;
+              const size_t idx = rs * slot_stride + (size_t)(c - n) * S + ic[h];
               hi = part[idx];
               lo = partlo[idx];
               e += pexp[idx];
@@ -485,19 +690,19 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           const int c = cc[h];
-          const float *Kp = Pm + PMS * c;
+          const float *Kp = c < n ? Pt + PT * c : Pi + PI * c;
           const HkyCoef K = {Kp[0], Kp[1], Kp[2], Kp[3], Kp[4]};
           if (c < n) {
-            hky_apply_tip(K, pi4, tips ? stip[c * S + i] : seq[(size_t)c * S + i], v[h]);
+            hky_apply_tip(K, pi4, ic[h], v[h]);
           } else {
             float4 Lc;
             if (CACHE && T.fresh[c]) {
-              const size_t ci = (size_t)(c - n) * cache_S + i;
+              const size_t ci = (size_t)(c - n) * cache_S + ic[h];
               Lc = cpart[ci];
               e += cexp[ci];
             } else {
               const int rs = T.fresh[c] ? 1 - T.slot[c] : T.slot[c];
-              const size_t idx = rs * slot_stride + (size_t)(c - n) * S + i;
+              const size_t idx = rs * slot_stride + (size_t)(c - n) * S + ic[h];
               Lc = part[idx];
               e += pexp[idx];
             }
@@ -606,7 +811,7 @@ __global__ void __launch_bounds__(HKY_BS) k_hky_fp64(Pools P, const ReqDev *reqs
   const LocusDev L = P.loci[it.locus];
   const int n = it.n, nl = 2 * n - 1, S = L.nsites, nint = n - 1;
   const int nlev = P.nlev[R.item];
-  const HkyLayout lay = hky_layout(maxnl, sizeof(double));
+  const HkyLayout lay = hky_layout64(maxnl);
   double *Pm = reinterpret_cast<double *>(smem);  // [maxnl][16]
   Tree T;
   T.nd = reinterpret_cast<NodeRec *>(smem + lay.nd);
@@ -731,35 +936,45 @@ __global__ void k_hky_commit(Pools P, const int32_t *items, const uint8_t *accep
   }
 }
 
-size_t hky_smem(int maxn, size_t elem) { return hky_layout(2 * maxn - 1, elem).total; }
-
 }  // namespace
 
 // Partials stay in shared memory when the largest chain-locus of the batch
 // fits in this budget (keeps >= 3 CTAs per SM).
 constexpr size_t HKY_CACHE_BUDGET = 64 * 1024;
-constexpr size_t HKY_TIP_BUDGET = 8 * 1024;
+constexpr int HKY_TASK_CAP = 768;  // tasks staged in shared memory (6 KB)
 
 template <bool FF, int BS, int MINB>
 static void hky_fast_bs(const Pools &P, const ReqDev *reqs, int nreq, int maxnl, int maxS, bool cache_ok,
                         double *result, int32_t *status, cudaStream_t st)
 {
-  // tip states staged in shared memory when the largest locus's fit in
-  // HKY_TIP_BUDGET bytes (a few KB: occupancy is unchanged)
   const size_t maxn = (size_t)(maxnl + 1) / 2;
-  const int tip_cap = (maxn * maxS <= HKY_TIP_BUDGET) ? (int)(maxn * maxS) : 0;
-  size_t base = hky_smem((int)maxn, FF ? 2 * sizeof(float) : sizeof(float)) + (((size_t)tip_cap + 15) & ~size_t(15));
+  const int task_cap = (int)std::min((size_t)HKY_TASK_CAP, (maxn - 1) * maxS + 1) & ~1;
+  const size_t base = hky_layout_fast(maxnl, FF).total + task_cap * sizeof(uint2);
   size_t cache = (size_t)(maxnl / 2) * maxS * ((FF ? 2 : 1) * sizeof(float4) + sizeof(int32_t));
   if (cache_ok && cache <= HKY_CACHE_BUDGET) {
     size_t sm = base + cache;
     if (sm > 48 * 1024)
       cudaFuncSetAttribute(k_hky_fast<FF, true, BS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_hky_fast<FF, true, BS, MINB><<<nreq, BS, sm, st>>>(P, reqs, result, status, maxnl, maxS, tip_cap);
+    k_hky_fast<FF, true, BS, MINB><<<nreq, BS, sm, st>>>(P, reqs, result, status, maxnl, maxS, task_cap);
   } else {
     if (base > 48 * 1024)
       cudaFuncSetAttribute(k_hky_fast<FF, false, BS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)base);
-    k_hky_fast<FF, false, BS, MINB><<<nreq, BS, base, st>>>(P, reqs, result, status, maxnl, 0, tip_cap);
+    k_hky_fast<FF, false, BS, MINB><<<nreq, BS, base, st>>>(P, reqs, result, status, maxnl, 0, task_cap);
   }
+}
+
+void launch_hky_classes(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, cudaStream_t st)
+{
+  if (nreq <= 0) return;
+  const int maxnl = 2 * maxn - 1, S = std::min(maxS, CLS_MAXS);
+  int logh = 6;
+  while ((1 << logh) < 2 * S) logh++;
+  const size_t hash = ((sizeof(NodeRec) * maxnl + 2 * (maxnl + 3) + 15) & ~size_t(15)) + CLS_WARPS * 6ul * (1ul << logh);
+  size_t sm = hash;
+  const size_t all = 2ul * (maxn - 1) * S;
+  if (all <= CLS_SHARED) sm += all;
+  if (sm > 48 * 1024) cudaFuncSetAttribute(k_hky_classes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_hky_classes<<<nreq, 32 * CLS_WARPS, sm, st>>>(P, reqs, maxnl, logh, all <= CLS_SHARED ? (int)(all / 2) : 0);
 }
 
 void launch_hky_fast(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, int variant,
@@ -804,14 +1019,22 @@ int hky_init_tables()
   const double a = 355.0 / 512.0;
   K.ln2a = make_float2((float)a, (float)(ln2 - a));
   K.ln2b = (float)(ln2 - a - (double)(float)(ln2 - a));
-  return cudaMemcpyToSymbol(c_ffh, &K, sizeof(K)) == cudaSuccess ? 0 : -1;
+  float2 t[64];
+  for (int j = 0; j < 64; j++) {
+    const double v = std::expm1((j - 32) * (0.69314718055994530942 / 64));
+    t[j] = make_float2((float)v, (float)(v - (double)(float)v));
+  }
+  return cudaMemcpyToSymbol(c_ffh, &K, sizeof(K)) == cudaSuccess &&
+                 cudaMemcpyToSymbol(d_exp64m1, t, sizeof(t)) == cudaSuccess
+             ? 0
+             : -1;
 }
 
 void launch_hky_fp64(const Pools &P, const ReqDev *reqs, int nreq, int maxn, double *result,
                      int32_t *status, cudaStream_t st)
 {
   if (nreq <= 0) return;
-  size_t sm = hky_smem(maxn, sizeof(double));
+  size_t sm = hky_layout64(2 * maxn - 1).total;
   if (sm > 48 * 1024)
     cudaFuncSetAttribute(k_hky_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   k_hky_fp64<<<nreq, HKY_BS, sm, st>>>(P, reqs, result, status, 2 * maxn - 1);

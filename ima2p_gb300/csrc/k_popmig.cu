@@ -128,15 +128,6 @@ struct PfGen {
   int na;                             // a, or 0: not for the fast form
 };
 
-__device__ __forceinline__ ff ff_split(double z)  // a positive double as float-float, truncated, on the integer pipe
-{
-  const int hi = __double2hiint(z), lo = __double2loint(z);
-  const uint32_t u = __funnelshift_l((uint32_t)lo, (uint32_t)hi, 3) - 0xC0000000u;
-  const int se = (int)(u >> 23) - 52;
-  const float l = (float)(lo & 0x1fffffff) * __int_as_float(max(se, 0) << 23);
-  return ff_make(__uint_as_float(u), l);
-}
-
 // S(x) / a or H(x) with n terms
 __device__ __forceinline__ ff pf_value(ff x, bool series, int na, int n, const float2 *rcp)
 {

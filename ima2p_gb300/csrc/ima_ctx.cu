@@ -38,8 +38,15 @@ struct LocusHost {
   bool sumlogk_done = false;
 };
 
+// HKY requests of similar size, launched together (a launch's shared memory
+// is that of its largest chain-locus)
+struct HkyBin {
+  int off, n, maxn, maxs;
+};
+
 struct Batch {
   bool live = false;
+  std::vector<HkyBin> bins;
   int n = 0, nis = 0, nhky = 0, nsw = 0, prec = IMA_PREC_FAST;
   std::vector<int> order;  // grouped position -> caller index
   ReqDev *d_req = nullptr;
@@ -60,7 +67,6 @@ struct Batch {
   int hky_variant = 0, sw_variant = 0;  // launch shapes (ima_gpu_batch_autotune)
   // MC3 sweep of the batch (ima_gpu_batch_sweep): its items and accept mask
   // on the device, and the graph of evaluation, commit and swaps
-  long long cls_gen = -1;  // ima_ctx::cls_gen when the pattern classes of its items were last brought up to date
   int32_t *d_items = nullptr;
   uint8_t *d_acc = nullptr;
   cudaGraphExec_t sgraph = nullptr;
@@ -260,12 +266,9 @@ struct ima_ctx {
   unsigned long long *d_ctr = nullptr;
   int32_t *d_is_site = nullptr;  // IS per-site mutation branches, valid while the topology is
   uint8_t *d_is_valid = nullptr;
-  // HKY pattern classes, allocated on first use; cls_gen counts the changes
-  // of topology, a batch remembers the count its items' classes match
-  uint2 *d_ctask = nullptr;
-  uint16_t *d_crep = nullptr;
-  int32_t *d_clev = nullptr;
-  long long cls_gen = 0;
+  uint32_t *d_planes = nullptr;  // HKY tips' states as bit planes
+  uint2 *d_task = nullptr;       // HKY task lists, allocated on first use
+  int32_t *d_toff = nullptr;
   double *d_uni = nullptr;
   size_t uni_cap = 0;
 
@@ -394,9 +397,9 @@ struct ima_ctx {
     P.sumlogk = d_sumlogk;
     P.is_site = d_is_site;
     P.is_valid = d_is_valid;
-    P.ctask = d_ctask;
-    P.crep = d_crep;
-    P.clev = d_clev;
+    P.planes = d_planes;
+    P.task = d_task;
+    P.toff = d_toff;
     P.pdg_new = d_pdg_new;
     P.part = d_part;
     P.partlo = d_partlo;
@@ -517,7 +520,7 @@ extern "C" void ima_gpu_destroy(ima_ctx *c)
                   c->d_pop, c->d_moff, c->d_inode_off, c->d_gl, c->d_gt, c->d_moff_start, c->d_bcnt, c->d_bicnt,
                   c->d_mig_p, c->d_rsamp, c->d_mbase, c->d_mig_t, c->d_tvr, c->d_len_hold, c->d_rhlog,
                   c->d_rh2, c->d_rsel, c->d_is_site, c->d_is_valid, c->d_lterm, c->d_ug,
-                  c->d_ctask, c->d_crep, c->d_clev};
+                  c->d_planes, c->d_task, c->d_toff};
   for (void *p : devs)
     if (p) cudaFree(p);
   void *hosts[] = {c->h_nodes, c->h_t64, c->h_sched, c->h_nlev, c->h_len, c->h_pi, c->h_al};
@@ -607,12 +610,25 @@ extern "C" int ima_gpu_set_chains(ima_ctx *c, int nruns, int chains_per_run)
   // locus tables
   std::vector<int8_t> seq;
   std::vector<int32_t> mult;
+  std::vector<uint32_t> planes;
   std::vector<LocusDev> ld;
   for (auto &L : c->loci) {
     L.d.seq_off = (int)seq.size();
     L.d.mult_off = (int)mult.size();
     seq.insert(seq.end(), L.seq.begin(), L.seq.end());
     mult.insert(mult.end(), L.mult.begin(), L.mult.end());
+    L.d.plane_off = (int)planes.size();
+    if (L.d.model == IMA_MODEL_HKY) {
+      const size_t W = ((size_t)L.d.nsites + 31) / 32;
+      planes.resize(planes.size() + 2 * W * L.d.n, 0u);
+      uint32_t *q = planes.data() + L.d.plane_off;
+      for (int t = 0; t < L.d.n; t++)
+        for (int k = 0; k < L.d.nsites; k++) {
+          const int x = L.seq[(size_t)t * L.d.nsites + k];
+          q[2 * W * t + k / 32] |= (uint32_t)(x & 1) << (k & 31);
+          q[2 * W * t + W + k / 32] |= (uint32_t)(x >> 1) << (k & 31);
+        }
+    }
     ld.push_back(L.d);
   }
   // placement of every chain-locus
@@ -637,7 +653,7 @@ extern "C" int ima_gpu_set_chains(ima_ctx *c, int nruns, int chains_per_run)
       sched += 2 * L.n + 2;
       if (L.model == IMA_MODEL_SW) al += (size_t)L.nlinked * nl;
       if (L.model == IMA_MODEL_HKY) {
-        part += 2 * (size_t)(L.n - 1) * L.nsites;
+        part += 2 * (size_t)(L.n - 1) * (L.nsites + 4);
         part64 += 2 * (size_t)(L.n - 1) * L.nsites;
       }
     }
@@ -652,6 +668,7 @@ extern "C" int ima_gpu_set_chains(ima_ctx *c, int nruns, int chains_per_run)
   c->d_loci = dev_alloc<LocusDev>(ld.size(), B, c->st);
   c->d_seq = dev_alloc<int8_t>(seq.size(), B, c->st);
   c->d_mult = dev_alloc<int32_t>(mult.size(), B, c->st);
+  c->d_planes = dev_alloc<uint32_t>(planes.size(), B, c->st);
   c->d_sumlogk = dev_alloc<double>(c->nloci, B, c->st);
   c->d_items = dev_alloc<ItemDev>(c->nitems, B, c->st);
   c->d_nodes = dev_alloc<NodeRec>(nodes, B, c->st);
@@ -684,7 +701,7 @@ extern "C" int ima_gpu_set_chains(ima_ctx *c, int nruns, int chains_per_run)
                  c->d_tff, c->d_slot32, c->d_fresh32, c->d_sched, c->d_nlev, c->d_len, c->d_pi,
                  c->d_al, c->d_dlike, c->d_part, c->d_pexp, c->d_pdg, c->d_pdg_new, c->d_beta,
                  c->d_allbetas, c->d_probg, c->d_S, c->d_swapcount, c->d_tempcount, c->d_used,
-                 c->d_swap0ok, c->d_ctr, c->d_is_site, c->d_is_valid};
+                 c->d_swap0ok, c->d_ctr, c->d_is_site, c->d_is_valid, c->d_planes};
   for (void *p : chk)
     if (!p) return c->fail(IMA_ERR_NOMEM, "device allocation failed (%zu bytes so far)", B);
   if (int r0 = c->cuda(cudaMemsetAsync(c->d_is_valid, 0, c->nitems, c->st), "IS site cache")) return r0;
@@ -705,6 +722,7 @@ extern "C" int ima_gpu_set_chains(ima_ctx *c, int nruns, int chains_per_run)
   r = r ? r : c->cuda(cudaMemcpyAsync(c->d_loci, ld.data(), ld.size() * sizeof(LocusDev), cudaMemcpyHostToDevice, c->st), "loci");
   if (!seq.empty()) r = r ? r : c->cuda(cudaMemcpyAsync(c->d_seq, seq.data(), seq.size(), cudaMemcpyHostToDevice, c->st), "seq");
   if (!mult.empty()) r = r ? r : c->cuda(cudaMemcpyAsync(c->d_mult, mult.data(), mult.size() * 4, cudaMemcpyHostToDevice, c->st), "mult");
+  if (!planes.empty()) r = r ? r : c->cuda(cudaMemcpyAsync(c->d_planes, planes.data(), planes.size() * 4, cudaMemcpyHostToDevice, c->st), "planes");
   r = r ? r : c->cuda(cudaMemcpyAsync(c->d_items, c->items.data(), c->items.size() * sizeof(ItemDev), cudaMemcpyHostToDevice, c->st), "items");
   r = r ? r : c->cuda(cudaMemcpyAsync(c->d_pi, c->h_pi, 4 * sizeof(double) * c->nitems, cudaMemcpyHostToDevice, c->st), "pi");
   // the host vectors above are about to go out of scope
@@ -1406,7 +1424,6 @@ static int flush(ima_ctx *c)
   r = r ? r : c->cuda(cudaMemcpyAsync(c->d_pi + 4 * (size_t)lo, c->h_pi + 4 * (size_t)lo, 4 * (hi - lo + 1) * sizeof(double), cudaMemcpyHostToDevice, st), "pi");
   if (a1 > a0) r = r ? r : c->cuda(cudaMemcpyAsync(c->d_al + a0, c->h_al + a0, (a1 - a0) * sizeof(int32_t), cudaMemcpyHostToDevice, st), "alleles");
   // topologies may have changed: the caches of the range are stale
-  c->cls_gen++;
   r = r ? r : c->cuda(cudaMemsetAsync(c->d_is_valid + lo, 0, hi - lo + 1, st), "IS site cache");
   c->dirty_lo = INT32_MAX;
   c->dirty_hi = -1;
@@ -1449,36 +1466,6 @@ static int ensure_ff_hky(ima_ctx *c)
   return c->cuda(cudaMemsetAsync(c->d_partlo, 0, c->npart * sizeof(float4), c->st), "float-float partials");
 }
 
-static int ensure_classes_alloc(ima_ctx *c)
-{
-  if (c->d_ctask || c->npart == 0) return IMA_OK;
-  c->d_ctask = dev_alloc<uint2>(c->npart / 2, c->dev_bytes, c->st);
-  c->d_crep = dev_alloc<uint16_t>(c->npart / 2, c->dev_bytes, c->st);
-  c->d_clev = dev_alloc<int32_t>(c->nsched, c->dev_bytes, c->st);
-  if (!c->d_ctask || !c->d_crep || !c->d_clev) {
-    cudaFree(c->d_ctask);
-    cudaFree(c->d_crep);
-    cudaFree(c->d_clev);
-    c->d_ctask = nullptr;
-    c->d_crep = nullptr;
-    c->d_clev = nullptr;
-    return c->fail(IMA_ERR_NOMEM, "HKY pattern classes (%zu tasks) do not fit", c->npart / 2);
-  }
-  return IMA_OK;
-}
-
-// The pattern classes of a batch's HKY items, after its flush and before its
-// kernels (or their graph) run
-static int ensure_classes(ima_ctx *c, Batch &b)
-{
-  if (!b.nhky || b.prec == IMA_PREC_FP64 || b.cls_gen == c->cls_gen) return IMA_OK;
-  if (int r = ensure_classes_alloc(c)) return r;
-  launch_hky_classes(c->pools(), b.d_req + b.nis, b.nhky, b.maxn_hky, b.maxs_hky, c->st);
-  c->launches++;
-  b.cls_gen = c->cls_gen;
-  return c->cuda(cudaGetLastError(), "pattern classes");
-}
-
 static double hky_bytes(ima_ctx *c, const Batch &b);
 static double sw_bytes(ima_ctx *c, const Batch &b);
 
@@ -1510,17 +1497,37 @@ static int build_batch(ima_ctx *c, Batch &b, int n, const int32_t *ci, const int
     const LocusDev &L = c->loci[li[k]].d;
     return L.model == IMA_MODEL_HKY ? (long long)(L.n - 1) * L.nsites : (long long)L.n;
   };
+  // (HKY: inside classes of 32 genes, the largest class first)
+  auto size = [&](int k) {
+    const LocusDev &L = c->loci[li[k]].d;
+    return L.model == IMA_MODEL_HKY ? (L.n + 31) / 32 : 0;
+  };
   for (int m = 1; m < 3; m++)
-    std::stable_sort(g[m].begin(), g[m].end(), [&](int a, int b) { return cost(a) > cost(b); });
+    std::stable_sort(g[m].begin(), g[m].end(), [&](int a, int b) {
+      const int sa = size(a), sb = size(b);
+      return sa != sb ? sa > sb : cost(a) > cost(b);
+    });
+  // a launch per class, where it and the rest fill the device a few times
+  b.bins.clear();
+  for (size_t k = 0; k < g[1].size(); k++) {
+    const LocusDev &L = c->loci[li[g[1][k]]].d;
+    if (k == 0 || (size(g[1][k]) != size(g[1][k - 1]) && b.bins.back().n >= 8 * c->nsm &&
+                   (int)(g[1].size() - k) >= 8 * c->nsm))
+      b.bins.push_back({(int)k, 0, 0, 0});
+    HkyBin &q = b.bins.back();
+    q.n++;
+    q.maxn = std::max(q.maxn, L.n);
+    q.maxs = std::max(q.maxs, L.nsites);
+  }
   b.n = n;
   b.prec = prec;
-  b.cls_gen = -1;
   b.nis = (int)g[0].size();
   b.nhky = (int)g[1].size();
   b.nsw = (int)g[2].size();
-  // fewer HKY chain-loci than SMs: each runs alone on its SM, so the
-  // widest CTA (256 threads) shortens the level chain
-  b.hky_variant = (b.nhky > 0 && b.nhky < c->nsm) ? 2 : 0;
+  // float-float HKY: 128-thread CTAs, 6 per SM, unless the batch is one wave
+  // of the 96-thread shape's 11 and more than one of 6 (1,600 chain-loci of 40
+  // genes: 41 us against 46; 12,800 of 12 to 180 genes: 861 against 741)
+  b.hky_variant = (prec == IMA_PREC_FAST && b.nhky > 6 * c->nsm && b.nhky <= 11 * c->nsm) ? 5 : 0;
   b.order.clear();
   b.h_req.clear();
   b.maxn_is = b.maxs_is = b.maxn_hky = b.maxs_hky = b.maxn_sw = 0;
@@ -1541,7 +1548,7 @@ static int build_batch(ima_ctx *c, Batch &b, int n, const int32_t *ci, const int
         r.totsites = Ld.totsites;
         r.seq_off = Ld.seq_off;
         r.mult_off = Ld.mult_off;
-        r.pad = 0;
+        r.plane_off = Ld.plane_off;
       }
       r.u = u[k];
       r.par = kappa ? kappa[k] : 1.0;
@@ -1559,6 +1566,11 @@ static int build_batch(ima_ctx *c, Batch &b, int n, const int32_t *ci, const int
   if (b.nhky && prec == IMA_PREC_FAST) {
     int r = ensure_ff_hky(c);
     if (r) return r;
+  }
+  if (b.nhky && prec != IMA_PREC_FP64 && !c->d_task) {
+    c->d_toff = c->d_toff ? c->d_toff : dev_alloc<int32_t>(c->nsched, c->dev_bytes, c->st);
+    c->d_task = c->d_toff ? dev_alloc<uint2>(c->npart / 2, c->dev_bytes, c->st) : nullptr;
+    if (!c->d_task) return c->fail(IMA_ERR_NOMEM, "HKY tasks (%zu) do not fit", c->npart / 2);
   }
   if (!c->d_slot64 && b.nhky) {
     // the commit kernel touches both slot sets; keep the FP64 marks allocated
@@ -1636,7 +1648,15 @@ static double sw_bytes(ima_ctx *c, const Batch &b)
   return s;
 }
 
-// kernels of a batch (no host work, graph-capturable once sumlogk is set)
+static void hky_bins(const Pools &P, const Batch &b, int variant, cudaStream_t st)
+{
+  for (const HkyBin &q : b.bins) {
+    const int o = b.nis + q.off;
+    if (b.prec == IMA_PREC_FP32) launch_hky_fp32(P, b.d_req + o, q.n, q.maxn, q.maxs, variant, b.d_res + o, b.d_st + o, st);
+    else launch_hky_fast(P, b.d_req + o, q.n, q.maxn, q.maxs, variant, b.d_res + o, b.d_st + o, st);
+  }
+}
+
 // kernels of a batch (no host work, graph-capturable once sumlogk is set)
 static void enqueue(ima_ctx *c, Batch &b, cudaStream_t on = nullptr)
 {
@@ -1648,10 +1668,8 @@ static void enqueue(ima_ctx *c, Batch &b, cudaStream_t on = nullptr)
     const ReqDev *r = b.d_req + b.nis;
     if (b.prec == IMA_PREC_FP64)
       c->launch(IMA_K_HKY_FP64, b.hky_bytes, [&] { launch_hky_fp64(P, r, b.nhky, b.maxn_hky, b.d_res + b.nis, b.d_st + b.nis, st); }, st);
-    else if (b.prec == IMA_PREC_FP32)
-      c->launch(IMA_K_HKY_FP32, b.hky_bytes, [&] { launch_hky_fp32(P, r, b.nhky, b.maxn_hky, b.maxs_hky, b.hky_variant, b.d_res + b.nis, b.d_st + b.nis, st); }, st);
     else
-      c->launch(IMA_K_HKY_FAST, b.hky_bytes, [&] { launch_hky_fast(P, r, b.nhky, b.maxn_hky, b.maxs_hky, b.hky_variant, b.d_res + b.nis, b.d_st + b.nis, st); }, st);
+      c->launch(b.prec == IMA_PREC_FP32 ? IMA_K_HKY_FP32 : IMA_K_HKY_FAST, b.hky_bytes, [&] { hky_bins(P, b, b.hky_variant, st); }, st);
   }
   if (b.nsw) {
     const ReqDev *r = b.d_req + b.nis + b.nhky;
@@ -1789,7 +1807,6 @@ extern "C" int ima_gpu_eval(ima_ctx *c, int n, const int32_t *ci, const int32_t 
   r = r ? r : flush(c);
   r = r ? r : (b.nis ? ensure_lengths(c) : IMA_OK);  // the infinite-sites likelihood reads them
   r = r ? r : init_sumlogk(c, b);
-  r = r ? r : ensure_classes(c, b);
   if (!r) enqueue(c, b);
   r = r ? r : c->cuda(cudaGetLastError(), "launch");
   r = r ? r : fetch(c, b, result, status);
@@ -1845,7 +1862,6 @@ extern "C" int ima_gpu_batch_run(ima_ctx *c, int batch, int use_graph)
   int r = flush(c);
   r = r ? r : (b.nis ? ensure_lengths(c) : IMA_OK);  // the infinite-sites likelihood reads them
   r = r ? r : init_sumlogk(c, b);
-  r = r ? r : ensure_classes(c, b);
   if (r) return r;
   if (!use_graph || c->profiling) {
     enqueue(c, b);
@@ -1881,7 +1897,6 @@ extern "C" int ima_gpu_batch_autotune(ima_ctx *c, int batch, int reps, int *hky_
   int r = flush(c);
   r = r ? r : (b.nis ? ensure_lengths(c) : IMA_OK);  // the infinite-sites likelihood reads them
   r = r ? r : init_sumlogk(c, b);
-  r = r ? r : ensure_classes(c, b);
   if (r) return r;
   if (reps < 1) reps = 1;
   if (b.prec != IMA_PREC_FP64 && (b.nhky || b.nsw)) {
@@ -1907,13 +1922,7 @@ extern "C" int ima_gpu_batch_autotune(ima_ctx *c, int batch, int reps, int *hky_
       return (t[0] >= 0.f && t[0] <= 1.02f * t[best]) ? 0 : best;
     };
     if (b.nhky) {
-      const ReqDev *rq = b.d_req + b.nis;
-      b.hky_variant = pick(HKY_FAST_VARIANTS, [&](int v) {
-        if (b.prec == IMA_PREC_FP32)
-          launch_hky_fp32(P, rq, b.nhky, b.maxn_hky, b.maxs_hky, v, b.d_res + b.nis, b.d_st + b.nis, st);
-        else
-          launch_hky_fast(P, rq, b.nhky, b.maxn_hky, b.maxs_hky, v, b.d_res + b.nis, b.d_st + b.nis, st);
-      });
+      b.hky_variant = pick(HKY_FAST_VARIANTS, [&](int v) { hky_bins(P, b, v, st); });
     }
     if (b.nsw) {
       const ReqDev *rq = b.d_req + b.nis + b.nhky;
@@ -2022,7 +2031,6 @@ extern "C" int ima_gpu_batch_sweep(ima_ctx *c, int batch, const uint8_t *accept,
   int r = flush(c);
   r = r ? r : (b.nis ? ensure_lengths(c) : IMA_OK);  // the infinite-sites likelihood reads them
   r = r ? r : init_sumlogk(c, b);
-  r = r ? r : ensure_classes(c, b);
   if (r) return r;
   if (!b.d_items) {
     std::vector<int32_t> items(b.n);
@@ -4526,10 +4534,6 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
           c->launch(IMA_K_UG, 0.0, [&] { launch_ug_sw(u_, sh); }, sh);
         } else {
           if (!u_.hky) cudaStreamWaitEvent(sh, evW[slot], 0);  // the IS likelihood reads the new lengths
-          if (u_.hky && precision != IMA_PREC_FP64) {  // the proposals changed the topologies
-            launch_hky_classes(c->pools(), b.d_req, b.nhky, b.maxn_hky, b.maxs_hky, sh);
-            c->launches++;
-          }
           enqueue(c, b, sh);
         }
         cudaEventRecord(evH[slot], sh);
@@ -4542,7 +4546,6 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
     }
   if (step > 0) cudaStreamWaitEvent(c->st, evD[(step - 1) % R], 0);  // st carries on after the last decision
   // the device's genealogies are newer than the mirror from here on
-  c->cls_gen++;
   for (int k = 0; k < nch; k++) {
     c->topo_lo = std::min(c->topo_lo, chains[k] * nl);
     c->topo_hi = std::max(c->topo_hi, chains[k] * nl + nl - 1);

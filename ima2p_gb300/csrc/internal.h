@@ -23,7 +23,7 @@ struct LocusDev {
   int nlinked;    // SW: linked markers
   int seq_off;    // int8 [n][nsites] in the seq pool
   int mult_off;   // int32 [nsites] in the mult pool
-  int pad;
+  int plane_off;  // HKY: uint32 [n][2][ceil(nsites / 32)] bit planes of the states
 };
 
 // Static placement of one chain-locus in the resident pools.
@@ -32,7 +32,7 @@ struct ItemDev {
   int n;
   int node_off;            // nodes / times / slot / fresh pools
   int sched_off;           // int16 [2n] level schedule
-  long long part_off;      // HKY: float4 index of slot 0 (slot 1 at + (n-1)*S)
+  long long part_off;      // HKY: float4 index of slot 0 (slot 1 at + (n-1)*(S+4))
   long long part64_off;    // HKY FP64: double index (x4 per pattern) of slot 0
   int al_off;              // SW: int32 [nlinked][2n-1] alleles
   int dl_off;              // SW: double [nlinked][2n-1] dlikeA
@@ -50,7 +50,7 @@ struct ReqDev {
   // request is built, so a kernel's first load brings them (the HKY kernel
   // otherwise chains request -> item -> locus before its tree loads)
   long long part_off;
-  int node_off, sched_off, n, nsites, totsites, seq_off, mult_off, pad;
+  int node_off, sched_off, n, nsites, totsites, seq_off, mult_off, plane_off;
 };
 
 // Everything a kernel may read; passed by value.
@@ -71,12 +71,10 @@ struct Pools {
   double *sumlogk;          // IS per-locus constant
   int32_t *is_site;         // IS: per item and site, (mutation node << 8) | branch (0 first daughter,
                             // 1 second, 2 both at the root); node -1 none, -2 two
-  uint8_t *is_valid;        // the item's cache (IS: sites; HKY: pattern classes) matches its topology
-  // HKY pattern classes (k_hky_classes), per item at part_off / 2: tasks and
-  // representatives; task starts per level at sched_off
-  uint2 *ctask;
-  uint16_t *crep;
-  int32_t *clev;
+  uint8_t *is_valid;        // the item's cache (IS: sites; HKY: the task list of a full evaluation) matches its topology
+  const uint32_t *planes;   // HKY: per locus and tip the two bit planes of its states, [n][2][ceil(S / 32)]
+  uint2 *task;              // HKY: an item's task list at part_off / 2
+  int32_t *toff;            // HKY: at sched_off, tasks before each node of the schedule, and their number
   double *pdg_new;          // last evaluated log P(D|G) per item
   // HKY state
   float4 *part;             // FP32 partials (float-float form: the hi parts)
@@ -93,16 +91,13 @@ void launch_is_sumlogk(const Pools &P, int item, int locus, int maxn, int maxS, 
 void launch_is(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, double *result,
                int32_t *status, int32_t *site_node, cudaStream_t st);
 // variant: launch shape chosen by the batch autotuner (0 is the default)
-constexpr int HKY_FAST_VARIANTS = 6;  // float-float: 128 threads with registers for 8 CTAs per SM, 64 threads
-                                      // (16 CTAs), 256 (4), 128 at 10 CTAs, 128 at 6, 96 at 11;
-                                      // FP32: 128 threads (12 CTAs per SM), 64, 256, 128 uncached, 128 at 8,
+constexpr int HKY_FAST_VARIANTS = 6;  // float-float: 128 threads with registers for 6 CTAs per SM, 64 threads
+                                      // (16 CTAs), 256 (4), 128 at 10 CTAs, 128 at 8, 96 at 11;
+                                      // FP32: 128 threads (12 CTAs per SM), 64, 256, 128 at 6, 128 at 8,
                                       // 96 at 16
 constexpr int SW_FAST_VARIANTS = 3;   // one wave (5 or 6 CTAs per SM), 8 chain-loci per CTA
 void launch_hky_fast(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, int variant,
                      double *result, int32_t *status, cudaStream_t st);
-// the pattern classes of the requests' items whose cache is stale (before
-// launch_hky_fast and launch_hky_fp32, after every change of topology)
-void launch_hky_classes(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, cudaStream_t st);
 void launch_hky_fp32(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, int variant,
                      double *result, int32_t *status, cudaStream_t st);
 void launch_hky_fp64(const Pools &P, const ReqDev *reqs, int nreq, int maxn, double *result,

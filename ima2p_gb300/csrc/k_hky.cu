@@ -203,208 +203,170 @@ __device__ __forceinline__ ff ff_fma_pos(ff a, ff b, ff c)
   return fast_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(pe, c.lo)));
 }
 
-struct HkyCoefFF {
-  ff a, bR, bY, dR, dY;
+// Two float-floats at once, in the packed FP32 instructions: states are
+// taken as the pairs (A, C) and (G, T), so that a pair holds one purine and
+// one pyrimidine and the two classes' sums and coefficients are pairs too.
+// A packed instruction takes one issue slot for two results (measured 105-119
+// results per cycle and SM against 83 of the scalar ones).
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2_pack(float x, float y)
+{
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 f2_un(f2 a)
+{
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b)
+{
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b)
+{
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c)
+{
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 f2_neg(f2 a) { return a ^ 0x8000000080000000ull; }
+__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) { return f2_add(a, f2_neg(b)); }
+struct ff2 {
+  f2 hi, lo;
 };
-__device__ __forceinline__ HkyCoefFF load_coef_ff(const float *Kp)  // 16-byte aligned
+__device__ __forceinline__ ff2 ff2_make(f2 h, f2 l)
 {
-  const float4 a = reinterpret_cast<const float4 *>(Kp)[0], b = reinterpret_cast<const float4 *>(Kp)[1];
-  const float2 c = reinterpret_cast<const float2 *>(Kp)[4];
-  HkyCoefFF K;
-  K.a = ff_make(a.x, a.y);
-  K.bR = ff_make(a.z, a.w);
-  K.bY = ff_make(b.x, b.y);
-  K.dR = ff_make(b.z, b.w);
-  K.dY = ff_make(c.x, c.y);
-  return K;
+  ff2 r;
+  r.hi = h;
+  r.lo = l;
+  return r;
 }
-// P(b) applied to a tip observed in state st: column st of P(b)
-__device__ __forceinline__ void hky_apply_tip_ff(const HkyCoefFF &K, const ff *pi, int st, ff *v)
+// a b and a b + c, every operand >= 0, left unnormalised (|lo| may reach a few
+// ulp(hi)): the next step's TwoSum is exact whatever lo is
+__device__ __forceinline__ ff2 ff2_mul_u(ff2 a, ff2 b)
 {
-  const ff p = st == 0 ? pi[0] : st == 1 ? pi[1] : st == 2 ? pi[2] : pi[3];
+  const f2 p = f2_mul(a.hi, b.hi);
+  return ff2_make(p, f2_fma(a.hi, b.lo, f2_fma(a.lo, b.hi, f2_fma(a.hi, b.hi, f2_neg(p)))));
+}
+__device__ __forceinline__ ff2 ff2_fma_u(ff2 a, ff2 b, ff2 c)
+{
+  const ff2 p = ff2_mul_u(a, b);
+  const f2 s = f2_add(p.hi, c.hi), bb = f2_sub(s, p.hi);
+  const f2 e = f2_add(f2_sub(p.hi, f2_sub(s, bb)), f2_sub(c.hi, bb));
+  return ff2_make(s, f2_add(e, f2_add(p.lo, c.lo)));
+}
+// the product renormalised; of unnormalised factors, so lo x lo counts
+__device__ __forceinline__ ff2 ff2_mul(ff2 a, ff2 b)
+{
+  const f2 p = f2_mul(a.hi, b.hi);
+  const f2 e = f2_fma(a.hi, b.lo, f2_fma(a.lo, b.hi, f2_fma(a.lo, b.lo, f2_fma(a.hi, b.hi, f2_neg(p)))));
+  const f2 s = f2_add(p, e);
+  return ff2_make(s, f2_sub(e, f2_sub(s, p)));
+}
+__device__ __forceinline__ void ff2_load(const float4 &hi, const float4 &lo, ff2 *v)
+{
+  v[0] = ff2_make(f2_pack(hi.x, hi.y), f2_pack(lo.x, lo.y));
+  v[1] = ff2_make(f2_pack(hi.z, hi.w), f2_pack(lo.z, lo.w));
+}
+
+// An internal branch's coefficients as pairs: (E1, E1), (b_R, b_Y), (d_R,
+// d_Y), hi parts then lo parts (12 floats).  v_j = E1 S_o + b_c S_c + d_c L_j,
+// left unnormalised: its only use is the product of the two daughters.
+__device__ __forceinline__ void hky_apply_ff(const float *K, const ff2 *pi, const ff2 *L, ff2 *v)
+{
+  const float4 k0 = reinterpret_cast<const float4 *>(K)[0], k1 = reinterpret_cast<const float4 *>(K)[1],
+               k2 = reinterpret_cast<const float4 *>(K)[2];
+  const ff2 a = ff2_make(f2_pack(k0.x, k0.y), f2_pack(k1.z, k1.w)), b = ff2_make(f2_pack(k0.z, k0.w), f2_pack(k2.x, k2.y)),
+            d = ff2_make(f2_pack(k1.x, k1.y), f2_pack(k2.z, k2.w));
+  const ff2 S = ff2_fma_u(pi[1], L[1], ff2_mul_u(pi[0], L[0]));  // (S_R, S_Y)
+  const float2 sh = f2_un(S.hi), sl = f2_un(S.lo);
+  const ff2 O = ff2_make(f2_pack(sh.y, sh.x), f2_pack(sl.y, sl.x));
+  const ff2 t = ff2_fma_u(b, S, ff2_mul_u(a, O));
+  v[0] = ff2_fma_u(d, L[0], t);
+  v[1] = ff2_fma_u(d, L[1], t);
+}
+
+// P(b) applied to a tip observed in state st: column st of P(b), (b_R, E1) or
+// (E1, b_Y) times pi_st, and d of its class added at st itself.  (Columns made
+// once per branch took 144 bytes of shared memory a tip, which cost more
+// resident CTAs than these thirty instructions do.)
+__device__ __forceinline__ void hky_apply_tip_ff(const float *K, float2 p, int st, ff2 *v)
+{
+  const float4 k0 = reinterpret_cast<const float4 *>(K)[0], k1 = reinterpret_cast<const float4 *>(K)[1],
+               k2 = reinterpret_cast<const float4 *>(K)[2];
   const bool isR = (st & 1) == 0;
-  const ff tR = ff_mul(isR ? K.bR : K.a, p), tY = ff_mul(isR ? K.a : K.bY, p);
-  const ff own = ff_add(isR ? tR : tY, isR ? K.dR : K.dY);  // the observed state's entry
-  v[0] = st == 0 ? own : tR;
-  v[2] = st == 2 ? own : tR;
-  v[1] = st == 1 ? own : tY;
-  v[3] = st == 3 ? own : tY;
+  const ff2 c = ff2_make(f2_pack(isR ? k0.z : k0.x, isR ? k0.x : k0.w), f2_pack(isR ? k2.x : k1.z, isR ? k1.z : k2.y));
+  const ff2 t = ff2_mul_u(c, ff2_make(f2_pack(p.x, p.x), f2_pack(p.y, p.y)));
+  const float2 th = f2_un(t.hi), tl = f2_un(t.lo);
+  const ff s = two_sum(isR ? th.x : th.y, isR ? k1.x : k1.y);
+  const float oh = s.hi, ol = __fadd_rn(s.lo, __fadd_rn(isR ? tl.x : tl.y, isR ? k2.z : k2.w));
+  v[0] = ff2_make(f2_pack(st == 0 ? oh : th.x, st == 1 ? oh : th.y), f2_pack(st == 0 ? ol : tl.x, st == 1 ? ol : tl.y));
+  v[1] = ff2_make(f2_pack(st == 2 ? oh : th.x, st == 3 ? oh : th.y), f2_pack(st == 2 ? ol : tl.x, st == 3 ? ol : tl.y));
 }
-// The same steps leaving the pair unnormalised (|lo| may reach a few
-// ulp(hi)), for intermediate values: the next step's TwoSum is exact
-// whatever lo is, so only the values that leave the apply are renormalised.
-__device__ __forceinline__ ff ff_mul_u(ff a, ff b)
-{
-  const float p = __fmul_rn(a.hi, b.hi);
-  return ff_make(p, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.hi, -p))));
-}
-__device__ __forceinline__ ff ff_fma_pos_u(ff a, ff b, ff c)
-{
-  const float p = __fmul_rn(a.hi, b.hi);
-  const float pe = __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.hi, -p)));
-  const ff s = two_sum(p, c.hi);
-  return ff_make(s.hi, __fadd_rn(s.lo, __fadd_rn(pe, c.lo)));
-}
-
-// v_j = E1 S_o + b_c S_c + d_c L_j, left unnormalised too: its only use is
-// the product of the two daughters, whose ff_mul renormalises
-__device__ __forceinline__ void hky_apply_ff(const HkyCoefFF &K, const ff *pi, const ff *L, ff *v)
-{
-  const ff SR = ff_fma_pos_u(pi[2], L[2], ff_mul_u(pi[0], L[0]));
-  const ff SY = ff_fma_pos_u(pi[3], L[3], ff_mul_u(pi[1], L[1]));
-  const ff tR = ff_fma_pos_u(K.bR, SR, ff_mul_u(K.a, SY));
-  const ff tY = ff_fma_pos_u(K.bY, SY, ff_mul_u(K.a, SR));
-  v[0] = ff_fma_pos_u(K.dR, L[0], tR);
-  v[2] = ff_fma_pos_u(K.dR, L[2], tR);
-  v[1] = ff_fma_pos_u(K.dY, L[1], tY);
-  v[3] = ff_fma_pos_u(K.dY, L[3], tY);
-}
-
 __device__ __forceinline__ ff ff_of(float2 v) { return ff_make(v.x, v.y); }
 
 // Shared-memory carve-up, identical on host (sizing) and device.
-// tip, inner: bytes of one branch's coefficients below a tip and below an
-// internal node; times: bytes of one node's time.
+// branch: bytes of one branch's coefficients; time: bytes of one node's time.
 struct HkyLayout {
-  size_t inner, nd, times, fresh, order, lev, total;
+  size_t nd, times, fresh, order, tip, off, total;
 };
-__host__ __device__ inline HkyLayout hky_layout(int maxnl, size_t tip, size_t inner, size_t time)
+__host__ __device__ inline HkyLayout hky_layout(int maxnl, size_t branch, size_t time)
 {
-  const size_t maxn = (size_t)(maxnl + 1) / 2;
   HkyLayout l;
-  l.inner = tip * maxn;
-  l.nd = l.inner + inner * maxn;
+  l.nd = branch * (size_t)maxnl;
   l.times = l.nd + sizeof(NodeRec) * (size_t)maxnl;
   l.fresh = l.times + time * (size_t)maxnl;
   l.order = (l.fresh + 3 * (size_t)maxnl + 15) & ~size_t(15);
-  l.lev = (l.order + sizeof(int16_t) * (size_t)(maxnl + 3) + 15) & ~size_t(15);
-  l.total = (l.lev + sizeof(int32_t) * (size_t)(maxnl / 2 + 2) + 15) & ~size_t(15);
+  l.tip = l.order + sizeof(int16_t) * (size_t)(maxnl + 3);
+  l.off = (l.tip + sizeof(int16_t) * (size_t)maxnl + 3) & ~size_t(3);
+  l.total = (l.off + sizeof(int32_t) * (size_t)(maxnl / 2 + 2) + 15) & ~size_t(15);
   return l;
 }
 __host__ __device__ inline HkyLayout hky_layout64(int maxnl)  // k_hky_fp64: a 4 x 4 matrix per branch
 {
-  return hky_layout(maxnl, 16 * sizeof(double), 16 * sizeof(double), 0);
+  return hky_layout(maxnl, 16 * sizeof(double), 0);
 }
-// k_hky_fast, in floats: a tip branch's 32 are padded so that lanes on
-// different branches of a level start in different banks
-__host__ __device__ constexpr int hky_tip_floats(bool ff) { return ff ? 36 : 8; }
-__host__ __device__ constexpr int hky_inner_floats(bool ff) { return ff ? 12 : 8; }
+// k_hky_fast: floats per branch (5 coefficients, as pairs in float-float)
+__host__ __device__ constexpr int hky_floats(bool ff) { return ff ? 12 : 8; }
 __host__ __device__ inline HkyLayout hky_layout_fast(int maxnl, bool ff)
 {
-  return hky_layout(maxnl, 4 * hky_tip_floats(ff), 4 * hky_inner_floats(ff), sizeof(float2));
+  return hky_layout(maxnl, 4 * hky_floats(ff), sizeof(float2));
 }
 
-// ----------------------------------------------------- pattern classes
-// Below a node, site patterns that agree on its tips have the same partial.
-// A node's classes are numbered in the order of their first patterns, which
-// depends only on the tips below it, so that a clean node's stored partials
-// (one per class, at the class's number) stay addressable whatever happens
-// above.  k_hky_classes lists, per level, one task per class of each node: x =
-// (node - n) | class << 16, y = the index of either daughter's value (a tip's
-// state, or the class in the daughter), the internal daughter first.  The
-// root keeps every pattern, for the sum.  On sequences simulated on their
-// genealogies 8-20% of the (node, pattern) pairs remain, on random ones 30-40%.
-// Loci of more than CLS_MAXS patterns keep every pattern (CLS_MAXS bounds a
-// warp's hash table).
-constexpr int CLS_MAXS = 2048;
-constexpr int CLS_WARPS = 8;
-constexpr size_t CLS_SHARED = 32 * 1024;  // class numbers of all nodes and patterns kept in shared memory up to this
-constexpr uint32_t CLS_EMPTY = 0xffffffffu;
-
-__device__ __forceinline__ int2 hky_children(const NodeRec &nd, int n)
+// ----------------------------------------------------- uniform patterns
+// Where every tip below a node shows the same state x, the node's partial at
+// that pattern depends on x alone.  So a node keeps one partial per pattern
+// that is mixed below it (in pattern order from entry 4 on) and one per state x
+// (at entry x) for all the others: on
+// sequences simulated on their genealogies 8-26% of the (node, pattern) pairs,
+// on random genealogies 33-49%.  Which patterns are mixed depends only on the
+// tips below, so a clean node's stored partials stay addressable whatever
+// happens above.  Masks of mixed patterns come bottom-up from the tips' states,
+// kept as two bit planes per tip (P.planes): mixed(v) = mixed(a) | mixed(b) |
+// (planes of a tip below a != planes of a tip below b).  The tasks (one per
+// recomputed node and entry) are listed in schedule order, x = (node - n) |
+// entry << 16, y = the daughters' entries (a tip's state), the internal
+// daughter first.  A full evaluation's list depends on the topology alone: it
+// is kept per item and read back while P.is_valid says so.  Loci whose masks
+// pass HKY_MASK_WORDS, or whose patterns 16 bits, keep every pattern.
+constexpr int HKY_MASK_WORDS = 8192;
+__host__ __device__ inline bool hky_uniform(int n, int S)
+{
+  return (long long)(n - 1) * ((S + 31) / 32) <= HKY_MASK_WORDS && S <= 65531 && n <= 32768;
+}
+__device__ __forceinline__ int2 hky_children(const NodeRec &nd, int n)  // the internal daughter first
 {
   return nd.up0 < n && nd.up1 >= n ? make_int2(nd.up1, nd.up0) : make_int2(nd.up0, nd.up1);
-}
-
-__global__ void __launch_bounds__(32 * CLS_WARPS) k_hky_classes(Pools P, const ReqDev *reqs, int maxnl, int logh, int cap)
-{
-  extern __shared__ __align__(16) char smem[];
-  const ReqDev R = reqs[blockIdx.x];
-  const int n = R.n, nl = 2 * n - 1, S = R.nsites, nint = n - 1;
-  if (S > CLS_MAXS || P.is_valid[R.item]) return;
-  const int H = 1 << logh;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  NodeRec *nd = reinterpret_cast<NodeRec *>(smem);
-  int16_t *order = reinterpret_cast<int16_t *>(nd + maxnl);
-  uint32_t *keys = reinterpret_cast<uint32_t *>(smem + ((sizeof(NodeRec) * maxnl + 2 * (maxnl + 3) + 15) & ~size_t(15))) +
-                   (size_t)warp * (H + H / 2);
-  uint16_t *vals = reinterpret_cast<uint16_t *>(keys + H);
-  __shared__ int count;  // tasks listed so far
-  for (int k = threadIdx.x; k < nl; k += 32 * CLS_WARPS) nd[k] = P.nodes[R.node_off + k];
-  for (int k = threadIdx.x; k < 2 * n; k += 32 * CLS_WARPS) order[k] = P.sched[R.sched_off + k];
-  if (threadIdx.x == 0) count = 0;
-  const int nlev = P.nlev[R.item];
-  const int16_t *lstart = order + nint;
-  const int8_t *seq = P.seq + R.seq_off;
-  // the classes of every node and pattern, read back by the parents
-  uint16_t *rep = nint * S <= cap ? reinterpret_cast<uint16_t *>(keys + (size_t)(CLS_WARPS - warp) * (H + H / 2))
-                                  : P.crep + R.part_off / 2;
-  uint2 *task = P.ctask + R.part_off / 2;
-  int32_t *clev = P.clev + R.sched_off;
-  __syncthreads();
-  for (int lv = 0; lv < nlev; lv++) {
-    if (threadIdx.x == 0) clev[lv] = count;
-    __syncthreads();
-    const int cnt = lstart[lv + 1] - lstart[lv];
-    for (int j = warp; j < cnt; j += CLS_WARPS) {
-      const int node = order[lstart[lv] + j];
-      const int2 c = hky_children(nd[node], n);
-      const bool root = nd[node].down < 0;  // its patterns are summed one by one
-      if (!root)
-        for (int h = lane; h < H; h += 32) keys[h] = CLS_EMPTY;
-      __syncwarp();
-      int ncls = 0;  // classes so far
-      for (int p0 = 0; p0 < S; p0 += 32) {
-        const int p = p0 + lane;
-        const bool in = p < S;
-        uint32_t ia = 0, ib = 0;
-        if (in) {
-          ia = c.x < n ? (uint32_t)seq[(size_t)c.x * S + p] : rep[(size_t)(c.x - n) * S + p];
-          ib = c.y < n ? (uint32_t)seq[(size_t)c.y * S + p] : rep[(size_t)(c.y - n) * S + p];
-        }
-        const uint32_t key = ia | ib << 16;
-        bool first = in;
-        unsigned f;
-        int r = p;
-        if (root) {
-          f = __ballot_sync(0xffffffffu, in);
-        } else {
-          const unsigned m = __match_any_sync(0xffffffffu, in ? key : CLS_EMPTY);
-          const int lead = __ffs(m) - 1;
-          first = false;
-          uint32_t h = 0;
-          if (in && lane == lead) {
-            // one lane per distinct key of these 32: find it or claim a slot
-            for (h = (key * 2654435761u) >> (32 - logh);; h = (h + 1) & (H - 1)) {
-              const uint32_t old = atomicCAS(&keys[h], CLS_EMPTY, key);
-              if (old == CLS_EMPTY) first = true;
-              else if (old == key) r = vals[h];
-              else continue;
-              break;
-            }
-          }
-          f = __ballot_sync(0xffffffffu, first);
-          if (first) {
-            r = ncls + __popc(f & ((1u << lane) - 1u));
-            vals[h] = (uint16_t)r;
-          }
-          ncls += __popc(f);
-          __syncwarp();
-          r = __shfl_sync(0xffffffffu, r, lead);
-          if (in) rep[(size_t)(node - n) * S + p] = (uint16_t)r;
-        }
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&count, __popc(f));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (first) task[base + __popc(f & ((1u << lane) - 1u))] = make_uint2((uint32_t)(node - n) | (uint32_t)r << 16, key);
-      }
-    }
-    __syncthreads();  // the level's classes before its parents
-  }
-  if (threadIdx.x == 0) {
-    clev[nlev] = count;
-    P.is_valid[R.item] = 1;
-  }
 }
 
 // Per-CTA shared state common to both precisions.
@@ -479,23 +441,19 @@ __device__ __forceinline__ int expo_of(float m)  // floor(log2(m)) for normal m 
 // parts of the partials in P.partlo); otherwise FP32 (which clears the lo
 // parts of what it writes when they exist, so a later FF evaluation reads
 // its partials as exact pairs).
-template <bool FF, bool CACHE, int BS, int MINB>
+template <bool FF, int BS, int MINB>
 __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *reqs,
                                                      double *result, int32_t *status, int maxnl,
-                                                     int cache_S, int task_cap)
+                                                     int mcap, int pcap, int tcap)
 {
   extern __shared__ __align__(16) char smem[];
   // the request carries the item's offsets and sizes, so the tree loads
   // below wait on this one load only
   const ReqDev R = reqs[blockIdx.x];
   const int n = R.n, nl = 2 * n - 1, S = R.nsites, nint = n - 1;
-  // per branch 5 coefficients (FF: pairs); FF tip branches hold instead the
-  // columns of P(b) for the four observed states, [4][4] pairs, so a tip
-  // daughter costs two loads
-  constexpr int PT = hky_tip_floats(FF), PI = hky_inner_floats(FF);
+  constexpr int PB = hky_floats(FF);
   const HkyLayout lay = hky_layout_fast(maxnl, FF);
-  float *Pt = reinterpret_cast<float *>(smem);                       // [tip][PT]
-  float *Pi = reinterpret_cast<float *>(smem + lay.inner) - n * PI;  // [internal node][PI]
+  float *Pm = reinterpret_cast<float *>(smem);                 // [branch][PB]
   float2 *stm = reinterpret_cast<float2 *>(smem + lay.times);        // node times
   Tree T;
   T.nd = reinterpret_cast<NodeRec *>(smem + lay.nd);
@@ -503,12 +461,15 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
   T.dirty = T.fresh + maxnl;
   T.slot = T.dirty + maxnl;
   T.order = reinterpret_cast<int16_t *>(smem + lay.order);
-  int32_t *lev = reinterpret_cast<int32_t *>(smem + lay.lev);
-  // the first task_cap tasks staged in shared memory
+  int16_t *tipof = reinterpret_cast<int16_t *>(smem + lay.tip);  // a tip below each node
+  int32_t *toff = reinterpret_cast<int32_t *>(smem + lay.off);   // tasks before the k-th node of the schedule
+  // the last tcap tasks (the narrow levels, where an L2 round trip of about
+  // 1,000 cycles would be the level), the masks of mixed patterns [nint][W],
+  // the tips' planes [n][2][W] where they fit in pcap words
   uint2 *stask = reinterpret_cast<uint2 *>(smem + lay.total);
-  float4 *cpart = reinterpret_cast<float4 *>(stask + task_cap);         // [nint][cache_S]
-  float4 *cpartlo = cpart + (FF ? (size_t)(maxnl / 2) * cache_S : 0);   // FF: lo parts
-  int32_t *cexp = reinterpret_cast<int32_t *>(cpartlo + (size_t)(maxnl / 2) * cache_S);
+  uint32_t *mixed = reinterpret_cast<uint32_t *>(stask + tcap);
+  uint32_t *splane = mixed + mcap;
+  uint16_t *ahead = reinterpret_cast<uint16_t *>(splane + pcap);  // mixed patterns of a node before each mask word
   __shared__ double red_d[BS / 32];
   __shared__ long long red_e[BS / 32];
   __shared__ float2 spi[4];   // pi (FP32: .x only)
@@ -529,12 +490,20 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
   for (int k = tid; k < 2 * n; k += BS) T.order[k] = P.sched[R.sched_off + k];
   const int nlev = P.nlev[R.item];
   T.lstart = T.order + nint;
-  const bool cls = S <= CLS_MAXS;
-  const uint2 *task = P.ctask + R.part_off / 2;
-  const int staged = cls ? (int)min((long long)task_cap, (long long)nint * S) : 0;
-  for (int k = tid; k < staged; k += BS) stask[k] = task[k];
-  if (cls)
-    for (int k = tid; k < n; k += BS) lev[k] = P.clev[R.sched_off + k];  // nlev + 1 <= n of them are meant
+  const bool uni = hky_uniform(n, S);
+  const int W = (S + 31) >> 5, S4 = S + 4;  // S4: partials stored per node
+  const int lw = W > 1 ? 32 - __clz(W - 1) : 0;  // words per node rounded up to 2^lw
+  const uint32_t *plane = P.planes + R.plane_off;
+  uint2 *task = P.task + R.part_off / 2;
+  int32_t *gtoff = P.toff + R.sched_off;
+  const bool listed = uni && full && P.is_valid[R.item];
+  // the list's offsets are loaded beside the flag that says whether they hold
+  if (uni && full)
+    for (int k = tid; k < n; k += BS) toff[k] = gtoff[k];
+  if (uni && !listed && n * 2 * W <= pcap) {
+    for (int k = tid; k < n * 2 * W; k += BS) splane[k] = plane[k];
+    plane = splane;
+  }
   if (tid == 0) {
     // mu = u / (totsites standfactor): 2 kappa (pA pG + pC pT) + 2 (pA + pG)
     // (pC + pT), in float-float (in FP64 one thread's fifty operations held up
@@ -566,63 +535,154 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
   if (FF)
     for (int k = tid; k < 64; k += BS) stab[k] = d_exp64m1[k];
   __syncthreads();
-  if (!full && tid == 0) {  // the reference's propagation rule, bottom-up
-    for (int q = 0; q < 4; q++)
-      if (R.e[q] >= 0 && R.e[q] < nl) T.dirty[R.e[q]] = 1;
-    for (int k = 0; k < nint; k++) {
-      int node = T.order[k];
-      int a = T.nd[node].up0, b = T.nd[node].up1;
-      T.fresh[node] = (T.dirty[node] || T.dirty[a] || T.dirty[b] || (a >= n && T.fresh[a]) ||
-                       (b >= n && T.fresh[b])) ? 1 : 0;
+  if (!full && tid < 32) {  // the reference's propagation rule, a level at a time
+    const int ed = tid == 0 ? R.e[0] : tid == 1 ? R.e[1] : tid == 2 ? R.e[2] : R.e[3];
+    if (tid < 4 && ed >= 0 && ed < nl) T.dirty[ed] = 1;
+    __syncwarp();
+    for (int lv = 0; lv < nlev; lv++) {
+      for (int k = T.lstart[lv] + tid; k < T.lstart[lv + 1]; k += 32) {
+        const int node = T.order[k], a = T.nd[node].up0, b = T.nd[node].up1;
+        T.fresh[node] = (T.dirty[node] || T.dirty[a] || T.dirty[b] || (a >= n && T.fresh[a]) || (b >= n && T.fresh[b])) ? 1 : 0;
+      }
+      __syncwarp();
     }
   }
   if (!full) __syncthreads();
-  for (int c = tid; c < nl; c += BS) {
+  // the masks and the nodes' task counts by the first warp, the branches'
+  // coefficients by the others
+  const bool build = uni && !listed;
+  if (listed) {  // the copies land during the coefficients
+    const int tbase = max(0, toff[nint] - tcap);
+    for (int k = tbase + tid; k < toff[nint]; k += BS)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(stask + k - tbase)),
+                   "l"(task + k)
+                   : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  if (build && tid < 32) {
+    for (int k = tid; k < n; k += 32) tipof[k] = (int16_t)k;
+    __syncwarp();
+    for (int lv = 0; lv < nlev; lv++) {
+      const int beg = T.lstart[lv], cnt = (T.lstart[lv + 1] - beg) << lw;
+      for (int q = tid; q < cnt; q += 32) {
+        const int w = q & ((1 << lw) - 1), node = T.order[beg + (q >> lw)];
+        if (w >= W) continue;
+        const int a = T.nd[node].up0, b = T.nd[node].up1, ta = tipof[a], tb = tipof[b];
+        uint32_t m = (plane[2 * W * ta + w] ^ plane[2 * W * tb + w]) | (plane[2 * W * ta + W + w] ^ plane[2 * W * tb + W + w]);
+        if (a >= n) m |= mixed[(a - n) * W + w];
+        if (b >= n) m |= mixed[(b - n) * W + w];
+        mixed[(node - n) * W + w] = m;
+        if (w == 0) tipof[node] = (int16_t)ta;
+      }
+      __syncwarp();
+    }
+    int before = 0;
+    for (int k0 = 0; k0 < nint; k0 += 32) {
+      int c = 0;
+      if (k0 + tid < nint) {
+        const int node = T.order[k0 + tid];
+        for (int w = 0; w < W; w++) {
+          ahead[(node - n) * W + w] = (uint16_t)c;
+          c += __popc(mixed[(node - n) * W + w]);
+        }
+        c = !T.fresh[node] ? 0 : T.nd[node].down < 0 ? S : c + 4;  // the root: every pattern, for the sum
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, c, o);
+        if (tid >= o) c += v;
+      }
+      if (k0 + tid < nint) toff[k0 + tid + 1] = before + c;
+      before += __shfl_sync(0xffffffffu, c, 31);
+    }
+    if (tid == 0) toff[0] = 0;
+  }
+  for (int c = build ? tid - 32 : tid; c < nl; c += build ? BS - 32 : BS) {
+    if (c < 0) break;
     int d = T.nd[c].down;
     if (d < 0 || !T.fresh[d]) continue;
     if constexpr (FF) {
-      const ff pif[4] = {ff_of(spi[0]), ff_of(spi[1]), ff_of(spi[2]), ff_of(spi[3])};
       const int u = T.nd[c].up0;
       const ff tc = ff_of(stm[c]);
       const ff br = (u < 0) ? tc : ff_sub(tc, ff_of(stm[u]));
       float Kc[10];
       hky_coef_ff(sH, stab, ff_mul(ff_of(smu), br), Kc);
-      float *dst = c < n ? Pt + PT * c : Pi + PI * c;
-      if (c < n) {
-        const HkyCoefFF K = {ff_make(Kc[0], Kc[1]), ff_make(Kc[2], Kc[3]), ff_make(Kc[4], Kc[5]), ff_make(Kc[6], Kc[7]),
-                             ff_make(Kc[8], Kc[9])};
-#pragma unroll
-        for (int st = 0; st < 4; st++) {
-          ff v[4];
-          hky_apply_tip_ff(K, pif, st, v);
-#pragma unroll
-          for (int j = 0; j < 4; j++) reinterpret_cast<float2 *>(dst)[4 * st + j] = make_float2(v[j].hi, v[j].lo);
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 10; j++) dst[j] = Kc[j];
-      }
+      float4 *dst = reinterpret_cast<float4 *>(Pm + PB * c);
+      dst[0] = make_float4(Kc[0], Kc[0], Kc[2], Kc[4]);
+      dst[1] = make_float4(Kc[6], Kc[8], Kc[1], Kc[1]);
+      dst[2] = make_float4(Kc[3], Kc[5], Kc[7], Kc[9]);
     } else {
       float pil[4] = {spi[0].x, spi[1].x, spi[2].x, spi[3].x};
-      hky_coef_fast(pil, skpa.x, smu.x * branch_ff(T.nd, stm, c), c < n ? Pt + PT * c : Pi + PI * c);
+      hky_coef_fast(pil, skpa.x, smu.x * branch_ff(T.nd, stm, c), Pm + PB * c);
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
+  const int tbase = uni ? max(0, toff[nint] - tcap) : 0;
+  if (build) {
+    // a thread takes eight patterns of a node
+    for (int q = tid; q < nint << (lw + 2); q += BS) {
+      const int j = q >> (lw + 2), b8 = q & ((4 << lw) - 1), w = b8 >> 2, node = T.order[j];
+      int at = toff[j];
+      if (w >= W || toff[j + 1] == at) continue;  // no such word; not recomputed
+      const int2 ch = hky_children(T.nd[node], n);
+      auto put = [&](int ea, int eb) {
+        const uint2 t = make_uint2((uint32_t)(node - n) | (uint32_t)(at - toff[j]) << 16, (uint32_t)ea | (uint32_t)eb << 16);
+        if (at >= tbase) stask[at - tbase] = t;
+        if (full || at < tbase) task[at] = t;
+        at++;
+      };
+      const int sh = 8 * (b8 & 3);
+      uint32_t m;
+      if (j == nint - 1) {
+        m = w == W - 1 && (S & 31) ? (1u << (S & 31)) - 1u : 0xffffffffu;
+        at += 32 * w;
+      } else {
+        m = mixed[(node - n) * W + w];
+        if (b8 == 0)
+          for (int x = 0; x < 4; x++) put(x, x);
+        else at += 4;
+        at += ahead[(node - n) * W + w];
+      }
+      at += __popc(m & ((1u << sh) - 1u));
+      m &= 0xffu << sh;
+      if (!m) continue;
+      // the daughters' entries: a tip's state, a mixed pattern's, or the state
+      // of the tips below
+      const int ta = tipof[ch.x], tb = tipof[ch.y];
+      const uint32_t a0 = plane[2 * W * ta + w], a1 = plane[2 * W * ta + W + w], b0 = plane[2 * W * tb + w],
+                     b1 = plane[2 * W * tb + W + w];
+      const uint32_t ma = ch.x < n ? 0u : mixed[(ch.x - n) * W + w], mb = ch.y < n ? 0u : mixed[(ch.y - n) * W + w];
+      const int pa = ch.x < n ? 0 : 4 + ahead[(ch.x - n) * W + w], pb = ch.y < n ? 0 : 4 + ahead[(ch.y - n) * W + w];
+      for (; m; m &= m - 1) {
+        const int k = __ffs(m) - 1;
+        const uint32_t below = (1u << k) - 1u;
+        put((ma >> k) & 1u ? pa + __popc(ma & below) : (int)((a0 >> k) & 1u) + 2 * (int)((a1 >> k) & 1u),
+            (mb >> k) & 1u ? pb + __popc(mb & below) : (int)((b0 >> k) & 1u) + 2 * (int)((b1 >> k) & 1u));
+      }
+    }
+    if (full)
+      for (int k = tid; k < n; k += BS) gtoff[k] = toff[k];
+    __syncthreads();
+    if (full && tid == 0) P.is_valid[R.item] = 1;  // read by later launches only
+  }
 
-  const size_t slot_stride = (size_t)nint * S;
+  const size_t slot_stride = (size_t)nint * S4;
   float4 *part = P.part + R.part_off;
   float4 *partlo = P.partlo ? P.partlo + R.part_off : nullptr;
   int32_t *pexp = P.pexp + R.part_off;
   const int8_t *seq = P.seq + R.seq_off;
   const float pi4[4] = {spi[0].x, spi[1].x, spi[2].x, spi[3].x};
-  // a level's tasks (one per node and class, or per node and pattern) are
-  // independent; the threads take them in turn
+  const ff2 pi2[2] = {ff2_make(f2_pack(spi[0].x, spi[1].x), f2_pack(spi[0].y, spi[1].y)),
+                      ff2_make(f2_pack(spi[2].x, spi[3].x), f2_pack(spi[2].y, spi[3].y))};
+  // a level's tasks are independent; the threads take them in turn
   for (int lv = 0; lv < nlev; lv++) {
-    const int beg = cls ? lev[lv] : 0, end = cls ? lev[lv + 1] : (T.lstart[lv + 1] - T.lstart[lv]) * S;
+    const int beg = uni ? toff[T.lstart[lv]] : 0,
+              end = uni ? toff[T.lstart[lv + 1]] : (T.lstart[lv + 1] - T.lstart[lv]) * S;
     for (int q = beg + tid; q < end; q += BS) {
-      int node, i, ic[2];
-      if (cls) {
-        const uint2 t = q < staged ? stask[q] : task[q];
+      int node, i, ic[2];  // the daughters' entries
+      if (uni) {
+        const uint2 t = q >= tbase ? stask[q - tbase] : task[q];
         node = n + (int)(t.x & 0xffffu);
         i = (int)(t.x >> 16);
         ic[0] = (int)(t.y & 0xffffu);
@@ -630,82 +690,59 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
       } else {
         node = T.order[T.lstart[lv] + q / S];
         i = q % S;
+        if (!T.fresh[node]) continue;
       }
-      if (!T.fresh[node]) continue;
       const int2 ch = hky_children(T.nd[node], n);
       const int cc[2] = {ch.x, ch.y};
-      if (!cls)
+      if (!uni)
         for (int h = 0; h < 2; h++) ic[h] = cc[h] < n ? seq[(size_t)cc[h] * S + i] : i;
       int e = 0;
       float4 ov, ol = make_float4(0.f, 0.f, 0.f, 0.f);
       if constexpr (FF) {
-        const ff pif[4] = {ff_of(spi[0]), ff_of(spi[1]), ff_of(spi[2]), ff_of(spi[3])};
-        ff v[2][4];
+        ff2 v[2][2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           const int c = cc[h];
           if (c < n) {
-            const float4 *col = reinterpret_cast<const float4 *>(Pt + PT * c) + 2 * ic[h];
-            const float4 a = col[0], b = col[1];
-            v[h][0] = ff_make(a.x, a.y);
-            v[h][1] = ff_make(a.z, a.w);
-            v[h][2] = ff_make(b.x, b.y);
-            v[h][3] = ff_make(b.z, b.w);
+            hky_apply_tip_ff(Pm + PB * c, spi[ic[h]], ic[h], v[h]);
           } else {
-            const HkyCoefFF K = load_coef_ff(Pi + PI * c);
-            float4 hi, lo;
-            if (CACHE && T.fresh[c]) {
-              const size_t ci = (size_t)(c - n) * cache_S + ic[h];
-              hi = cpart[ci];
-              lo = cpartlo[ci];
-              e += cexp[ci];
-            } else {
-              const int rs = T.fresh[c] ? 1 - T.slot[c] : T.slot[c];
-              const size_t idx = rs * slot_stride + (size_t)(c - n) * S + ic[h];
-              hi = part[idx];
-              lo = partlo[idx];
-              e += pexp[idx];
-            }
-            const ff Lc[4] = {ff_make(hi.x, lo.x), ff_make(hi.y, lo.y), ff_make(hi.z, lo.z), ff_make(hi.w, lo.w)};
-            hky_apply_ff(K, pif, Lc, v[h]);
+            const int rs = T.fresh[c] ? 1 - T.slot[c] : T.slot[c];
+            const size_t idx = rs * slot_stride + (size_t)(c - n) * S4 + ic[h];
+            ff2 L[2];
+            ff2_load(part[idx], partlo[idx], L);
+            e += pexp[idx];
+            hky_apply_ff(Pm + PB * c, pi2, L, v[h]);
           }
         }
-        ff o[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) o[j] = ff_mul(v[0][j], v[1][j]);
+        const ff2 o0 = ff2_mul(v[0][0], v[1][0]), o1 = ff2_mul(v[0][1], v[1][1]);
+        const float2 h0 = f2_un(o0.hi), h1 = f2_un(o1.hi), l0 = f2_un(o0.lo), l1 = f2_un(o1.lo);
+        ov = make_float4(h0.x, h0.y, h1.x, h1.y);
+        ol = make_float4(l0.x, l0.y, l1.x, l1.y);
         // normalise by an exact power of two when the largest entry drops
         // below 2^-20: the lo parts (2^-24 below) stay far from subnormal
-        const float m = fmaxf(fmaxf(o[0].hi, o[1].hi), fmaxf(o[2].hi, o[3].hi));
+        const float m = fmaxf(fmaxf(ov.x, ov.y), fmaxf(ov.z, ov.w));
         if (m < 9.5367432e-07f && m > 0.f) {
           const int k = expo_of(m);
           const float sc = pow2f(-k);
-#pragma unroll
-          for (int j = 0; j < 4; j++) o[j] = ff_make(o[j].hi * sc, o[j].lo * sc);
+          ov = make_float4(ov.x * sc, ov.y * sc, ov.z * sc, ov.w * sc);
+          ol = make_float4(ol.x * sc, ol.y * sc, ol.z * sc, ol.w * sc);
           e += k;
         }
-        ov = make_float4(o[0].hi, o[1].hi, o[2].hi, o[3].hi);
-        ol = make_float4(o[0].lo, o[1].lo, o[2].lo, o[3].lo);
       } else {
         float v[2][4];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           const int c = cc[h];
-          const float *Kp = c < n ? Pt + PT * c : Pi + PI * c;
+          const float *Kp = Pm + PB * c;
           const HkyCoef K = {Kp[0], Kp[1], Kp[2], Kp[3], Kp[4]};
           if (c < n) {
             hky_apply_tip(K, pi4, ic[h], v[h]);
           } else {
             float4 Lc;
-            if (CACHE && T.fresh[c]) {
-              const size_t ci = (size_t)(c - n) * cache_S + ic[h];
-              Lc = cpart[ci];
-              e += cexp[ci];
-            } else {
-              const int rs = T.fresh[c] ? 1 - T.slot[c] : T.slot[c];
-              const size_t idx = rs * slot_stride + (size_t)(c - n) * S + ic[h];
-              Lc = part[idx];
-              e += pexp[idx];
-            }
+            const int rs = T.fresh[c] ? 1 - T.slot[c] : T.slot[c];
+            const size_t idx = rs * slot_stride + (size_t)(c - n) * S4 + ic[h];
+            Lc = part[idx];
+            e += pexp[idx];
             hky_apply(K, pi4, Lc, v[h]);
           }
         }
@@ -726,16 +763,10 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
           }
         }
       }
-      const size_t widx = (1 - T.slot[node]) * slot_stride + (size_t)(node - n) * S + i;
+      const size_t widx = (1 - T.slot[node]) * slot_stride + (size_t)(node - n) * S4 + i;
       part[widx] = ov;
       if (partlo) partlo[widx] = ol;
       pexp[widx] = e;
-      if (CACHE) {
-        const size_t ci = (size_t)(node - n) * cache_S + i;
-        cpart[ci] = ov;
-        if (FF) cpartlo[ci] = ol;
-        cexp[ci] = e;
-      }
     }
     __syncthreads();
   }
@@ -749,17 +780,10 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
   for (int i = tid; i < S; i += BS) {
     float4 Lr, Ll = make_float4(0.f, 0.f, 0.f, 0.f);
     int er;
-    if (CACHE && T.fresh[root]) {
-      size_t ci = (size_t)(root - n) * cache_S + i;
-      Lr = cpart[ci];
-      if (FF) Ll = cpartlo[ci];
-      er = cexp[ci];
-    } else {
-      size_t idx = rs * slot_stride + (size_t)(root - n) * S + i;
-      Lr = part[idx];
-      if (FF) Ll = partlo[idx];
-      er = pexp[idx];
-    }
+    const size_t idx = rs * slot_stride + (size_t)(root - n) * S4 + i;
+    Lr = part[idx];
+    if (FF) Ll = partlo[idx];
+    er = pexp[idx];
     const int mlt = mult[i];
     if constexpr (FF) {
       ff f = ff_mul(ff_of(spi[0]), ff_make(Lr.x, Ll.x));
@@ -938,43 +962,19 @@ __global__ void k_hky_commit(Pools P, const int32_t *items, const uint8_t *accep
 
 }  // namespace
 
-// Partials stay in shared memory when the largest chain-locus of the batch
-// fits in this budget (keeps >= 3 CTAs per SM).
-constexpr size_t HKY_CACHE_BUDGET = 64 * 1024;
-constexpr int HKY_TASK_CAP = 768;  // tasks staged in shared memory (6 KB)
+constexpr size_t HKY_TASK_CAP = 640, HKY_PLANE_CAP = 1024;  // tasks and words kept in shared memory
 
 template <bool FF, int BS, int MINB>
-static void hky_fast_bs(const Pools &P, const ReqDev *reqs, int nreq, int maxnl, int maxS, bool cache_ok,
-                        double *result, int32_t *status, cudaStream_t st)
+static void hky_fast_bs(const Pools &P, const ReqDev *reqs, int nreq, int maxnl, int maxS, double *result,
+                        int32_t *status, cudaStream_t st)
 {
-  const size_t maxn = (size_t)(maxnl + 1) / 2;
-  const int task_cap = (int)std::min((size_t)HKY_TASK_CAP, (maxn - 1) * maxS + 1) & ~1;
-  const size_t base = hky_layout_fast(maxnl, FF).total + task_cap * sizeof(uint2);
-  size_t cache = (size_t)(maxnl / 2) * maxS * ((FF ? 2 : 1) * sizeof(float4) + sizeof(int32_t));
-  if (cache_ok && cache <= HKY_CACHE_BUDGET) {
-    size_t sm = base + cache;
-    if (sm > 48 * 1024)
-      cudaFuncSetAttribute(k_hky_fast<FF, true, BS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_hky_fast<FF, true, BS, MINB><<<nreq, BS, sm, st>>>(P, reqs, result, status, maxnl, maxS, task_cap);
-  } else {
-    if (base > 48 * 1024)
-      cudaFuncSetAttribute(k_hky_fast<FF, false, BS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)base);
-    k_hky_fast<FF, false, BS, MINB><<<nreq, BS, base, st>>>(P, reqs, result, status, maxnl, 0, task_cap);
-  }
-}
-
-void launch_hky_classes(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, cudaStream_t st)
-{
-  if (nreq <= 0) return;
-  const int maxnl = 2 * maxn - 1, S = std::min(maxS, CLS_MAXS);
-  int logh = 6;
-  while ((1 << logh) < 2 * S) logh++;
-  const size_t hash = ((sizeof(NodeRec) * maxnl + 2 * (maxnl + 3) + 15) & ~size_t(15)) + CLS_WARPS * 6ul * (1ul << logh);
-  size_t sm = hash;
-  const size_t all = 2ul * (maxn - 1) * S;
-  if (all <= CLS_SHARED) sm += all;
-  if (sm > 48 * 1024) cudaFuncSetAttribute(k_hky_classes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_hky_classes<<<nreq, 32 * CLS_WARPS, sm, st>>>(P, reqs, maxnl, logh, all <= CLS_SHARED ? (int)(all / 2) : 0);
+  const size_t maxn = (size_t)(maxnl + 1) / 2, W = ((size_t)maxS + 31) / 32;
+  const size_t mcap = std::min((size_t)HKY_MASK_WORDS, (maxn - 1) * W);
+  const size_t pcap = std::min(HKY_PLANE_CAP, 2 * maxn * W), tcap = std::min(HKY_TASK_CAP, (maxn - 1) * (maxS + 4));
+  const size_t sm = hky_layout_fast(maxnl, FF).total + 4 * (mcap + pcap) + 2 * ((mcap + 1) & ~size_t(1)) + tcap * sizeof(uint2);
+  if (sm > 40 * 1024)  // (48 KB with the static part)
+    cudaFuncSetAttribute(k_hky_fast<FF, BS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_hky_fast<FF, BS, MINB><<<nreq, BS, sm, st>>>(P, reqs, result, status, maxnl, (int)mcap, (int)pcap, (int)tcap);
 }
 
 void launch_hky_fast(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, int variant,
@@ -983,12 +983,12 @@ void launch_hky_fast(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int
   if (nreq <= 0) return;
   const int maxnl = 2 * maxn - 1;
   switch (variant) {
-    case 1: hky_fast_bs<true, 64, 16>(P, reqs, nreq, maxnl, maxS, true, result, status, st); break;
-    case 2: hky_fast_bs<true, 256, 4>(P, reqs, nreq, maxnl, maxS, true, result, status, st); break;
-    case 3: hky_fast_bs<true, 128, 10>(P, reqs, nreq, maxnl, maxS, true, result, status, st); break;
-    case 4: hky_fast_bs<true, 128, 6>(P, reqs, nreq, maxnl, maxS, true, result, status, st); break;
-    case 5: hky_fast_bs<true, 96, 11>(P, reqs, nreq, maxnl, maxS, true, result, status, st); break;
-    default: hky_fast_bs<true, 128, 8>(P, reqs, nreq, maxnl, maxS, true, result, status, st); break;
+    case 1: hky_fast_bs<true, 64, 16>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
+    case 2: hky_fast_bs<true, 256, 4>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
+    case 3: hky_fast_bs<true, 128, 10>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
+    case 4: hky_fast_bs<true, 128, 8>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
+    case 5: hky_fast_bs<true, 96, 11>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
+    default: hky_fast_bs<true, 128, 6>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
   }
 }
 
@@ -998,12 +998,12 @@ void launch_hky_fp32(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int
   if (nreq <= 0) return;
   const int maxnl = 2 * maxn - 1;
   switch (variant) {
-    case 1: hky_fast_bs<false, 64, 24>(P, reqs, nreq, maxnl, maxS, true, result, status, st); break;
-    case 2: hky_fast_bs<false, 256, 6>(P, reqs, nreq, maxnl, maxS, true, result, status, st); break;
-    case 3: hky_fast_bs<false, 128, 12>(P, reqs, nreq, maxnl, maxS, false, result, status, st); break;
-    case 4: hky_fast_bs<false, 128, 8>(P, reqs, nreq, maxnl, maxS, true, result, status, st); break;
-    case 5: hky_fast_bs<false, 96, 16>(P, reqs, nreq, maxnl, maxS, true, result, status, st); break;
-    default: hky_fast_bs<false, 128, 12>(P, reqs, nreq, maxnl, maxS, true, result, status, st); break;
+    case 1: hky_fast_bs<false, 64, 24>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
+    case 2: hky_fast_bs<false, 256, 6>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
+    case 3: hky_fast_bs<false, 128, 6>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
+    case 4: hky_fast_bs<false, 128, 8>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
+    case 5: hky_fast_bs<false, 96, 16>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
+    default: hky_fast_bs<false, 128, 12>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
   }
 }
 

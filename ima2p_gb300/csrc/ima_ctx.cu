@@ -281,7 +281,7 @@ struct ima_ctx {
   void *d_mscratch = nullptr;  // marginal densities: points, partial sums
   size_t mscratch_cap = 0;
   // row-derived surface operands held in the scratch: 0 none, 1 FP32 (split
-  // precision screen), 2 FP32 + bf16 planes (tensor-core screen); for the
+  // precision screen), 2 FP32 + FP16 tiles and FP32 lines (tensor-core screen); for the
   // model type srows_model
   int srows_state = 0, srows_model = -1;
   double *d_sx = nullptr, *d_sq = nullptr, *d_sess = nullptr;

@@ -35,38 +35,9 @@ constexpr int DT = SURF_DENSE_TILE;
 constexpr int DW = 8;            // warps per CTA, sharing 32 points
 constexpr int DENSE_FRAC = 16;   // dense from one sampled genealogy in 16 within MARGIN
 constexpr float DENSE_OVF = 40.0f;  // nats above ref at which a point is left to the retake: w^2 and its sums stay in FP32's range
+__device__ float2 d_exp64[64];  // 2^(j/64) as float-float
+
 constexpr int FLUSH = 8;         // tiles (of DT / DW terms per warp) between FP64 flushes
-
-// ln 2 / 64 = L64_A + L64_B + L64_C: the first two of 11 significant bits, so
-// k times them is exact for |k| < 2^13
-constexpr float L64_A = 0.01082611083984375f;
-constexpr float L64_B = 4.3101608753204346e-06f;
-constexpr float L64_C = 3.695530104153022e-09f;
-
-__constant__ float2 c_exp64[64];  // 2^(j/64) as float-float
-
-// e^(dh + dl) for |dh| <= 86: d = k ln2 / 64 + r, |r| <= ln2 / 128, e^r from
-// its series (r and r^2/2 in float-float, r^3 .. r^5 in FP32), times
-// 2^(k/64).  Relative error below 2e-14 for |d| < 1 and 3e-14 |d| beyond.
-__device__ __forceinline__ ff exp_tab(float dh, float dl, const float2 *tab)
-{
-  const float z = __fmaf_rn(dh, 92.33248262f, 12582912.f);
-  const float kf = __fsub_rn(z, 12582912.f);
-  const int k = __float_as_int(z) - 0x4B400000;
-  float h = __fmaf_rn(-kf, L64_B, __fmaf_rn(-kf, L64_A, dh));  // both exact
-  const ff r = two_sum(h, __fmaf_rn(-kf, L64_C, dl));
-  h = r.hi;
-  const float p = __fmul_rn(h, h), pe = __fmaf_rn(h, h, -p);
-  const float q = __fmul_rn(__fmul_rn(p, h), __fmaf_rn(h, __fmaf_rn(h, 1.f / 120, 1.f / 24), 1.f / 6));
-  const ff u = fast_two_sum(h, 0.5f * p);  // r + r^2/2
-  const float w = __fadd_rn(u.lo, __fmaf_rn(u.hi, r.lo, __fadd_rn(r.lo, __fmaf_rn(0.5f, pe, q))));
-  const float2 T = tab[k & 63];
-  const float a = __fmul_rn(T.x, u.hi), ae = __fmaf_rn(T.x, u.hi, -a);
-  const float lo = __fadd_rn(__fmaf_rn(T.x, w, __fmaf_rn(T.y, u.hi, ae)), T.y);
-  const ff s = fast_two_sum(T.x, a);
-  const float sc = __int_as_float((127 + (k >> 6)) << 23);
-  return ff_make(s.hi * sc, __fadd_rn(s.lo, lo) * sc);
-}
 
 // One warp per sample group, lanes are points; counts[0] = dense points
 // (their list in any order: each is evaluated on its own), sparse[t] = points
@@ -150,7 +121,7 @@ __global__ void __launch_bounds__(32 * DW, KC <= 12 ? 3 : KC <= 20 ? 2 : 1)
   int per;
   const int nch = surf_dense_chunks(nd, gridDim.x, S.G, &per);
   const int groups = (nd + 31) / 32;
-  if (tid < 64) tab[tid] = c_exp64[tid];
+  if (tid < 64) tab[tid] = d_exp64[tid];
   const float2 *bias = S.biasff;
   for (int u = blockIdx.x; u < groups * nch; u += gridDim.x) {
     const int grp = u % groups, chunk = u / groups;
@@ -263,10 +234,16 @@ int surf_init_tables()
 {
   float2 t[64];
   for (int j = 0; j < 64; j++) {
-    const long double v = exp2l((long double)j / 64);
-    t[j] = make_float2((float)v, (float)(v - (long double)(float)v));
+    const double v = std::exp2(j / 64.0);
+    t[j] = make_float2((float)v, (float)(v - (double)(float)v));
   }
-  return cudaMemcpyToSymbol(c_exp64, t, sizeof(t)) == cudaSuccess ? 0 : -1;
+  return cudaMemcpyToSymbol(d_exp64, t, sizeof(t)) == cudaSuccess ? 0 : -1;
+}
+
+float2 *surf_exp_table()
+{
+  void *p = nullptr;
+  return cudaGetSymbolAddress(&p, d_exp64) == cudaSuccess ? static_cast<float2 *>(p) : nullptr;
 }
 
 int surf_dense_cols(const SurfArgs &a, int *col0)
@@ -277,7 +254,6 @@ int surf_dense_cols(const SurfArgs &a, int *col0)
 
 void surf_split(const SurfPrep &S, int npoints, const SurfSplit &D, cudaStream_t st)
 {
-  cudaMemsetAsync(D.counts, 0, sizeof(int) * (1 + (npoints + SURF_TC_M - 1) / SURF_TC_M), st);
   k_surf_split<<<(npoints + 31) / 32, 256, 0, st>>>(S, npoints, D.dense, D.list, D.counts, D.counts + 1);
 }
 

@@ -19,7 +19,7 @@
 // only on the earlier tiles: the candidate set, each thread's fold order and
 // so the result are the same on every run.
 //
-// Screens: FP32 FMA on CUDA cores (this file) and a bf16 tcgen05 GEMM
+// Screens: FP32 FMA on CUDA cores (this file) and an FP16 tcgen05 GEMM
 // (k_surf_tc.cu).  Partial (max, sum) per point and genealogy chunk are
 // merged in FP64.
 #include <cfloat>
@@ -164,8 +164,7 @@ int launch_surface_fast(const SurfArgs &a, void *scratch, size_t scratch_bytes, 
   SurfPrep S;
   char *base = static_cast<char *>(scratch);
   SurfPart *part = surf_prep_carve(&S, base, a.G, a.npoints);
-  surf_prep(a, S, false, rows_ready, st);
-  surf_seed(S, a.npoints, SURF_SEED, st);
+  const int nprep = surf_prep(a, S, false, rows_ready, SURF_SEED, SurfZero(), st);
   int nchunks = (a.G + 65535) / 65536;
   if (nchunks > SURF_MAX_CHUNKS) nchunks = SURF_MAX_CHUNKS;
   int chunk = (a.G + nchunks - 1) / nchunks;
@@ -174,6 +173,6 @@ int launch_surface_fast(const SurfArgs &a, void *scratch, size_t scratch_bytes, 
   dim3 grid((a.npoints + TP - 1) / TP, nchunks);
   k_surf_screen_fp32<<<grid, BS, 0, st>>>(S, a.npoints, chunk, part);
   surf_merge(a, part, nchunks, st);
-  *nkernels = (rows_ready ? 0 : 1) + 4;  // rows, points, seed, screen, merge
+  *nkernels = nprep + 2;  // and the screen and the merge
   return 0;
 }

@@ -1,36 +1,44 @@
 // k_surf_tc.cu -- tensor-core screen of the L-mode surface (tcgen05, sm_103a).
 //
-// The screen of the split-precision surface (see k_surf_fast.cu) as a
-// split-bf16 GEMM on the 5th-generation tensor cores: D[point][genealogy] =
-// phi(x_point) . s_genealogy over 32 columns (26 statistics, the bias, zero
-// padding), with both operands split into bf16 hi + lo planes and
-// D = phi_hi s_hi + phi_lo s_hi + phi_hi s_lo accumulated in FP32 in tensor
-// memory (three K = 32 products, six tcgen05.mma per tile): about 16
-// significant bits per product, so few terms reach the exact recomputation.
+// The screen of the split-precision surface (see k_surf_fast.cu) as a GEMM on
+// the 5th-generation tensor cores: D[point][genealogy] = phi(x_point) .
+// s_genealogy over 32 columns (up to 30 statistics, the bias in two parts),
+// FP16 operands in units that suit each column and FP32 accumulation in
+// tensor memory.  The screen only has to tell which terms may lie within
+// MARGIN of the maximum: the statistics are counts and rates that FP16 holds
+// exactly or to 2^-12, so one product is enough, and every point carries a
+// bound on its error (S.err, from the columns' largest rounding errors and
+// its own coefficients') that widens its threshold.
 //
 // One CTA owns 128 points (the A operand, loaded once) and streams tiles of
-// 256 genealogies (the B operand) through a 4-stage shared-memory ring
+// 256 genealogies (the B operand) through an 8-stage shared-memory ring
 // filled by 1-D bulk copies (the TMA engine; the prepared operand is already
 // in the tile layout, so one copy per tile).  Warp roles:
-//   warp 0     one thread issues the bulk copies;
-//   warp 1     one thread issues six K=16 MMAs per tile into one of two
-//              256-column TMEM accumulators;
-//   warps 4-19 drain the accumulators with tcgen05.ld -- warp w reads TMEM
-//              lane quarter w % 4 (32 points, one per thread) and 64
-//              genealogy columns -- and a max tree over each thread's values
-//              decides whether any lies within MARGIN + screen error of the
-//              point's lower bound; such candidates go to a ring;
-//   warps 2-3  take the rings' candidates 32 at a time, recompute them
+//   warp 0     issues the bulk copies;
+//   warps 1-2  issue, each for its half of every tile, two K=16 MMAs into one
+//              of four 128-column TMEM accumulators (the tensor cores hold few
+//              instructions: one warp's waits would leave them idle);
+//   warps 3-6  take the rings' candidates 32 at a time, recompute them
 //              exactly (phi of every point is staged in shared memory) and
-//              add exp(p - ref) to the point's sums.
+//              add exp(p - ref) to the point's sums;
+//   warps 7-22 drain the accumulators, four warps to each: a warp reads TMEM
+//              lane quarter w % 4 (32 points, one per thread) by
+//              tcgen05.ld.red of 32 columns, which return the maximum of
+//              their 32 values too; where it lies within MARGIN +
+//              screen error of the point's lower bound, the values above that
+//              become candidates and go to a ring.
+//
+// 7.1 ms a call, 2.9 in the first pass and 3.7 in the second, against 20.3 with
+// bf16 operands split into two halves (three products), two 256-column
+// accumulators and one issuing thread; the first pass's products alone are 2.1.
 //
 // Results are bit-for-bit reproducible.  Two things would otherwise follow
 // timing: which terms pass the screen, and the order in which they are added.
 //   * The set: a drain warp's threshold is the point's lower bound from the
-//     max-only pre-pass (a maximum over a fixed set of values, so fixed) raised
-//     only by the screened maxima of the warp's own earlier tiles.  Nothing
-//     another warp or chunk found moves it, so every warp screens the same
-//     terms on every run.
+//     max-only pre-pass (a maximum over a fixed set of values, so fixed);
+//     without a pre-pass it is raised by the screened maxima of the warp's own
+//     earlier values.  Nothing another warp or chunk found moves it, so every
+//     warp screens the same terms on every run.
 //   * The order: each term's weight w = exp(p - ref), with ref the pre-pass
 //     bound, is added as a 256-bit fixed-point integer (w * 2^64) by 64-bit
 //     shared-memory atomics with exact carries.  Integer addition is
@@ -45,7 +53,7 @@
 // Every wait is bounded: a wait that runs out sets the error word, the CTA
 // stops issuing work, waits (bounded) for the copies and MMAs it started,
 // frees its TMEM and returns.
-#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <algorithm>
 #include <cmath>
@@ -58,52 +66,47 @@ namespace {
 
 constexpr int TC_M = SURF_TC_M;  // points per CTA (TMEM lanes)
 constexpr int TC_N = SURF_TC_N;  // genealogies per tile (accumulator columns)
-constexpr int NACC = 512 / TC_N;     // TMEM accumulators of TC_N columns
-constexpr uint32_t A_PLANE = TC_M * SURF_KP * 2;   // 8 KB
-constexpr uint32_t B_PLANE = TC_N * SURF_KP * 2;
-constexpr uint32_t A_BYTES = 2 * A_PLANE;          // hi + lo
-constexpr uint32_t B_BYTES = 2 * B_PLANE;
+constexpr int ACC_N = TC_N / 2;       // genealogies per accumulator: half a tile
+constexpr int NACC = 512 / ACC_N;    // TMEM accumulators
+constexpr uint32_t A_BYTES = TC_M * SURF_KP * 2;   // 8 KB
+constexpr uint32_t B_BYTES = TC_N * SURF_KP * 2;   // 16 KB
 constexpr int TC_STAGES = (128 * 1024) / B_BYTES;  // operand ring stages (128 KB of B tiles)
-static_assert(TC_STAGES >= NACC, "a stage's done barrier also marks its accumulator ready");
 // shared memory requested per CTA: more than half an SM's, so one CTA holds
 // an SM and its 512 TMEM columns at a time (the operand ring, phi of the
 // CTA's points, the candidate rings and the per-point log-sum-exp states)
 constexpr size_t TC_SMEM = 212 * 1024;
 constexpr uint32_t WAIT_LIMIT = 1u << 24;          // try_wait rounds before a wait gives up
-constexpr int TC_THREADS = 640;                    // roles: see the file comment
-
-// split-bf16 screen error, relative to sum_k colmax_k |phi_k| (u = 2^-8, the
-// bf16 unit roundoff): the dropped lo*lo product and the residuals of both
-// splits, <= 3 u^2 = 4.6e-5 per product, plus the FP32 accumulation of 96
-// products even if every addition truncates, <= 96 * 2^-23 = 1.1e-5;
-// bounded with margin by 1e-4.
-constexpr float BF16_SCREEN_ERR = 1e-4f;
 
 constexpr int PHI_STRIDE = SURF_K + 1;   // float2 per point row of staged phi (padded)
-constexpr int EPI_WARPS = 16;            // warps 4-19 drain the accumulators
-constexpr int COL_GROUPS = EPI_WARPS / 4;          // accumulator column groups (TMEM lane quarters x 4)
-constexpr int GROUP_COLS = TC_N / COL_GROUPS;      // columns per epilogue warp and tile
-constexpr int REF_WARPS = 2;             // warps 2-3 recompute candidates exactly
-constexpr int RING = 1024;               // candidate slots per refine warp
+constexpr int REF_WARPS = 4;             // warps recomputing candidates exactly
+constexpr int MMA_WARPS = 2;             // a warp issues the products of one half of every tile
+constexpr int REF_WARP0 = 1 + MMA_WARPS; // the first of the refining warps
+constexpr int EPI_WARP0 = REF_WARP0 + REF_WARPS;
+constexpr int EPI_WARPS = 16;            // warps draining the accumulators
+constexpr int ACC_WARPS = EPI_WARPS / NACC;  // warps of an accumulator: its 4 lane quarters
+constexpr int TC_THREADS = 32 * (EPI_WARP0 + EPI_WARPS);
+static_assert(ACC_WARPS == 4 && NACC == 4 && ACC_N % 64 == 0, "a warp drains a lane quarter of one accumulator");
+constexpr int RING = 256;                // candidate slots per epilogue warp
+static_assert(REF_WARPS == 4, "refine warp r takes the candidates of epilogue warps r, r + 4, ...: one lane quarter");
 
 constexpr int FIXW = 4;  // 64-bit words of the fixed-point sums
 
 struct TcSmem {
-  // full[s]: B tile of stage s landed; done[s]: the MMAs of the tile in stage
-  // s completed (stage free, accumulator ready); accempty[a]: accumulator a
-  // drained by every epilogue warp
-  uint64_t full[TC_STAGES], done[TC_STAGES], accempty[NACC], abar;
+  // full[s]: B tile of stage s landed; done[s]: its MMAs completed (stage
+  // free); accfull[a], accempty[a]: accumulator a complete, drained
+  uint64_t full[TC_STAGES], done[TC_STAGES], accfull[NACC], accempty[NACC], abar;
   uint32_t tmem;
   int err;
   int epi_done;                       // epilogue warps that have finished
-  unsigned head[REF_WARPS];           // slots reserved so far in each ring
-  int ring[REF_WARPS][RING];          // candidates: genealogy << 7 | point; -1 = free
+  unsigned head[EPI_WARPS], tail[EPI_WARPS];  // candidates put into and taken from each ring
+  int ring[EPI_WARPS][RING];          // candidates: genealogy << 7 | point
   unsigned long long sum[TC_M][FIXW];   // sum of w * 2^64, w = exp(p - ref), 256-bit fixed point
   unsigned long long sum2[TC_M][FIXW];  // sum of w^2 * 2^64
   float ref[TC_M];                    // the point's lower bound after the pre-pass
   unsigned xmax[TC_M];                // largest exact value refined (ordered bits)
   int ovf[TC_M];                      // a term left the fixed-point range
   float2 phi[TC_M * PHI_STRIDE];      // float-float phi of the CTA's points
+  float2 etab[64];                    // 2^(j/64)
 };
 
 // w >= 2^80 (55.45 nats above ref) leaves the range the sums are sized for:
@@ -166,103 +169,136 @@ __device__ __forceinline__ void set_err(int *err_shared, int *err_global, int co
   atomicCAS(err_global, 0, code);
 }
 
-// hand one candidate (point pl, genealogy g) to the refine warp owning pl
-__device__ __forceinline__ void push_candidate(TcSmem &sh, int *gerr, int pl, int g)
-{
-  const int r = pl & 1;
-  const unsigned slot = atomicAdd(&sh.head[r], 1u);
-  volatile int *dst = &sh.ring[r][slot % RING];
-  // the slot is free once the refine warp has taken its previous occupant
-  for (uint32_t it = 0; *dst != -1; it++) {
-    if (it > WAIT_LIMIT || *(volatile int *)&sh.err) {
-      set_err(&sh.err, gerr, 6);
-      return;
+// An epilogue warp's side of its candidate ring.  The ring has one writing
+// and one reading warp, so its ends are plain counters.
+struct CandidateRing {
+  unsigned head = 0, tail = 0;  // put so far; taken, as last seen
+
+  // the warp's lanes hand over (point pl, genealogies g0 + the set bits of mask)
+  __device__ __forceinline__ void put(TcSmem &sh, int *gerr, int ew, int lane, int pl, int g0, unsigned mask)
+  {
+    for (;;) {
+      const unsigned b = __ballot_sync(0xffffffffu, mask != 0);
+      if (!b) return;
+      const unsigned n = __popc(b);
+      for (uint32_t it = 0; head + n - tail > RING; it++) {
+        tail = __shfl_sync(0xffffffffu, *(volatile unsigned *)&sh.tail[ew], 0);
+        if (head + n - tail <= RING) break;
+        if (__any_sync(0xffffffffu, it > WAIT_LIMIT || *(volatile int *)&sh.err)) {
+          set_err(&sh.err, gerr, 6);
+          return;
+        }
+        __nanosleep(32);
+      }
+      if (mask) {
+        *(volatile int *)&sh.ring[ew][(head + __popc(b & ((1u << lane) - 1u))) % RING] = ((g0 + __ffs(mask) - 1) << 7) | pl;
+        mask &= mask - 1;
+      }
+      head += n;
+      __threadfence_block();
+      __syncwarp();
+      if (lane == 0) *(volatile unsigned *)&sh.head[ew] = head;
     }
-    __nanosleep(32);
   }
-  *dst = (g << 7) | pl;
+};
+
+// below w = exp(d) < 2^-66 a term adds nothing at the sums' scale of 2^-64
+constexpr float ZERO_NATS = -46.0f;
+
+// One candidate per lane, recomputed exactly; its weight is added to its
+// point's sums.
+__device__ __forceinline__ void refine(const SurfPrep &S, TcSmem &sh, int e)
+{
+  const int pl = e & (TC_M - 1), g = e >> 7;
+  const ff y = surf_exact_row(S, g, &sh.phi[pl * PHI_STRIDE]);
+  const unsigned yo = f2ord(y.hi);
+  if (yo > *(volatile unsigned *)&sh.xmax[pl]) atomicMax(&sh.xmax[pl], yo);
+  const ff d = ff_sub(y, ff_from(sh.ref[pl]));
+  if (d.hi > (float)OVF_NATS) {
+    sh.ovf[pl] = 1;
+  } else if (!(d.hi < ZERO_NATS)) {
+    // w = e^d in float-float (FP32 pipes: GB300 runs FP64 at 1/64 of the FP32
+    // rate); hi + lo is exact in a double, and w^2 (up to 2^160, beyond FP32's
+    // range) is squared there
+    const ff x = exp_tab(d.hi, d.lo, sh.etab);
+    const double w = (double)x.hi + (double)x.lo;
+    unsigned long long f[FIXW];
+    fixw(w, f);
+    atomic_addw(sh.sum[pl], f);
+    fixw(w * w, f);
+    atomic_addw(sh.sum2[pl], f);
+  }
 }
 
-// Refine warp r: takes its ring's candidates 32 at a time, recomputes each
-// exactly (one per lane) and adds its weight to its point's sums.  It stops
-// when every epilogue warp has finished and the ring is drained.
+// Refine warp r: takes the candidates of its four rings 32 at a time.  It
+// stops when every epilogue warp has finished and the rings are drained.
 __device__ void refine_loop(const SurfPrep &S, TcSmem &sh, int *gerr, int r, int lane)
 {
-  for (unsigned next = 0;; next += 32) {
-    const unsigned slot = next + lane;
-    volatile int *src = &sh.ring[r][slot % RING];
-    int e = -1;
-    for (uint32_t it = 0;; it++) {
-      e = *src;
-      if (e != -1) break;
-      if (*(volatile int *)&sh.epi_done == EPI_WARPS && slot >= *(volatile unsigned *)&sh.head[r]) break;
-      if (*(volatile int *)&sh.err) break;
-      if (it > WAIT_LIMIT) {
-        set_err(&sh.err, gerr, 7);
-        break;
-      }
-      __nanosleep(64);
+  constexpr int NR = EPI_WARPS / REF_WARPS;
+  unsigned tail = 0;  // lane j < NR: of ring r + REF_WARPS j
+  for (uint32_t idle = 0;;) {
+    const bool last = __shfl_sync(0xffffffffu, *(volatile int *)&sh.epi_done, 0) == EPI_WARPS;
+    __threadfence_block();
+    const unsigned have = *(volatile unsigned *)&sh.head[r + REF_WARPS * (lane % NR)] - tail;
+    __threadfence_block();
+    const unsigned ready = __ballot_sync(0xffffffffu, lane < NR && (have >= 32 || (last && have > 0)));
+    if (ready) {
+      idle = 0;
+      const int j = __ffs(ready) - 1, ew = r + REF_WARPS * j;
+      const unsigned n = min(32u, __shfl_sync(0xffffffffu, have, j)), t = __shfl_sync(0xffffffffu, tail, j);
+      const int e = *(volatile int *)&sh.ring[ew][(t + lane) % RING];
+      __syncwarp();
+      if (lane == j) *(volatile unsigned *)&sh.tail[ew] = tail += n;
+      if (lane < n) refine(S, sh, e);
+      __syncwarp();
+      continue;
     }
-    const bool have = e != -1;
-    if (have) {
-      *src = -1;
-      const int pl = e & (TC_M - 1), g = e >> 7;
-      const ff y = surf_exact(S, g, S.sT + g, S.Gpad, &sh.phi[pl * PHI_STRIDE]);
-      atomicMax(&sh.xmax[pl], f2ord(y.hi));
-      const ff d = ff_sub(y, ff_from(sh.ref[pl]));
-      if (d.hi > (float)OVF_NATS) {
-        sh.ovf[pl] = 1;
-      } else {
-        // w = e^d in float-float (FP32 pipes: GB300 runs FP64 at 1/64 of
-        // the FP32 rate); hi + lo is exact in a double, and w^2 (up to 2^160,
-        // beyond FP32's range) is squared there
-        ff e, em1;
-        ff_exp_expm1(d, &e, &em1);
-        const double w = (double)e.hi + (double)e.lo;
-        unsigned long long x[FIXW];
-        fixw(w, x);
-        atomic_addw(sh.sum[pl], x);
-        fixw(w * w, x);
-        atomic_addw(sh.sum2[pl], x);
-      }
+    if (last) break;
+    if (__any_sync(0xffffffffu, ++idle > WAIT_LIMIT || *(volatile int *)&sh.err)) {
+      if (idle > WAIT_LIMIT) set_err(&sh.err, gerr, 7);
+      break;
     }
-    if (!__any_sync(0xffffffffu, have)) break;
+    __nanosleep(64);
   }
 }
 
-// stride > 0: max-only pass over genealogy tiles 0, stride, 2 stride, ...
-// that only raises the per-point lower bounds S.best (no candidates, no
-// partials); stride == 0: the full pass over every tile, which reads S.best
-// and leaves it unchanged.  dense, sparse (may be null: every point): the
+// MAXONLY: a pass that only raises the per-point lower bounds S.best (no
+// candidates, no partials); otherwise the full pass, which reads S.best and
+// leaves it unchanged (raise: there was no pre-pass).  Over every 2nd or 4th
+// tile the first pass would be cheaper and its bounds lower: where the terms
+// are alike it would pay (32,768 points x 2,097,152 genealogies: 7.7 ms, 6.3
+// with every 4th), where a few genealogies dominate a point it would not
+// (8,192 x 1,048,576: 1.35 ms, 1.83 with every 2nd).  dense, sparse (may be null: every point): the
 // full pass leaves the points with dense[p] = 1 to k_surf_dense, and skips
 // the tiles without others (sparse[tile] = 0).
+template <bool MAXONLY>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-    k_surf_tc(SurfPrep S, int npoints, int tiles_per_chunk, int stride, const uint8_t *dense, const int *sparse,
-              double2 *part, int *gerr)
+    k_surf_tc(SurfPrep S, int npoints, int tiles_per_chunk, bool raise, const float2 *etab,
+              const uint8_t *dense, const int *sparse, double2 *part, int *gerr)
 {
   extern __shared__ __align__(1024) char smem[];
   if (sparse && sparse[blockIdx.x] == 0) return;
   char *bufA = smem;
   char *bufB = smem + A_BYTES;
   TcSmem &sh = *reinterpret_cast<TcSmem *>(smem + A_BYTES + TC_STAGES * B_BYTES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int ptile = blockIdx.x;
-  const bool maxonly = stride > 0;
-  const int step = maxonly ? stride : 1;
-  const int ntiles_all = (S.Gpad / TC_N + step - 1) / step;  // tiles of this pass
+  const int ntiles_all = S.Gpad / TC_N;
   const int t0 = blockIdx.y * tiles_per_chunk, t1 = min(ntiles_all, t0 + tiles_per_chunk);
   const int ntiles = max(0, t1 - t0);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_STAGES; s++) {
       tc::mbar_init(&sh.full[s], 1);
-      tc::mbar_init(&sh.done[s], 1);
+      tc::mbar_init(&sh.done[s], MMA_WARPS);
     }
-    for (int a = 0; a < NACC; a++) tc::mbar_init(&sh.accempty[a], EPI_WARPS);  // one arrival per epilogue warp
+    for (int a = 0; a < NACC; a++) {
+      tc::mbar_init(&sh.accfull[a], 1);
+      tc::mbar_init(&sh.accempty[a], ACC_WARPS);  // one arrival per warp draining it
+    }
     tc::mbar_init(&sh.abar, 1);
     sh.err = 0;
     sh.epi_done = 0;
-    for (int r = 0; r < REF_WARPS; r++) sh.head[r] = 0;
     tc::fence_barrier_init();
   }
   // every thread stages phi, the rings and the per-point states
@@ -270,7 +306,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int pl = i / SURF_K, k = i % SURF_K, p = ptile * TC_M + pl;
     sh.phi[pl * PHI_STRIDE + k] = p < npoints ? S.phiff[(size_t)p * SURF_K + k] : make_float2(0.f, 0.f);
   }
-  for (int i = threadIdx.x; i < REF_WARPS * RING; i += TC_THREADS) (&sh.ring[0][0])[i] = -1;
+  if (threadIdx.x < EPI_WARPS) sh.head[threadIdx.x] = sh.tail[threadIdx.x] = 0;
+  if (threadIdx.x < 64) sh.etab[threadIdx.x] = etab[threadIdx.x];
   for (int pl = threadIdx.x; pl < TC_M; pl += TC_THREADS) {
     for (int w = 0; w < FIXW; w++) sh.sum[pl][w] = sh.sum2[pl][w] = 0ull;
     const int p = ptile * TC_M + pl;
@@ -278,7 +315,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     sh.xmax[pl] = f2ord(-INFINITY);
     sh.ovf[pl] = 0;
   }
-  if (warp == 1) {
+  if (warp == 0) {
     tc::tmem_alloc(&sh.tmem, 512);
     tc::tmem_relinquish();
   }
@@ -287,147 +324,144 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   tc::fence_after_sync();
   const uint32_t tmem = sh.tmem;
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
     // ------------------------------------------------------------ loader
-    tc::mbar_expect_tx(&sh.abar, A_BYTES);
-    tc::bulk_g2s(bufA, S.pbf + (size_t)ptile * (A_BYTES / 2), A_BYTES, &sh.abar);
+    if (tc::elect_one()) {
+      tc::mbar_expect_tx(&sh.abar, A_BYTES);
+      tc::bulk_g2s(bufA, S.ph + (size_t)ptile * (A_BYTES / 2), A_BYTES, &sh.abar);
+    }
+    __syncwarp();
     int issued = 0;
     for (int i = 0; i < ntiles; i++) {
       const int s = i % TC_STAGES;
-      if (i >= TC_STAGES && !tc::mbar_wait(&sh.done[s], ((i / TC_STAGES) - 1) & 1, WAIT_LIMIT)) {
-        set_err(&sh.err, gerr, 1);
-        break;
+      const bool ok = i < TC_STAGES || tc::mbar_wait(&sh.done[s], ((i / TC_STAGES) - 1) & 1, WAIT_LIMIT);
+      if (!ok) set_err(&sh.err, gerr, 1);
+      if (!__all_sync(0xffffffffu, ok && !*(volatile int *)&sh.err)) break;
+      if (tc::elect_one()) {
+        tc::mbar_expect_tx(&sh.full[s], B_BYTES);
+        tc::bulk_g2s(bufB + s * B_BYTES, S.sh + (size_t)(t0 + i) * (B_BYTES / 2), B_BYTES, &sh.full[s]);
       }
-      if (*(volatile int *)&sh.err) break;
-      tc::mbar_expect_tx(&sh.full[s], B_BYTES);
-      tc::bulk_g2s(bufB + s * B_BYTES, S.sbf + (size_t)(t0 + i) * step * (B_BYTES / 2), B_BYTES, &sh.full[s]);
+      __syncwarp();
       issued = i + 1;
     }
-    // copies this thread started must land before the CTA can leave
+    // copies this warp started must land before the CTA can leave
     for (int i = max(0, issued - TC_STAGES); i < issued; i++)
       tc::mbar_wait(&sh.full[i % TC_STAGES], (i / TC_STAGES) & 1, WAIT_LIMIT);
     tc::mbar_wait(&sh.abar, 0, WAIT_LIMIT);
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp < REF_WARP0) {
     // --------------------------------------------------------------- MMA
-    const uint32_t idesc = tc::idesc_bf16_f32(TC_M, TC_N);
+    const int half = warp - 1;
+    const uint32_t idesc = tc::idesc_f16_f32(TC_M, ACC_N);
     // descriptors: the address field counts 16-byte units, so offsets add
     const uint64_t ad = tc::sdesc(tc::smem_u32(bufA), 128, 512);
-    const uint64_t bd0 = tc::sdesc(tc::smem_u32(bufB), 128, 512);
+    const uint64_t bd0 = tc::sdesc(tc::smem_u32(bufB) + half * (B_BYTES / 2), 128, 512);
     bool ok = tc::mbar_wait(&sh.abar, 0, WAIT_LIMIT);
     if (!ok) set_err(&sh.err, gerr, 2);
     int ndone = 0;
-    for (int i = 0; ok && i < ntiles; i++) {
-      const int s = i % TC_STAGES, a = i % NACC;
-      if (!tc::mbar_wait(&sh.full[s], (i / TC_STAGES) & 1, WAIT_LIMIT)) {
+    for (int i = 0; i < ntiles; i++) {
+      const int s = i % TC_STAGES, h = 2 * i + half, a = h % NACC;
+      if (ok && !tc::mbar_wait(&sh.full[s], (i / TC_STAGES) & 1, WAIT_LIMIT)) {
         set_err(&sh.err, gerr, 3);
-        break;
+        ok = false;
       }
-      if (i >= NACC && !tc::mbar_wait(&sh.accempty[a], ((i / NACC) - 1) & 1, WAIT_LIMIT)) {
+      if (ok && h >= NACC && !tc::mbar_wait(&sh.accempty[a], ((h / NACC) - 1) & 1, WAIT_LIMIT)) {
         set_err(&sh.err, gerr, 4);
-        break;
+        ok = false;
       }
-      if (*(volatile int *)&sh.err) break;
+      // all of the warp goes on or none
+      if (!__all_sync(0xffffffffu, ok && !*(volatile int *)&sh.err)) break;
       tc::fence_after_sync();
-      const uint32_t d = tmem + (uint32_t)(a * TC_N);
+      const uint32_t d = tmem + (uint32_t)(a * ACC_N);
       const uint64_t bd = bd0 + (uint64_t)((s * B_BYTES) >> 4);
-      // phi_hi s_hi + phi_lo s_hi + phi_hi s_lo, each K = 32 as two K = 16
-      const uint64_t ap[3] = {ad, ad + (A_PLANE >> 4), ad};
-      const uint64_t bp[3] = {bd, bd, bd + (B_PLANE >> 4)};
+      if (tc::elect_one()) {
 #pragma unroll
-      for (int t = 0; t < 3; t++)
-#pragma unroll
-        for (int kh = 0; kh < 2; kh++)
-          tc::mma_bf16(d, ap[t] + kh * 16, bp[t] + kh * 16, idesc, (t | kh) ? 1u : 0u);
-      tc::mma_commit(&sh.done[s]);  // stage s free and accumulator a ready once these complete
+        for (int kh = 0; kh < 2; kh++) tc::mma_f16(d, ad + kh * 16, bd + kh * 16, idesc, kh);
+        tc::mma_commit(&sh.accfull[a]);
+        tc::mma_commit(&sh.done[s]);  // and, with the other half's, stage s free
+      }
+      __syncwarp();
       ndone = i + 1;
     }
-    if (ndone > 0) tc::mbar_wait(&sh.done[(ndone - 1) % TC_STAGES], ((ndone - 1) / TC_STAGES) & 1, WAIT_LIMIT);
-  } else if ((warp == 2 || warp == 3) && !maxonly) {
+    // the products this warp started end before the CTA frees its TMEM
+    if (ndone > 0) {
+      const int h = 2 * (ndone - 1) + half;
+      tc::mbar_wait(&sh.accfull[h % NACC], (h / NACC) & 1, WAIT_LIMIT);
+    }
+  } else if (warp >= REF_WARP0 && warp < EPI_WARP0) {
     // ------------------------------------------------------------ refine
-    refine_loop(S, sh, gerr, warp - 2, lane);
-  } else if (warp >= 4) {
+    if (!MAXONLY) refine_loop(S, sh, gerr, warp - REF_WARP0, lane);
+  } else if (warp >= EPI_WARP0) {
     // ---------------------------------------------------------- epilogue
-    const int ew = warp - 4;            // epilogue warp
+    const int ew = warp - EPI_WARP0;
     const int q = warp & 3;             // TMEM lane quarter of this warp
-    const int cg = ew >> 2;             // genealogy columns [GROUP_COLS cg, +GROUP_COLS)
+    const int a = ew / ACC_WARPS;       // its accumulator: half a & 1 of the tiles a / 2, a / 2 + 2, ...
     const int pl = q * 32 + lane;       // point within the tile = TMEM lane
     const int p = ptile * TC_M + pl;
     const bool live = p < npoints && !(dense && dense[p]);
-    const float err = live ? BF16_SCREEN_ERR * S.mag[p] : 0.f;  // screen error bound
-    const float off = err + SURF_MARGIN;
-    // lb: a lower bound on the point's maximum -- the pre-pass bound raised
-    // by this warp's own screened values less their error bound, in tile
-    // order, so the threshold of every tile is the same on every run
+    const float err = live ? S.err[p] : 0.f;  // screen error bound
+    // lb: a lower bound on the point's maximum
     float lb = live ? sh.ref[pl] : -INFINITY;
-    for (int i = 0; i < ntiles; i++) {
-      const int a = i % NACC;
-      if (!tc::mbar_wait(&sh.done[i % TC_STAGES], (i / TC_STAGES) & 1, WAIT_LIMIT)) {
+    float thr = live ? lb - (err + SURF_MARGIN) : INFINITY;
+    const uint32_t tl = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * ACC_N);
+    float mx = -INFINITY;  // pre-pass: largest screened value
+    CandidateRing ring;
+    uint32_t parity = 0;
+    int gc = (t0 + a / 2) * TC_N + (a & 1) * ACC_N;  // genealogy of the first column
+    for (int i = a / 2; i < ntiles; i += NACC / 2, gc += (NACC / 2) * TC_N, parity ^= 1) {
+      if (!tc::mbar_wait(&sh.accfull[a], parity, WAIT_LIMIT)) {
         set_err(&sh.err, gerr, 5);
         break;
       }
       tc::fence_after_sync();
-      const int gbase = (t0 + i) * step * TC_N + cg * GROUP_COLS;
-      const uint32_t tl = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * TC_N + cg * GROUP_COLS);
-      float mxv;
-      float v[32];
-      if constexpr (GROUP_COLS == 32) {
-        // one load and a max tree; the candidate masks come from the same
-        // registers
-        uint32_t r[32];
-        tc::tmem_ld32_nowait(tl, r);
-        tc::tmem_wait_ld(r);
 #pragma unroll
-        for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]);
-        float mx[16];
+      for (int c = 0; c < ACC_N; c += 64) {
+        // two loads in flight; nothing but straight-line code runs before
+        // they have landed
+        uint32_t r[2][32], m[2];
+        tc::tmem_ld32_max_nowait(tl + c, r[0], m[0]);
+        tc::tmem_ld32_max_nowait(tl + c + 32, r[1], m[1]);
+        tc::tmem_wait_ld(r[0]);
+        tc::reg_fence32(r[1]);
+        tc::reg_fence(m[0]);
+        tc::reg_fence(m[1]);
+        if (c + 64 == ACC_N) {  // the accumulator has been read
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&sh.accempty[a]);
+        }
+        const float m0 = __uint_as_float(m[0]), m1 = __uint_as_float(m[1]);
+        if (MAXONLY) {
+          // padded genealogies (g >= G) screen to 0 and must not count
+          if (gc + ACC_N <= S.G) {
+            mx = fmaxf(mx, fmaxf(m0, m1));
+          } else {
+            if (gc + c + 32 <= S.G) mx = fmaxf(mx, m0);
+            if (gc + c + 64 <= S.G) mx = fmaxf(mx, m1);
+          }
+          continue;
+        }
+        if (raise) {
+          if (gc + c + 32 <= S.G) lb = fmaxf(lb, m0 - err);
+          if (gc + c + 64 <= S.G) lb = fmaxf(lb, m1 - err);
+          if (live) thr = lb - (err + SURF_MARGIN);
+        }
+        if (!__any_sync(0xffffffffu, fmaxf(m0, m1) > thr)) continue;
 #pragma unroll
-        for (int j = 0; j < 16; j++) mx[j] = fmaxf(v[j], v[j + 16]);
-#pragma unroll
-        for (int w = 8; w >= 1; w >>= 1)
-#pragma unroll
-          for (int j = 0; j < w; j++) mx[j] = fmaxf(mx[j], mx[j + w]);
-        mxv = mx[0];
-      } else {
-        // both loads in flight, one wait, a max tree in place; a passing
-        // value reloads the columns
-        static_assert(GROUP_COLS == 64, "one or two 32-column loads per warp and tile");
-        uint32_t r[64];
-        tc::tmem_ld32_nowait(tl, r);
-        tc::tmem_ld32_nowait(tl + 32, r + 32);
-        tc::tmem_wait_ld(r);
-        tc::reg_fence32(r + 32);
-        float w64[64];
-#pragma unroll
-        for (int j = 0; j < 64; j++) w64[j] = __uint_as_float(r[j]);
-#pragma unroll
-        for (int w = 32; w >= 1; w >>= 1)
-#pragma unroll
-          for (int j = 0; j < w; j++) w64[j] = fmaxf(w64[j], w64[j + w]);
-        mxv = w64[0];
-      }
-      // padded genealogies (g >= G) screen to 0 and must not raise lb
-      if (gbase + GROUP_COLS <= S.G) lb = fmaxf(lb, mxv - err);
-      const float thr = lb - off;
-      const bool hit = live && !maxonly && mxv > thr;
-      if (__any_sync(0xffffffffu, hit)) {
-#pragma unroll 1
-        for (int c = 0; c < GROUP_COLS / 32; c++) {
-          if constexpr (GROUP_COLS != 32) tc::tmem_ld32(tl + c * 32, v);
+        for (int j = 0; j < 2; j++) {
+          if (!__any_sync(0xffffffffu, __uint_as_float(m[j]) > thr)) continue;
           unsigned mask = 0;
 #pragma unroll
-          for (int j = 0; j < 32; j++)
-            if (v[j] > thr) mask |= 1u << j;
-          const int gc = gbase + c * 32, nv = S.G - gc;
-          if (!hit) mask = 0;
-          else if (nv < 32) mask &= nv > 0 ? (1u << nv) - 1u : 0u;
-          for (; mask; mask &= mask - 1) push_candidate(sh, gerr, pl, gc + __ffs(mask) - 1);
+          for (int b = 0; b < 32; b++)
+            if (__uint_as_float(r[j][b]) > thr) mask |= 1u << b;
+          const int gj = gc + c + 32 * j, nv = S.G - gj;
+          if (nv < 32) mask &= nv > 0 ? (1u << nv) - 1u : 0u;
+          ring.put(sh, gerr, ew, lane, pl, gj, mask);
         }
       }
-      tc::fence_before_sync();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&sh.accempty[a]);
     }
+    if (MAXONLY) lb = fmaxf(lb, mx - err);
     // the pre-pass publishes its bound once: a maximum, whatever the order
-    if (maxonly && live) atomicMax(&S.best[p], f2ord(lb));
+    if (MAXONLY && live) atomicMax(&S.best[p], f2ord(lb));
     __syncwarp();
     if (lane == 0) {
       __threadfence_block();
@@ -436,11 +470,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 0) {
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem, 512);
   }
-  if (threadIdx.x < TC_M && !maxonly) {
+  if (threadIdx.x < TC_M && !MAXONLY) {
     const int p = ptile * TC_M + threadIdx.x;
     const bool mine = p < npoints && !(dense && dense[p]);
     if (mine) atomicMax(&S.xmax[p], sh.xmax[threadIdx.x]);
@@ -507,12 +541,11 @@ __global__ void k_surf_tc_scatter(const int *flag, const double *qs, const doubl
 }
 
 // ------------------------------------------------------------ self-test
-// One 128 x 256 x 32 tile of small integers (exact in bf16 and FP32),
+// One 128 x 256 x 32 tile of small integers (exact in FP16 and FP32),
 // checked element by element against CUDA cores.
 __global__ void __launch_bounds__(128, 1) k_tc_selftest(const uint16_t *A, const uint16_t *B, float *D,
                                                          int *err)
 {
-  constexpr uint32_t A_BYTES = A_PLANE, B_BYTES = B_PLANE;
   extern __shared__ __align__(1024) char smem[];
   char *bufA = smem, *bufB = smem + A_BYTES;
   __shared__ uint64_t bar, mbar;
@@ -542,10 +575,10 @@ __global__ void __launch_bounds__(128, 1) k_tc_selftest(const uint16_t *A, const
       atomicCAS(err, 0, 1);
     } else {
       tc::fence_after_sync();
-      const uint32_t idesc = tc::idesc_bf16_f32(TC_M, TC_N);
+      const uint32_t idesc = tc::idesc_f16_f32(TC_M, TC_N);
       const uint32_t aa = tc::smem_u32(bufA), bb = tc::smem_u32(bufB);
       for (int kh = 0; kh < 2; kh++)
-        tc::mma_bf16(tmem, tc::sdesc(aa + kh * 256, 128, 512), tc::sdesc(bb + kh * 256, 128, 512), idesc, kh);
+        tc::mma_f16(tmem, tc::sdesc(aa + kh * 256, 128, 512), tc::sdesc(bb + kh * 256, 128, 512), idesc, kh);
       tc::mma_commit(&mbar);
     }
   }
@@ -579,13 +612,13 @@ __global__ void k_tc_selftest_fill(uint16_t *A, uint16_t *B)
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < TC_M * SURF_KP) {
     int r = i / SURF_KP, k = i % SURF_KP;
-    __nv_bfloat16 v = __float2bfloat16_rn((float)st_a(r, k));
-    *reinterpret_cast<__nv_bfloat16 *>(reinterpret_cast<char *>(A) + tc::tile_off(r, k)) = v;
+    const __half v = __float2half_rn((float)st_a(r, k));
+    *reinterpret_cast<__half *>(reinterpret_cast<char *>(A) + tc::tile_off(r, k)) = v;
   }
   if (i < TC_N * SURF_KP) {
     int n = i / SURF_KP, k = i % SURF_KP;
-    __nv_bfloat16 v = __float2bfloat16_rn((float)st_b(n, k));
-    *reinterpret_cast<__nv_bfloat16 *>(reinterpret_cast<char *>(B) + tc::tile_off(n, k)) = v;
+    const __half v = __float2half_rn((float)st_b(n, k));
+    *reinterpret_cast<__half *>(reinterpret_cast<char *>(B) + tc::tile_off(n, k)) = v;
   }
 }
 
@@ -618,11 +651,6 @@ size_t surface_tc_scratch_bytes(int G, int npoints)
 
 namespace {
 
-// tile stride of the max-only pre-pass: every tile, so the bound is the
-// screened maximum itself and the full pass refines the fewest candidates
-// (config 5: 1,311 per point with every 8th tile, 812 with every 2nd; 67.0,
-// 48.7 and 44.4 ms per evaluation with every 8th, 2nd and every tile)
-constexpr int PRE_STRIDE = 1;
 constexpr int SEED_TC = 32;    // exact samples per point before the pre-pass (one per lane)
 
 // genealogy chunks for a pass over `ntiles` tiles: one CTA holds an SM, so
@@ -656,13 +684,14 @@ int surf_tc_chunks(int ptiles, int ntiles, int nsm, int *per)
 static int tc_passes(const SurfArgs &a, const SurfPrep &S, const SurfSplit *D, double2 *part, int *flag, int *d_err,
                      int nsm, bool pre, cudaStream_t st)
 {
+  const float2 *etab = surf_exp_table();
   const int ntiles = S.Gpad / TC_N;
   const int ptiles = (a.npoints + TC_M - 1) / TC_M;
   int per = 0, nk = 0;
+  const int nchunks = surf_tc_chunks(ptiles, ntiles, nsm, &per);
   if (pre) {
-    const int nch = surf_tc_chunks(ptiles, (ntiles + PRE_STRIDE - 1) / PRE_STRIDE, nsm, &per);
-    k_surf_tc<<<dim3(ptiles, nch), TC_THREADS, TC_SMEM, st>>>(S, a.npoints, per, PRE_STRIDE, nullptr, nullptr, part,
-                                                              d_err);
+    k_surf_tc<true><<<dim3(ptiles, nchunks), TC_THREADS, TC_SMEM, st>>>(S, a.npoints, per, false, etab, nullptr, nullptr,
+                                                                        part, d_err);
     nk++;
   }
   const uint8_t *dense = nullptr;
@@ -676,10 +705,8 @@ static int tc_passes(const SurfArgs &a, const SurfPrep &S, const SurfSplit *D, d
     surf_dense(a, S, *D, db, part, st);
     nk += 2;
   }
-  const int nchunks = surf_tc_chunks(ptiles, ntiles, nsm, &per);
-  k_surf_tc<<<dim3(ptiles, nchunks), TC_THREADS, TC_SMEM, st>>>(S, a.npoints, per, 0, dense,
-                                                                counts ? counts + 1 : nullptr, part, d_err);
-  cudaMemsetAsync(flag, 0, sizeof(int), st);
+  k_surf_tc<false><<<dim3(ptiles, nchunks), TC_THREADS, TC_SMEM, st>>>(S, a.npoints, per, !pre, etab,
+                                                                dense, counts ? counts + 1 : nullptr, part, d_err);
   k_surf_tc_merge<<<(a.npoints + 127) / 128, 128, 0, st>>>(a, S, part, nchunks, dense, counts, db, flag);
   return nk + 2;
 }
@@ -708,19 +735,24 @@ int launch_surface_tc(const SurfArgs &a, void *scratch, size_t scratch_bytes, in
   D.list = D.counts + 2 + np / TC_M;
   D.dense = reinterpret_cast<uint8_t *>(D.list + np);
   static_assert(A_BYTES + TC_STAGES * B_BYTES + sizeof(TcSmem) + 1024 <= TC_SMEM, "smem");
-  cudaFuncSetAttribute(k_surf_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
+  cudaFuncSetAttribute(k_surf_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
+  cudaFuncSetAttribute(k_surf_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
   int nsm = 152;
   {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   }
-  surf_prep(a, S, true, rows_ready, st);
-  surf_seed(S, a.npoints, SEED_TC, st);
-  // a max-only pre-pass over every PRE_STRIDE-th tile gives every point a
-  // lower bound at (or near) its screened maximum before the full pass
-  const bool pre = S.Gpad / TC_N >= 4 * PRE_STRIDE;
-  int nk = (rows_ready ? 0 : 1) + 2 + tc_passes(a, S, &D, part, flag, d_err, nsm, pre, st);
+  SurfZero z;
+  z.z0 = flag;
+  z.n0 = 1;
+  z.z1 = D.counts;
+  z.n1 = 1 + (a.npoints + TC_M - 1) / TC_M;
+  int nk = surf_prep(a, S, true, rows_ready, SEED_TC, z, st);
+  // a max-only pre-pass gives every point a lower bound at (or near) its
+  // screened maximum before the full pass
+  const bool pre = S.Gpad / TC_N >= 4;
+  nk += tc_passes(a, S, &D, part, flag, d_err, nsm, pre, st);
   // points whose terms left the fixed-point range: a second evaluation of
   // just them, referenced to their exact maxima
   int nflag = 0;
@@ -737,7 +769,10 @@ int launch_surface_tc(const SurfArgs &a, void *scratch, size_t scratch_bytes, in
     b.ess = a.ess ? es : nullptr;
     SurfPrep S2;
     double2 *part2 = reinterpret_cast<double2 *>(surf_prep_carve(&S2, base, a.G, nflag));
-    surf_prep(b, S2, true, true, st);
+    SurfZero z2;
+    z2.z0 = flag2;
+    z2.n0 = 1;
+    surf_prep(b, S2, true, true, 0, z2, st);
     k_surf_tc_setref<<<(nflag + 127) / 128, 128, 0, st>>>(S2.best, S2.xmax, refs, nflag);
     nk += 3 + tc_passes(b, S2, nullptr, part2, flag2, d_err, nsm, false, st);
     k_surf_tc_scatter<<<(nflag + 127) / 128, 128, 0, st>>>(flag, qs, es, a.q, a.ess);
@@ -749,7 +784,6 @@ int launch_surface_tc(const SurfArgs &a, void *scratch, size_t scratch_bytes, in
 
 int tc_selftest(cudaStream_t st, void *scratch, size_t bytes, int *h_bad, float *h_maxerr)
 {
-  constexpr uint32_t A_BYTES = A_PLANE, B_BYTES = B_PLANE;
   // scratch: A (8 KB) | B (16 KB) | D (128 KB) | bad, maxerr, err
   const size_t need = A_BYTES + B_BYTES + (size_t)TC_M * TC_N * 4 + 16;
   if (bytes < need) return 3;

@@ -27,12 +27,16 @@ struct SurfPrep {
   float2 *phiff;    // [npoints][SURF_K] phi as float-float
   float *phi32;     // [npoints][SURF_KP] phi rounded, 1 in the bias column
   float *mag;       // [npoints] sum_k colmax_k |phi_k|: scale of screening errors
+  float *err;       // [npoints] error bound of the tensor-core screen
   float *seed;      // [npoints] exact max over a sample of genealogies
   unsigned *best;   // [npoints] best exact maximum found so far (ordered bits), shared by chunks
   unsigned *xmax;   // [npoints] largest exact value the refinement met (ordered bits; tensor-core screen)
   unsigned *colmax; // [SURF_KP] max |column| as float bits
-  uint16_t *sbf;    // bf16 statistics, hi and lo planes of 256-row MMA tiles (tensor-core screen)
-  uint16_t *pbf;    // bf16 phi, hi and lo planes of 128-row MMA tiles (tensor-core screen)
+  unsigned *emax;   // [SURF_KP] max |column - its FP16 form| as float bits (tensor-core screen)
+  uint16_t *sh;     // FP16 statistics in 256-row MMA tiles (tensor-core screen)
+  uint16_t *ph;     // FP16 phi in 128-row MMA tiles (tensor-core screen)
+  float4 *sR;       // [Gpad][SURF_KP / 4] a genealogy's statistics in one line, columns 30, 31 its bias
+                    // as float-float (tensor-core form: single terms)
 };
 
 // Per (point, chunk) partial of the online log-sum-exp.
@@ -67,6 +71,67 @@ __device__ __forceinline__ ff surf_exact(const SurfPrep &S, int g, const float *
     comp = __fadd_rn(comp, __fadd_rn(te, __fmaf_rn(s, f.y, pe)));
   }
   return fast_two_sum(sum, comp);
+}
+
+// the same from the genealogy's line: seven or eight 16-byte loads issued
+// together where the columns of sT would be as many sectors as statistics
+__device__ __forceinline__ ff surf_exact_row(const SurfPrep &S, int g, const float2 *phi)
+{
+  const float4 *r = S.sR + (size_t)g * (SURF_KP / 4);
+  float v[SURF_KP];
+#pragma unroll
+  for (int q = 0; q < SURF_KP / 4; q++) {
+    const float4 t = 4 * q < S.K || q == SURF_KP / 4 - 1 ? __ldg(r + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[4 * q] = t.x;
+    v[4 * q + 1] = t.y;
+    v[4 * q + 2] = t.z;
+    v[4 * q + 3] = t.w;
+  }
+  float sum = v[SURF_KP - 2], comp = v[SURF_KP - 1];
+#pragma unroll
+  for (int q = 0; q < (SURF_K + 3) / 4; q++) {
+    if (4 * q >= S.K) break;
+#pragma unroll
+    for (int k = 4 * q; k < 4 * q + 4 && k < SURF_K; k++) {
+      const float2 f = phi[k];
+      const float p = __fmul_rn(v[k], f.x);
+      const float pe = __fmaf_rn(v[k], f.x, -p);
+      const ff t = two_sum(sum, p);
+      sum = t.hi;
+      comp = __fadd_rn(comp, __fadd_rn(t.lo, __fmaf_rn(v[k], f.y, pe)));
+    }
+  }
+  return fast_two_sum(sum, comp);
+}
+
+// ln 2 / 64 = L64_A + L64_B + L64_C: the first two of 11 significant bits, so
+// k times them is exact for |k| < 2^13
+constexpr float L64_A = 0.01082611083984375f;
+constexpr float L64_B = 4.3101608753204346e-06f;
+constexpr float L64_C = 3.695530104153022e-09f;
+
+// e^(dh + dl) for |dh| <= 86: d = k ln2 / 64 + r, |r| <= ln2 / 128, e^r from
+// its series (r and r^2/2 in float-float, r^3 .. r^5 in FP32), times tab[k &
+// 63] = 2^((k & 63)/64) (float-float).  Relative error below 2e-14 for |d| < 1
+// and 3e-14 |d| beyond.
+__device__ __forceinline__ ff exp_tab(float dh, float dl, const float2 *tab)
+{
+  const float z = __fmaf_rn(dh, 92.33248262f, 12582912.f);
+  const float kf = __fsub_rn(z, 12582912.f);
+  const int k = __float_as_int(z) - 0x4B400000;
+  float h = __fmaf_rn(-kf, L64_B, __fmaf_rn(-kf, L64_A, dh));  // both exact
+  const ff r = two_sum(h, __fmaf_rn(-kf, L64_C, dl));
+  h = r.hi;
+  const float p = __fmul_rn(h, h), pe = __fmaf_rn(h, h, -p);
+  const float q = __fmul_rn(__fmul_rn(p, h), __fmaf_rn(h, __fmaf_rn(h, 1.f / 120, 1.f / 24), 1.f / 6));
+  const ff u = fast_two_sum(h, 0.5f * p);  // r + r^2/2
+  const float w = __fadd_rn(u.lo, __fmaf_rn(u.hi, r.lo, __fadd_rn(r.lo, __fmaf_rn(0.5f, pe, q))));
+  const float2 T = tab[k & 63];
+  const float a = __fmul_rn(T.x, u.hi), ae = __fmaf_rn(T.x, u.hi, -a);
+  const float lo = __fadd_rn(__fmaf_rn(T.x, w, __fmaf_rn(T.y, u.hi, ae)), T.y);
+  const ff s = fast_two_sum(T.x, a);
+  const float sc = __int_as_float((127 + (k >> 6)) << 23);
+  return ff_make(s.hi * sc, __fadd_rn(s.lo, lo) * sc);
 }
 
 struct LseState {
@@ -156,11 +221,16 @@ __device__ __forceinline__ float ord2f(unsigned u)
 
 size_t surf_prep_bytes(int G, int npoints);
 SurfPart *surf_prep_carve(SurfPrep *S, char *base, int G, int npoints);
-// rows_ready: the row-derived operands (sT, biasff, colmax, sbf) are already
-// in place from an earlier evaluation of the same rows and model type
-void surf_prep(const SurfArgs &a, SurfPrep &S, bool bf16, bool rows_ready, cudaStream_t st);
+// The operands.  tc: the tensor-core ones too.  rows_ready: the row-derived
+// ones (sT, biasff, colmax, samp; tc: emax, sh, sR) are already in place from
+// an earlier evaluation of the same rows and model type.  nseed > 0: seed,
+// best and xmax from the exact terms of that many evenly spaced genealogies
+// (32 or 256).  z0, z1: words to clear on the way.  Returns the kernels queued.
+struct SurfZero {
+  int *z0 = nullptr, n0 = 0, *z1 = nullptr, n1 = 0;
+};
+int surf_prep(const SurfArgs &a, SurfPrep &S, bool tc, bool rows_ready, int nseed, const SurfZero &z, cudaStream_t st);
 void surf_merge(const SurfArgs &a, const SurfPart *part, int nchunks, cudaStream_t st);
-void surf_seed(const SurfPrep &S, int npoints, int samples, cudaStream_t st);
 
 // How the points of an evaluation are taken (k_surf_dense.cu): dense[p] = 1
 // where every term is evaluated directly, the list of those points,
@@ -171,6 +241,7 @@ struct SurfSplit {
   int *list, *counts;
 };
 int surf_init_tables();
+float2 *surf_exp_table();  // device address of 2^(j/64), j < 64, as float-float
 void surf_split(const SurfPrep &S, int npoints, const SurfSplit &D, cudaStream_t st);
 int surf_dense_grid(const SurfArgs &a, int nsm);
 // the chunking of nd dense points over a grid of nb CTAs: about three equal

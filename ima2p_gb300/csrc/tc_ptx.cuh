@@ -1,6 +1,6 @@
 // tc_ptx.cuh -- inline PTX for the sm_103a tensor-core path: TMEM
 // allocation, mbarriers with bounded waits, 1-D bulk copies (TMA engine),
-// tcgen05.mma (kind::f16, bf16 inputs, FP32 accumulation in TMEM) and
+// tcgen05.mma (kind::f16, f16 inputs, FP32 accumulation in TMEM) and
 // tcgen05.ld.  Operand tiles use the no-swizzle K-major layout: 8-row x
 // 16-byte core matrices, LBO = distance between core matrices along K,
 // SBO = distance between 8-row groups.
@@ -12,6 +12,18 @@ namespace tc {
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+// true in one lane of a converged warp.  The operands of tcgen05.mma and of
+// the bulk copies are uniform registers: under this test the compiler knows
+// that one lane issues them, under a test of the lane's number it loops over
+// the lanes (two 128 x 256 x 16 products, a commit and a wait: 381 clocks, and
+// 256, the tensor cores' own time, with this).
+__device__ __forceinline__ bool elect_one()
+{
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+  return p != 0;
 }
 
 // ------------------------------------------------------------ mbarrier
@@ -98,14 +110,14 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t
   return d;                // base offset 0, layout type 0 (no swizzle)
 }
 
-// instruction descriptor: D f32, A and B bf16, both K-major, dense
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N)
+// instruction descriptor: D f32, A and B f16, both K-major, dense
+__host__ __device__ constexpr uint32_t idesc_f16_f32(int M, int N)
 {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+  return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 // D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread
-__device__ __forceinline__ void mma_bf16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+__device__ __forceinline__ void mma_f16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate)
 {
   asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -139,19 +151,20 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v)
   for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// 32 consecutive FP32 columns of this thread's TMEM lane, without waiting:
-// r[] holds the values only after tmem_wait_ld on the same registers
-__device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t *r)
+// 32 consecutive FP32 columns of this thread's TMEM lane and their maximum
+// (taken on the way by the load itself, sm_103a), without waiting: r[] and m
+// hold the values only after tmem_wait_ld and reg_fence on the same registers
+__device__ __forceinline__ void tmem_ld32_max_nowait(uint32_t taddr, uint32_t *r, uint32_t &m)
 {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+  asm volatile("tcgen05.ld.red.sync.aligned.32x32b.x32.max.f32 "
                "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-               "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+               "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, %32, [%33];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
                  "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
                  "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
                  "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
                  "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-                 "=r"(r[31])
+                 "=r"(r[31]), "=r"(m)
                : "r"(taddr));
 }
 
@@ -170,7 +183,8 @@ __device__ __forceinline__ void tmem_wait_ld(uint32_t *r)
                : "memory");
 }
 
-// orders later uses of 32 registers after the preceding asm statements
+// orders later uses of registers after the preceding asm statements
+__device__ __forceinline__ void reg_fence(uint32_t &a) { asm volatile("" : "+r"(a)::"memory"); }
 __device__ __forceinline__ void reg_fence32(uint32_t *r)
 {
   asm volatile(""
@@ -184,7 +198,7 @@ __device__ __forceinline__ void reg_fence32(uint32_t *r)
                : "memory");
 }
 
-// byte offset of element (row, k) in a no-swizzle K-major tile of 32 bf16
+// byte offset of element (row, k) in a no-swizzle K-major tile of 32 f16
 // columns: 8-row x 16-byte core matrices, 4 along K (LBO = 128 B), then the
 // next 8 rows (SBO = 512 B)
 __host__ __device__ constexpr uint32_t tile_off(int row, int k)

@@ -278,7 +278,7 @@ int ima_gpu_surface_load(ima_ctx *ctx, int G, int rowlen, const float *gsampinf,
  * from the rows between calls while the rows and modeltype are unchanged. */
 int ima_gpu_surface_eval(ima_ctx *ctx, int npoints, const double *x, int modeltype, int method,
                          double *q, double *ess);
-/* Checks the tensor-core path on this device: one 128 x 256 x 32 bf16 tile of
+/* Checks the tensor-core path on this device: one 128 x 256 x 32 FP16 tile of
  * small integers through TMA, tcgen05.mma and tcgen05.ld, compared element by
  * element with CUDA cores.  *mismatches = 0 when every element matches. */
 int ima_gpu_tc_selftest(ima_ctx *ctx, int *mismatches, float *max_abs_err);

@@ -4309,14 +4309,26 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
   if (!tw_fits(P)) return c->fail(IMA_ERR_TOO_LARGE, "a genealogy has %lld events", Emax);
   // the weights kernel writes every migration cell of the model, nomig or not
   const size_t Etot = (size_t)evoff[ni], M1 = std::max(1, h.M), mx = 2 * (size_t)maxn;
-  // steps in flight: a ring of per-step buffers (backups, proposal flags,
+  // a sweep's launches: runs of consecutive loci of one model, an IS locus by
+  // itself (its decision draws from the chain's generator)
+  const int K = ug_loci_per_launch(nl, maxn);
+  std::vector<int> first;
+  for (int l = 0, e; l < nl; l = e) {
+    const int m = c->loci[l].d.model;
+    for (e = l + 1; e < nl && m != IMA_MODEL_IS && c->loci[e].d.model == m;) e++;
+    const int parts = (e - l + K - 1) / K;  // of much the same size
+    for (int i = 0; i < parts; i++) first.push_back(l + (int)((long long)(e - l) * i / parts));
+  }
+  const int nlaunch = (int)first.size();
+  first.push_back(nl);
+  // launches in flight: a ring of their buffers (backups, proposal flags,
   // slide terms, acceptance uniforms); at most one sweep of loci deep, so a
   // locus's batch and weights are never rewritten before their decision ran
-  const int R = std::min(4, nl);
-  const size_t rn = (size_t)R * nch;
+  const int R = std::min(4, nlaunch);
+  const size_t rn = (size_t)R * K * nch;
   const size_t bytes = carve_size({nch * sizeof(ima_ug_rng), nch * 4ul, np * 4, np * 4, rn * mx * sizeof(NodeRec),
                                    rn * mx * 8, rn * mx * 4, rn * mx * 2, rn * 8, rn * 4, rn * 8, rn * 8, rn * 8,
-                                   rn * 16, rn * mx * 4, rn * mx * 8, rn * 8, rn * 8, rn * 8, np * 8, nl * 8ul,
+                                   rn * 16, rn * mx * 4, rn * mx * 8, rn * 8, rn * 4, rn * 8, rn * 8, rn * 8, np * 8, nl * 8ul,
                                    8, nch * T * 4ul, nch * T * 8ul, nch * T * 8ul, nch * (size_t)nth * 8, np * 4, np * 4,
                                    ni * T * 4ul, ni * M1 * 4, ni * 4ul, ni * T * 8ul, ni * T * 8ul, ni * M1 * 8,
                                    2ul * ni * 8, (ni + 1) * 8ul, Etot * 8, Etot * 4, ni * 4ul});
@@ -4344,6 +4356,8 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
   a.edges = cv.take<int32_t>(4 * rn);
   a.bk_A = cv.take<int32_t>(rn * mx);
   a.bk_dl = cv.take<double>(rn * mx);
+  a.lallele = cv.take<double>(rn);
+  a.neg = cv.take<int32_t>(rn);
   a.swnew = cv.take<double>(rn);
   a.aterm = cv.take<double>(rn);
   a.holdsis = cv.take<double>(rn);
@@ -4369,7 +4383,6 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
   w.ev_t = cv.take<double>(Etot);
   w.ev_c = cv.take<uint32_t>(Etot);
   w.ev_n = cv.take<int32_t>(ni);
-  w.ngen = nch;
   w.P = P;
   w.model = c->d_tw;
   w.ev_off = d_evoff;
@@ -4392,21 +4405,24 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
   w.err = c->d_twerr;
   // per-locus evaluation requests: the listed chains, full evaluations whose
   // HKY edits the proposal fills in
-  if ((int)c->ugb.size() < nl) c->ugb.resize(nl);
+  if ((int)c->ugb.size() < nlaunch) c->ugb.resize(nlaunch);
   std::vector<int32_t> reqof(np), perm(np);
-  for (int l = 0; l < nl && !r; l++) {
-    for (int k = 0; k < nch; k++) perm[(size_t)l * nch + k] = c->item_of(chains[k], l);
-    if (c->loci[l].d.model == IMA_MODEL_SW) continue;  // its update runs in k_ug_sw
-    Batch &b = c->ugb[l];
-    std::vector<int32_t> lli(nch, l);
-    std::vector<double> lu(nch), lk(nch);
-    for (int k = 0; k < nch; k++) {
-      lu[k] = u[(size_t)k * nl + l];
-      lk[k] = kap[(size_t)k * nl + l];
+  for (int s = 0; s < nlaunch && !r; s++) {
+    const int l0 = first[s], nr = (first[s + 1] - l0) * nch;
+    std::vector<int32_t> lci(nr), lli(nr);
+    std::vector<double> lu(nr), lk(nr);
+    for (int k = 0; k < nr; k++) {
+      lci[k] = chains[k % nch];
+      lli[k] = l0 + k / nch;
+      perm[(size_t)l0 * nch + k] = c->item_of(lci[k], lli[k]);
+      lu[k] = u[(size_t)(k % nch) * nl + lli[k]];
+      lk[k] = kap[(size_t)(k % nch) * nl + lli[k]];
     }
-    r = build_batch(c, b, nch, chains, lli.data(), lu.data(), lk.data(), nullptr, nullptr, precision);
+    if (c->loci[l0].d.model == IMA_MODEL_SW) continue;  // its update runs in k_ug_sw
+    Batch &b = c->ugb[s];
+    r = build_batch(c, b, nr, lci.data(), lli.data(), lu.data(), lk.data(), nullptr, nullptr, precision);
     r = r ? r : init_sumlogk(c, b);
-    for (int k = 0; k < nch && !r; k++) reqof[(size_t)l * nch + b.order[k]] = k;
+    for (int k = 0; k < nr && !r; k++) reqof[(size_t)l0 * nch + b.order[k]] = k;
   }
   if (r) return r;
   r = c->cuda(cudaMemcpyAsync(a.rng, rng, nch * sizeof(ima_ug_rng), cudaMemcpyHostToDevice, c->st), "generators");
@@ -4471,13 +4487,13 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
     c->ug_ev.push_back(e);
   }
   cudaEvent_t *evP = c->ug_ev.data(), *evW = evP + 4, *evH = evP + 8, *evD = evP + 12;
-  // The steps: one locus of every listed chain at a time.  Each chain's
+  // The steps: one run of loci of every listed chain at a time.  Each chain's
   // proposals follow one another on st (they share its generator), its
   // decisions on ug_sd (they share its sums); a step's weights (on three
   // streams used by turns) and its likelihoods (on two; consecutive steps
-  // touch different loci) wait for its proposal, its decision for both and
-  // for the previous decision.  So proposals, weights and likelihoods of
-  // the next steps run while a decision does, up to R steps ahead.  After an
+  // touch different loci) wait for its proposals, its decisions for both and
+  // for the previous decisions.  So proposals, weights and likelihoods of
+  // the next steps run while decisions do, up to R steps ahead.  After an
   // IS step the next proposal waits for the decision: an IS decision draws
   // the acceptance uniform only when the likelihood does not reject, so the
   // generator's position is known only then (an HKY proposal draws it
@@ -4486,12 +4502,13 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
   long long step = 0;
   int prev_is = 0;
   for (int s = 0; s < nsweeps && !r; s++)
-    for (int l = 0; l < nl && !r; l++, step++) {
-      const int slot = (int)(step % R);
-      const size_t so = (size_t)slot * nch;
-      Batch &b = c->ugb[l];
+    for (int q = 0; q < nlaunch && !r; q++, step++) {
+      const int l = first[q], slot = (int)(step % R);
+      const size_t so = (size_t)slot * K * nch;
+      Batch &b = c->ugb[q];
       UgArgs u_ = a0;
       u_.locus = l;
+      u_.k = first[q + 1] - l;
       u_.hky = c->loci[l].d.model == IMA_MODEL_HKY;
       u_.sw = c->loci[l].d.model == IMA_MODEL_SW;
       u_.predraw = u_.hky || u_.sw;
@@ -4511,6 +4528,8 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
       u_.edges = a0.edges + 4 * so;
       u_.bk_A = a0.bk_A + so * mx;
       u_.bk_dl = a0.bk_dl + so * mx;
+      u_.lallele = a0.lallele + so;
+      u_.neg = a0.neg + so;
       u_.swnew = a0.swnew + so;
       u_.aterm = a0.aterm + so;
       u_.holdsis = a0.holdsis + so;
@@ -4519,6 +4538,7 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
       c->launch(IMA_K_UG, 0.0, [&] { launch_ug_propose(u_, c->st); });
       cudaEventRecord(evP[slot], c->st);
       w.perm = d_perm + (size_t)l * nch;
+      w.ngen = nch * u_.k;
       cudaStream_t sw = (step % 3 == 0) ? c->ug_sw : (step % 3 == 1 ? c->ug_sw2 : c->ug_sw3);
       cudaStreamWaitEvent(sw, evP[slot], 0);
       int lr = 0;

@@ -312,8 +312,9 @@ int launch_ry_decide(const RyArgs &a, cudaStream_t st);
 // chain per step (k_updgen.cu): a warp per chain proposes (edge, slide,
 // reattachment), the weights and the likelihood of the proposed genealogies
 // run as batches, and a warp per chain decides, then commits or restores.
+constexpr int UG_K = 12;  // loci of one model in one launch, at most
 struct UgArgs {
-  int nch, nloci, locus, maxn, nsplit, hky;
+  int nch, nloci, locus, k, maxn, nsplit, hky;  // loci [locus, locus + k)
   const int32_t *chains;                   // [nch]
   const ItemDev *items;
   NodeRec *nodes;
@@ -327,9 +328,10 @@ struct UgArgs {
   const TwModel *model;
   const double *tvals;                     // [nchains][nsplit]
   ima_ug_rng *rng;                         // [nch] the listed chains' generators
-  ReqDev *req;                             // the locus's evaluation requests
-  const int32_t *req_of;                   // [nch] request of each listed chain
-  // per listed chain: the genealogy before the proposal, for a rejection
+  ReqDev *req;                             // the loci's evaluation requests
+  // below [nch] stands for [k][nch]: per locus of the launch and listed chain
+  const int32_t *req_of;                   // [nch] request
+  // the genealogy before the proposal, for a rejection
   NodeRec *bk_nodes;                       // [nch][2 maxn]
   double *bk_t;                            // [nch][2 maxn]
   int32_t *bk_pop;                         // [nch][2 maxn]
@@ -339,7 +341,7 @@ struct UgArgs {
   int32_t *prop;                           // [nch][2]: topology changed, tmrca changed
   double *slidew;                          // [nch] the slide's Hastings term
   // predraw: the proposal draws the acceptance uniform itself, right after
-  // its own draws, into ustore [nch] (an HKY locus always draws it, so the
+  // its own draws, and keeps its logarithm in ustore [nch] (an HKY locus always draws it, so the
   // stream's order is the reference's); otherwise the decision draws it
   int predraw;
   double *ustore;
@@ -352,6 +354,8 @@ struct UgArgs {
   const double *u_cl;                      // [nch][nloci] mutation rates
   int32_t *bk_A;                           // [nch][2 maxn] alleles before the proposal
   double *bk_dl;                           // [nch][2 maxn] branch terms before the proposal
+  double *lallele;                         // [nch] the allele step: its log deviate
+  int32_t *neg;                            // [nch] and its sign
   double *swnew;                           // [nch] proposed G.pdg
   double *aterm;                           // [nch] the allele proposal's Hastings term
   double *holdsis;                         // [nch] the new sister's term before the update
@@ -363,6 +367,7 @@ struct UgArgs {
   const double *nfc, *nhcc;
   int32_t *cc;                             // committed weights [items][T]
   double *fc, *hcc;
+  // per listed chain, and per chain and locus, whatever k
   int32_t *ag_cc;                          // the chains' summed weights [nch][T]
   double *ag_fc, *ag_hcc;
   double *qint;                            // [nch][nth] the chains' integrals
@@ -375,6 +380,7 @@ struct UgArgs {
   int32_t *nacc, *ntopo;                   // [nch][nloci] accepted proposals, accepted topology changes
 };
 enum { UG_E_SLIDE = 1, UG_E_ROOTTIME = 2, UG_E_ISFAIL = 3, UG_E_TERM = 4, UG_E_TREE = 5 };
+int ug_loci_per_launch(int nloci, int maxn);
 void launch_ug_propose(const UgArgs &a, cudaStream_t st);
 void launch_ug_sw(const UgArgs &a, cudaStream_t st);  // k_sw.cu
 void launch_ug_decide(const UgArgs &a, cudaStream_t st);

@@ -474,25 +474,29 @@ float2 split(double v)
 // rounded one at a time (no contraction), as the reference writes them.
 __global__ void __launch_bounds__(32) k_ug_sw(UgArgs a)
 {
-  const int w = blockIdx.x, lane = threadIdx.x;
-  const int ci = a.chains[w], item = ci * a.nloci + a.locus;
+  const int wj = blockIdx.x, w = wj % a.nch, locus = a.locus + wj / a.nch, lane = threadIdx.x;
+  const int ci = a.chains[w], item = ci * a.nloci + locus;
   const ItemDev it = a.items[item];
   const int n = it.n, maxnl = 2 * a.maxn;
   const NodeRec *nd = a.nodes + it.node_off;
   const double *t = a.t64 + it.node_off;
-  const int32_t *A = a.alleles + it.al_off;
+  int32_t *A = a.alleles + it.al_off;
   double *dl = a.dlike + it.dl_off;
-  const int32_t *bka = a.bk_A + (size_t)w * maxnl;
-  const double *bkd = a.bk_dl + (size_t)w * maxnl;
-  const NodeRec *bkn = a.bk_nodes + (size_t)w * maxnl;
-  const int32_t *eo = a.edges + 4 * (size_t)w;
+  const int32_t *bka = a.bk_A + (size_t)wj * maxnl;
+  const double *bkd = a.bk_dl + (size_t)wj * maxnl;
+  const NodeRec *bkn = a.bk_nodes + (size_t)wj * maxnl;
+  const int32_t *eo = a.edges + 4 * (size_t)wj;
   const int edge = eo[0], freed = eo[1], oldsis = eo[2], newsis = eo[3];
-  const double u = a.u_cl[(size_t)w * a.nloci + a.locus];
+  const double u = a.u_cl[(size_t)w * a.nloci + locus];
   const int e[3] = {edge, newsis, nd[edge].down};
-  // the proposal drew the freed node's allele (bka holds the alleles before)
-  const int oldA = bka[freed], newA = A[freed], dA = newA - oldA;
+  // finishSWupdateA's allele draw (update_gtree_common.cpp:2219-2362): a
+  // geometric step whose parameter comes from the freed node's neighbours'
+  // distances, signed by bitran, clamped to the locus's range (bka holds the
+  // alleles before)
+  const int oldA = bka[freed];
   double holdsis = 0.0, oldlikeadj = 0.0, geotermnew = 0.0;
   bool fdown = false;
+  int newA = 0;
   if (lane == 0) {
     holdsis = (newsis != oldsis) ? dl[newsis] : 0.0;
     fdown = bkn[freed].down != -1;
@@ -506,12 +510,20 @@ __global__ void __launch_bounds__(32) k_ug_sw(UgArgs a)
       }
     geotermnew = j / ((double)(wsumdiff + j));
     if (geotermnew > 0.95) geotermnew = 0.95;
+    int dA = (int)ceil(a.lallele[wj] / log(1.0 - geotermnew)) - 1;  // geometric(), utilities.cpp:609-617
+    if (a.neg[wj]) dA = -dA;
+    const int minA = a.arange[2 * locus], maxA = a.arange[2 * locus + 1];
+    if (dA >= 0) newA = (maxA < oldA + dA) ? maxA : oldA + dA;
+    else newA = (minA > oldA + dA) ? minA : oldA + dA;
+    A[freed] = newA;
   }
+  newA = __shfl_sync(0xffffffffu, newA, 0);
+  const int dA = newA - oldA;
   // The four branch terms, one lane each through one code path: lane 0 the
   // old sister's branch, lane 1 + i the branch above e[i], from the alleles
   // after the draw.  -(len * u) is the reference's (-len) * u exactly:
   // rounding to nearest is symmetric in sign.
-  auto allele = [&](int v) { return A[v]; };
+  auto allele = [&](int v) { return v == freed ? newA : bka[v]; };
   bool has = false;
   int d = 0;
   double len = 0.0;
@@ -559,9 +571,9 @@ __global__ void __launch_bounds__(32) k_ug_sw(UgArgs a)
     const double adA = (double)abs(dA);
     const double at = __dadd_rn(__dmul_rn(adA, log(1 - geotermold)), log(geotermold)) -
                       __dadd_rn(__dmul_rn(adA, log(1 - geotermnew)), log(geotermnew));
-    a.aterm[w] = at;
-    a.holdsis[w] = holdsis;
-    a.swnew[w] = 0.0 + (a.pdg[item] + __dadd_rn(likeadj, -oldlikeadj));
+    a.aterm[wj] = at;
+    a.holdsis[wj] = holdsis;
+    a.swnew[wj] = 0.0 + (a.pdg[item] + __dadd_rn(likeadj, -oldlikeadj));
   }
 }
 
@@ -666,7 +678,7 @@ void launch_sw_fast(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int 
   else sw_fast_launch<16, 5>(P, reqs, nreq, maxn, 0, result, status, st);
 }
 
-void launch_ug_sw(const UgArgs &a, cudaStream_t st) { k_ug_sw<<<a.nch, 32, 0, st>>>(a); }
+void launch_ug_sw(const UgArgs &a, cudaStream_t st) { k_ug_sw<<<a.nch * a.k, 32, 0, st>>>(a); }
 
 void launch_sw_fp64(const Pools &P, const ReqDev *reqs, int nreq, double *result,
                     int32_t *status, cudaStream_t st)

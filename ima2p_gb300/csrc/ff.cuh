@@ -61,6 +61,25 @@ __device__ __forceinline__ ff ff_split(double z)
   return ff_make(h, (float)(lo & 0x1fffffff) * __int_as_float((e - 52) << 23));
 }
 
+// (float)z and (float)(z - hi), both to nearest, of a double that is not
+// negative, on the integer pipe
+__device__ __forceinline__ float2 ff_round(double z)
+{
+  const int hi = __double2hiint(z);
+  const uint32_t lo = (uint32_t)__double2loint(z);
+  const int e = (hi >> 20) - 896;  // the float's biased exponent
+  if (e < 60 || e > 253) {
+    const float h = (float)z;
+    return make_float2(h, (float)(z - (double)h));
+  }
+  uint32_t m = ((uint32_t)(hi & 0xfffff) << 3) | (lo >> 29);  // 23 bits
+  const uint32_t rest = lo & 0x1fffffffu;                       // in units of 2^-29 of the last
+  m += rest > 0x10000000u || (rest == 0x10000000u && (m & 1u));
+  const int r = (int)(lo << 3) >> 3;                            // the rest less the carry, but for a tie to even below
+  const float h = __int_as_float((int)(((uint32_t)e << 23) + m));
+  return make_float2(h, (float)(rest == 0x10000000u && !((lo >> 29) & 1u) ? 0x10000000 : r) * __int_as_float((e - 52) << 23));
+}
+
 __device__ __forceinline__ ff ff_neg(ff a) { return ff_make(-a.hi, -a.lo); }
 __device__ __forceinline__ ff ff_sub(ff a, ff b) { return ff_add(a, ff_neg(b)); }
 

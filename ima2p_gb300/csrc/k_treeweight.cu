@@ -31,6 +31,7 @@
 // rounding, not bit for bit.
 #include "internal.h"
 
+#include <algorithm>
 #include <cfloat>
 
 #include "igamma.cuh"
@@ -64,6 +65,8 @@ __device__ void tw_fail(int32_t *err, int code, int who)
 // Pass 1, one warp per genealogy: lay out the events in shared memory, sort
 // them and write the sorted list to ev_t/ev_c at the genealogy's offset;
 // ev_n[g] = the number of events, or -1 for a genealogy the model cannot hold.
+constexpr int RANK_PER_LANE = 4;  // events of a lane sorted by their ranks
+
 __global__ void __launch_bounds__(32 * TW_WPB) k_tw_events(TwArgs a, int wpb)
 {
   extern __shared__ __align__(16) unsigned char sm[];
@@ -156,12 +159,7 @@ __global__ void __launch_bounds__(32 * TW_WPB) k_tw_events(TwArgs a, int wpb)
     ev_t[run + lane] = tv[lane];
     ev_c[run + lane] = ev_pack(EV_SPLIT, 0, 0, run + lane);
   }
-  int Pg = 1;
-  while (Pg < E) Pg <<= 1;
-  for (int i = E + lane; i < Pg; i += 32) {
-    ev_t[i] = __longlong_as_double(0x7ff0000000000000LL);  // +inf: after every event
-    ev_c[i] = ev_pack(EV_PAD, 0, 0, i);
-  }
+  const long long off = a.ev_off[g];
   if (__any_sync(~0u, bad)) {
     const int code = __reduce_max_sync(~0u, bad);
     if (lane == 0) {
@@ -169,6 +167,49 @@ __global__ void __launch_bounds__(32 * TW_WPB) k_tw_events(TwArgs a, int wpb)
       tw_fail(a.err, code, g);
     }
     return;
+  }
+  if (lane == 0) a.ev_n[g] = E;
+  if (E <= 32 * RANK_PER_LANE) {
+    // a few events: each one's rank is the number of earlier ones, counted
+    // by a lane for four of them at a time against every event in turn
+    // (broadcast loads; E^2 / 32 comparisons, where a bitonic sort's
+    // log^2 E passes load and store every event: 95 events 85 -> 61 us for
+    // 12,800 genealogies; four events a lane are as many as fit in registers).  Equal times leave a
+    // rank out, which the sum of the ranks tells: those are sorted below.
+    if (lane == 0 && (E & 1)) ev_t[E] = __longlong_as_double(0x7ff0000000000000LL);
+    __syncwarp();
+    long long key[RANK_PER_LANE];
+    int rank[RANK_PER_LANE];
+#pragma unroll
+    for (int q = 0; q < RANK_PER_LANE; q++) {
+      const int i = lane + 32 * q;
+      key[q] = i < E ? __double_as_longlong(ev_t[i]) : 0;
+      rank[q] = 0;
+    }
+    const longlong2 *pair = reinterpret_cast<const longlong2 *>(ev_t);
+    for (int j = 0; j < (E + 1) / 2; j++) {
+      const longlong2 v = pair[j];
+#pragma unroll
+      for (int q = 0; q < RANK_PER_LANE; q++) rank[q] += (v.x < key[q]) + (v.y < key[q]);
+    }
+    int sum = 0;
+#pragma unroll
+    for (int q = 0; q < RANK_PER_LANE; q++) sum += lane + 32 * q < E ? rank[q] : 0;
+    if (__reduce_add_sync(~0u, sum) == E * (E - 1) / 2) {
+#pragma unroll
+      for (int q = 0; q < RANK_PER_LANE; q++)
+        if (lane + 32 * q < E) {
+          a.ev_t[off + rank[q]] = __longlong_as_double(key[q]);
+          a.ev_c[off + rank[q]] = ev_c[lane + 32 * q];
+        }
+      return;
+    }
+  }
+  int Pg = 1;
+  while (Pg < E) Pg <<= 1;
+  for (int i = E + lane; i < Pg; i += 32) {
+    ev_t[i] = __longlong_as_double(0x7ff0000000000000LL);  // +inf: after every event
+    ev_c[i] = ev_pack(EV_PAD, 0, 0, i);
   }
   __syncwarp();
 
@@ -192,19 +233,25 @@ __global__ void __launch_bounds__(32 * TW_WPB) k_tw_events(TwArgs a, int wpb)
       __syncwarp();
     }
   }
-  const long long off = a.ev_off[g];
   for (int j = lane; j < E; j += 32) {
     a.ev_t[off + j] = ev_t[j];
     a.ev_c[off + j] = ev_c[j];
   }
-  if (lane == 0) a.ev_n[g] = E;
 }
 
 // Pass 2, the sweep (update_gtree_common.cpp:1827-1927): one group of GW
-// lanes per genealogy (GW = the smallest power of two >= npops), 32/GW
+// lanes per genealogy (GW = the smallest power of two >= npops), gpw
 // genealogies per warp, taken in the order perm gives (most events first) so
 // that a warp's groups sweep about as many events each.  Lane l of a group
 // owns population l of the current period.
+//
+// A sweep is a chain of FP64 operations, and the groups of a warp wait for
+// each other's splits.  So a warp carries one genealogy while that makes at
+// most TW_SWEEP_WARPS warps an SM, and up to 32/GW of them in larger batches,
+// which the FP64 pipe bounds: 640 genealogies of 90 events 78 -> 54 us by
+// themselves, but beside other kernels of FP64 chains (the genealogy update's)
+// more warps cost more than they gain, hence 2 an SM (2.40 ms, 2.66 at 8);
+// 12,800 genealogies 154 -> 145 from the even spread of one-warp CTAs.
 //
 // With MERGE (npops < GW: a group lane without a population), lane npops
 // carries G->length and G->tlength through the same two multiply-adds the
@@ -213,21 +260,20 @@ __global__ void __launch_bounds__(32 * TW_WPB) k_tw_events(TwArgs a, int wpb)
 // across it and 0 after it, each factor exact -- so the FP64 pipe does 8
 // operations per event instead of 12, with the reference's values.
 template <int GW, bool MERGE>
-__global__ void __launch_bounds__(32 * TW_WPB) k_tw_sweep(TwArgs a, int wpb, int gbytes)
+__global__ void __launch_bounds__(32) k_tw_sweep(TwArgs a, int gpw, int gbytes)
 {
   extern __shared__ __align__(16) unsigned char sm[];
-  constexpr int GPW = 32 / GW;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x;
   const int grp = lane / GW, gl = lane % GW;
   const unsigned gmask = GW == 32 ? 0xffffffffu : ((1u << GW) - 1) << (grp * GW);
-  const int slot = (blockIdx.x * wpb + warp) * GPW + grp;
-  if (slot >= a.ngen) return;  // whole groups only
+  const int slot = blockIdx.x * gpw + grp;
+  if (grp >= gpw || slot >= a.ngen) return;  // whole groups only
   const int g = a.perm[slot];
   const int E = a.ev_n[g];
   if (E < 0) return;  // pass 1 rejected it
   const TwModel &M = *a.model;
   const int npops = M.npops, nsplit = npops - 1, T = M.T, MM = M.M;
-  double *fc_s = reinterpret_cast<double *>(sm + (size_t)(warp * GPW + grp) * gbytes);
+  double *fc_s = reinterpret_cast<double *>(sm + (size_t)grp * gbytes);
   double *fm_s = fc_s + T;
   int *cc_s = reinterpret_cast<int *>(fm_s + MM);
   int *mc_s = cc_s + T;
@@ -262,8 +308,7 @@ __global__ void __launch_bounds__(32 * TW_WPB) k_tw_sweep(TwArgs a, int wpb, int
   };
   const bool lenlane = MERGE && gl == npops;
   // one event: returns true when the genealogy is found bad
-  auto event = [&](const double t, const uint32_t c) -> bool {
-    const double dt = t - last;
+  auto event = [&](const double t, const double dt, const uint32_t c) -> bool {
     const bool before = __double_as_longlong(t) < lsb, lbefore = __double_as_longlong(last) < lsb;
     const int w = npops - k;
     if constexpr (MERGE) {
@@ -363,10 +408,11 @@ __global__ void __launch_bounds__(32 * TW_WPB) k_tw_sweep(TwArgs a, int wpb, int
     if (j + 5 < E) { q1 = et[j + 5]; r1 = ec[j + 5]; }
     if (j + 6 < E) { q2 = et[j + 6]; r2 = ec[j + 6]; }
     if (j + 7 < E) { q3 = et[j + 7]; r3 = ec[j + 7]; }
-    if (event(t0, c0)) break;
-    if (j + 1 < E && event(t1, c1)) break;
-    if (j + 2 < E && event(t2, c2)) break;
-    if (j + 3 < E && event(t3, c3)) break;
+    const double d0 = t0 - last, d1 = t1 - t0, d2 = t2 - t1, d3 = t3 - t2;
+    if (event(t0, d0, c0)) break;
+    if (j + 1 < E && event(t1, d1, c1)) break;
+    if (j + 2 < E && event(t2, d2, c2)) break;
+    if (j + 3 < E && event(t3, d3, c3)) break;
   }
   if (!bad && nsum != 1) bad = TW_E_COUNT;
   if (bad) {
@@ -551,6 +597,14 @@ __global__ void __launch_bounds__(128) k_tp_final(TwProbArgs a)
 // forward the chain's counts are added up (each node time twice, once per
 // daughter edge, as the reference counts them) and the item's length is
 // saved; going back (o and n exchanged by the caller) the length is restored.
+//
+// The FP64 pipe (1/64 of the FP32 rate) bounds it: times, which are not
+// negative, are compared as integers, the float-float copy is cut on the
+// integer pipe, and the division by what is the same for a whole chain goes by
+// its reciprocal and two corrections with the exact remainder, which give the
+// correctly rounded quotient (Markstein 1990): 8 FP64 operations a time, 25
+// before.  128 chains x 100 loci of 96 genes: 157 -> 106 us, and back on half of
+// them 105 -> 75.
 constexpr int BAND_WPB = 8;  // chain-loci (warps) per block
 constexpr int RY_STAGE_MAX = 3000;  // loci staged in shared memory (48 KB of rows)
 
@@ -566,16 +620,28 @@ __global__ void __launch_bounds__(32 * BAND_WPB) k_band(BandArgs a)
   const double *P = a.prm + 5 * (size_t)c;
   const int period = (int)P[0];
   const double o = P[1], n = P[2], tu = P[3], td = P[4];
+  // Both sides as base + (t - base) factor / width (below the first split
+  // base 0, which is t n / o; above it the reference's td - (td - n) (td - t)
+  // / (td - o), whose signs change no rounding), so that lanes on either side
+  // go through the same operations.
+  const bool last = period == a.last - 1;
+  const double base_lo = period == 0 ? 0.0 : tu, width_lo = o - base_lo, width_hi = td - o;
+  const double r = 1.0 / (lane & 1 ? width_hi : width_lo);
+  const double r_lo = __shfl_sync(~0u, r, 0), r_hi = __shfl_sync(~0u, r, 1);
+  const double f_lo = n - base_lo, f_hi = td - n;
+  const long long ob = __double_as_longlong(o), ub = __double_as_longlong(tu), db = __double_as_longlong(td);
   auto band = [&](double t, int *lo, int *hi) -> double {
-    if (t <= o && t > tu) {
-      (*lo)++;
-      return period == 0 ? t * n / o : tu + (t - tu) * (n - tu) / (o - tu);
-    }
-    if (t > o && t < td) {
-      (*hi)++;
-      return period == a.last - 1 ? t + n - o : td - (td - n) * (td - t) / (td - o);
-    }
-    return t;
+    const long long b = __double_as_longlong(t);
+    const bool below = b <= ob;
+    if (b <= ub || b >= db) return t;
+    if (below) (*lo)++;
+    else (*hi)++;
+    if (last && !below) return t + n - o;
+    const double base = below ? base_lo : td, d = below ? width_lo : width_hi, r = below ? r_lo : r_hi;
+    const double x = (t - base) * (below ? f_lo : f_hi);
+    double q = x * r;
+    q = __fma_rn(__fma_rn(-q, d, x), r, q);
+    return base + __fma_rn(__fma_rn(-q, d, x), r, q);
   };
   int lo = 0, hi = 0, mlo = 0, mhi = 0;
   const int32_t *mo = a.moff + off + item;
@@ -587,8 +653,7 @@ __global__ void __launch_bounds__(32 * BAND_WPB) k_band(BandArgs a)
     const double tn = band(t, &lo, &hi);
     if (lo + hi != moved) {
       a.t64[off + k] = tn;
-      const float h = (float)tn;
-      a.tff[off + k] = make_float2(h, (float)(tn - (double)h));
+      a.tff[off + k] = ff_round(tn);
     }
     for (int j = mo[k]; j < mo[k + 1]; j++) a.mig_t[mb + j] = band(a.mig_t[mb + j], &mlo, &mhi);
   }
@@ -705,6 +770,8 @@ int launch_gather_rows(const float *rows, int rowlen, const int32_t *groups, int
   return 0;
 }
 
+constexpr int TW_SWEEP_WARPS = 2;
+
 size_t tw_stage_bytes(const TwModel &h) { return ((size_t)(h.T + h.M) * 12 + 15) / 16 * 16; }
 
 bool tw_fits(int P) { return (size_t)P * 12 <= 200 * 1024; }
@@ -713,10 +780,9 @@ template <int GW, bool MERGE>
 static void launch_sweep(const TwArgs &a, const TwModel &h, cudaStream_t st)
 {
   const size_t per = tw_stage_bytes(h);
-  const int wpb = TW_WPB;
-  const size_t smem = per * (32 / GW) * wpb;
-  const int per_block = wpb * (32 / GW);
-  k_tw_sweep<GW, MERGE><<<(a.ngen + per_block - 1) / per_block, 32 * wpb, smem, st>>>(a, wpb, (int)per);
+  const int warps = TW_SWEEP_WARPS * 152;
+  const int gpw = std::min(32 / GW, (a.ngen + warps - 1) / warps);
+  k_tw_sweep<GW, MERGE><<<(a.ngen + gpw - 1) / gpw, 32, per * gpw, st>>>(a, gpw, (int)per);
 }
 
 int launch_treeweight(const TwArgs &a, const TwModel &h, cudaStream_t st)

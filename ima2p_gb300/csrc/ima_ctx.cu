@@ -294,6 +294,11 @@ struct ima_ctx {
   bool tw_ready = false;
   double *d_logfact = nullptr;
   int32_t *d_twerr = nullptr;
+  // what d_twin holds of the resident genealogies' processing order and event
+  // offsets (twin_dev null: nothing)
+  const void *twin_dev = nullptr;
+  std::vector<int32_t> twin_perm;
+  std::vector<long long> twin_evoff;
   void *d_twin = nullptr, *d_twout = nullptr, *d_tpbuf = nullptr;
   size_t twin_cap = 0, twout_cap = 0, tpbuf_cap = 0;
   int tw_ngen = 0, tw_ntv = 0;
@@ -3371,6 +3376,7 @@ extern "C" int ima_gpu_treeweight(ima_ctx *c, int ngen, const int32_t *node_off,
                                  ngen * 4ul});
   const size_t outb = carve_size({ngen * T * 4, ngen * MM * 4, ngen * 4ul, ngen * T * 8, ngen * T * 8,
                                   ngen * MM * 8, 2 * ngen * 8ul});
+  c->twin_dev = nullptr;
   int r = grow(c, &c->d_twin, &c->twin_cap, inb, "treeweight inputs");
   r = r ? r : grow(c, &c->d_twout, &c->twout_cap, outb, "treeweight weights");
   if (r) return r;
@@ -3900,11 +3906,10 @@ static int band_run(ima_ctx *c, int nch, const int32_t *chains, const int32_t *p
   c->launches += nk - 1;
   r = c->cuda(cudaGetLastError(), "band launch");
   if (!r && counts && !inverse) r = c->cuda(cudaMemcpyAsync(counts, c->d_bcnt, 16ul * nch, cudaMemcpyDeviceToHost, c->st), "band counts");
-  // the parameter block is host memory of this call: wait for its copy
-  r = r ? r : c->cuda(cudaStreamSynchronize(c->st), "band");
+  // (the parameter block is pageable host memory: its copy has been staged)
+  if (sync) r = r ? r : c->cuda(cudaStreamSynchronize(c->st), "band");
   if (!r) dev_newer(c, nch, chains);
   if (d_chains) *d_chains = d_ch;
-  (void)sync;
   return r;
 }
 
@@ -3991,9 +3996,19 @@ static int chain_weights_run(ima_ctx *c, int nch, const int32_t *chains, const d
   a.lens = co.take<double>(2ul * ni);
   a.len_out = c->d_len;
   a.err = c->d_twerr;
-  r = c->cuda(cudaMemcpyAsync(d_perm, perm.data(), ns * 4, cudaMemcpyHostToDevice, c->st), "weights");
-  r = r ? r : c->cuda(cudaMemcpyAsync(d_evoff, evoff.data(), (ni + 1) * 8ul, cudaMemcpyHostToDevice, c->st), "weights");
-  r = r ? r : c->cuda(cudaMemcpyAsync(c->d_tvr, c->h_tvr.data(), c->h_tvr.size() * 8, cudaMemcpyHostToDevice, c->st), "weights");
+  // the order and the offsets follow from the genealogies' sizes and migration
+  // counts: copied when they are not what the device holds already (a copy of
+  // this size from pageable memory waits for the work before it)
+  if (c->twin_dev != c->d_twin || c->twin_perm != perm || c->twin_evoff != evoff) {
+    c->twin_dev = nullptr;
+    r = c->cuda(cudaMemcpyAsync(d_perm, perm.data(), ns * 4, cudaMemcpyHostToDevice, c->st), "weights");
+    r = r ? r : c->cuda(cudaMemcpyAsync(d_evoff, evoff.data(), (ni + 1) * 8ul, cudaMemcpyHostToDevice, c->st), "weights");
+    if (r) return r;
+    c->twin_dev = c->d_twin;
+    c->twin_perm = std::move(perm);
+    c->twin_evoff = std::move(evoff);
+  }
+  r = c->cuda(cudaMemcpyAsync(c->d_tvr, c->h_tvr.data(), c->h_tvr.size() * 8, cudaMemcpyHostToDevice, c->st), "weights");
   r = r ? r : c->cuda(cudaMemsetAsync(c->d_twerr, 0, 8, c->st), "weights");
   if (r) return r;
   c->tw_ngen = 0;
@@ -4129,13 +4144,12 @@ extern "C" int ima_gpu_changet_ry1_sweep(ima_ctx *c, int nch, const int32_t *cha
   }
   r = commit(c, nch * nl, ci.data(), li.data(), acc_items.data(), true, true);
   if (!r && !rc.empty())
-    r = band_run(c, (int)rc.size(), rc.data(), rp.data(), ro.data(), rn.data(), ru.data(), rd.data(), 1, nullptr, true);
-  if (!r && probg) {  // the resident p(G) of each chain after the decision
-    std::vector<double> all(c->nchains);
+    r = band_run(c, (int)rc.size(), rc.data(), rp.data(), ro.data(), rn.data(), ru.data(), rd.data(), 1, nullptr, false);
+  std::vector<double> all(c->nchains);
+  if (!r && probg)  // the resident p(G) of each chain after the decision
     r = c->cuda(cudaMemcpyAsync(all.data(), c->d_probg, c->nchains * 8ul, cudaMemcpyDeviceToHost, c->st), "probg");
-    r = r ? r : c->cuda(cudaStreamSynchronize(c->st), "probg");
-    for (int k = 0; !r && k < nch; k++) probg[k] = all[chains[k]];
-  }
+  r = r ? r : c->cuda(cudaStreamSynchronize(c->st), "split-time update");
+  for (int k = 0; !r && probg && k < nch; k++) probg[k] = all[chains[k]];
   return r;
 }
 

@@ -9,9 +9,12 @@
 //
 // k_surf_split counts, per point, how many of up to 256 evenly spaced
 // genealogies lie within MARGIN of the point's bound.  A point with at least
-// one in DENSE_FRAC is taken here, the others by the screen.  The line: one
-// term here costs about 4-8 ps (10-26 columns), one refined candidate about
-// 180 ps and one screened term 0.3 ps, so the two meet at 3-6% of the terms.
+// one in DENSE_FRAC is taken here, the others by the screen.  The line lies
+// where a refined candidate costs as much as twelve terms here: 500 points x
+// 100,000 genealogies of three widths take 544, 482 and 368 us with one in 12,
+// 559, 543 and 399 with one in 16, 596, 556 and 296 with one in 8 (all here:
+// 518, 519, 470; 1,300 points of 26 columns 1,670, 1,100 and 398 against 1,930,
+// 1,790 and 1,790).
 //
 // k_surf_dense: lanes are points, phi in registers; a CTA's 8 warps share 32
 // points and take a tile's 64 genealogies by turns, reading each statistic
@@ -33,7 +36,7 @@ namespace {
 
 constexpr int DT = SURF_DENSE_TILE;
 constexpr int DW = 8;            // warps per CTA, sharing 32 points
-constexpr int DENSE_FRAC = 16;   // dense from one sampled genealogy in 16 within MARGIN
+constexpr int DENSE_FRAC = 12;   // dense from one sampled genealogy in 12 within MARGIN
 constexpr float DENSE_OVF = 40.0f;  // nats above ref at which a point is left to the retake: w^2 and its sums stay in FP32's range
 __device__ float2 d_exp64[64];  // 2^(j/64) as float-float
 

@@ -487,7 +487,7 @@ extern "C" int ima_gpu_create(int device, ima_ctx **out)
   cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device);
   cudaDeviceGetAttribute(&c->pageable_access, cudaDevAttrPageableMemoryAccess, device);
   if (sw_init_tables() != 0 || hky_init_tables() != 0 || surf_init_tables() != 0 ||
-      margin_init_tables() != 0 || popmig_init_tables() != 0 || is_init_tables() != 0) {
+      margin_init_tables() != 0 || popmig_init_tables() != 0) {
     delete c;
     return IMA_ERR_CUDA;
   }

@@ -183,7 +183,6 @@ struct PopmigArgs {
   int32_t *err;                            // first failing series / fraction (0 = none)
 };
 int popmig_init_tables();
-int is_init_tables();
 int popmig_log_block(int most);  // lognx for at most `most` points of one term
 int popmig_chunks(int G, int nblocks, int expo);
 // uniform prior: n points in blocks of 2^lognx of one term each

@@ -8,20 +8,14 @@
 // does not change), finds the node whose daughters carry {0,1}, and takes the
 // branch that carries the mutation.  Labels live in shared memory, laid out
 // [node][thread] so the walks of a warp hit distinct banks.  log(t*u) is
-// formed per site, by a table and fixed point (the FP64 pipe, 1/64 of the FP32
-// rate, bounded the kernel: 12,800 chain-loci of 96 genes 103 us, 83 so); the site terms are then added in site order by one
+// formed per site in FP64; the site terms are then added in site order by one
 // thread, so the FP64 sum has the reference's association.  Each site's
 // mutation branch is cached per chain-locus and reused while its topology is
 // unchanged (the context clears the cache of every item whose topology it
 // uploads), so re-timing updates skip the labelling.
-#include "fxexp.cuh"
 #include "internal.h"
 
-const FxLogTab &fx_log_table();  // k_popmig.cu
-
 namespace {
-
-__device__ FxLogTab d_is_log;
 
 constexpr int IS_BS = 64;
 constexpr double REJECT_IS = -1000000000.0;  // imamp.hpp:157
@@ -147,9 +141,7 @@ __global__ void __launch_bounds__(IS_BS) k_is(Pools P, const ReqDev *reqs, doubl
       if (br == 2) t = branch64(s.nd, s.t, a) + branch64(s.nd, s.t, b);
       else if (br == 1) t = branch64(s.nd, s.t, b);
       else t = branch64(s.nd, s.t, a);
-      const double x = t * R.u;
-      const int ex = __double2hiint(x) >> 20;  // and the sign
-      v = ex >= 1023 - 64 && ex < 1023 + 64 ? fx_ln(x, d_is_log) : log(x);
+      v = log(t * R.u);
     }
     s.sv[site] = v;
     s.sst[site] = st;
@@ -231,11 +223,6 @@ void launch_is(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS,
   size_t sm = is_smem(maxn, maxS);
   if (sm > 48 * 1024) cudaFuncSetAttribute(k_is, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   k_is<<<nreq, IS_BS, sm, st>>>(P, reqs, result, status, site_node);
-}
-
-int is_init_tables()
-{
-  return cudaMemcpyToSymbol(d_is_log, &fx_log_table(), sizeof(FxLogTab)) == cudaSuccess ? 0 : -1;
 }
 
 void launch_is_sumlogk(const Pools &P, int item, int locus, int maxn, int maxS, int *d_flag,

@@ -413,26 +413,16 @@ __global__ void k_popmig_merge(PopmigArgs a, int nchunks, const double *part, do
 }  // namespace
 
 // the tables, made once per process (long double is slow in software on aarch64)
-const FxLogTab &fx_log_table()
-{
-  static const FxLogTab t = [] {
-    FxLogTab v{};
-    for (int j = 0; j < FX_TAB; j++) {
-      const uint64_t r = (4294967296ull * FX_TAB + FX_TAB + j - 1) / (FX_TAB + j);  // ceil
-      v.r[j] = (uint32_t)(r - 1);
-      v.l[j] = j ? (uint64_t)(-log2l((long double)r / 4294967296.0L) * 18446744073709551616.0L) : 0ull;
-    }
-    return v;
-  }();
-  return t;
-}
-
 static const PfTables &pf_tables()
 {
   static const PfTables t = [] {
     PfTables v{};
-    for (int j = 0; j < FX_TAB; j++) v.ex[j] = (uint64_t)(exp2l((long double)j / FX_TAB) * 9223372036854775808.0L);
-    v.lg = fx_log_table();
+    for (int j = 0; j < FX_TAB; j++) {
+      v.ex[j] = (uint64_t)(exp2l((long double)j / FX_TAB) * 9223372036854775808.0L);
+      const uint64_t r = (4294967296ull * FX_TAB + FX_TAB + j - 1) / (FX_TAB + j);  // ceil
+      v.lg.r[j] = (uint32_t)(r - 1);
+      v.lg.l[j] = j ? (uint64_t)(-log2l((long double)r / 4294967296.0L) * 18446744073709551616.0L) : 0ull;
+    }
     for (int k = 1; k < PF_RCP; k++) {
       const long double w = 1.0L / k;
       v.rcp[k] = make_float2((float)w, (float)(w - (long double)(float)w));

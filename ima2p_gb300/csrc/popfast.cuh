@@ -27,6 +27,35 @@ constexpr int PF_AMAX = 192;   // counts below this
 constexpr int PF_RCP = PF_AMAX + PF_NMAX;  // reciprocals 1 / k, k < PF_RCP
 constexpr double PF_LOG2E = 1.4426950408889634074;
 
+// log2 of a normal positive double: integer part, and fraction in units of
+// 2^-64 within 2^-60.  1 + j/512 <= m < 1 + (j+1)/512: u = m R_j - 1 >= 0 with
+// R_j = 2^-32 ceil(2^32 512 / (512 + j)), then -log2 R_j + log2(1 + u).
+struct FxLogTab {
+  uint32_t r[FX_TAB];   // R_j 2^32 - 1 (R_0 = 1)
+  uint64_t l[FX_TAB];   // -log2(R_j) 2^64, R_j = (r + 1) 2^-32
+};
+constexpr uint64_t FX_P0 = 0xb8aa3b295c17f041ull;  // 2^63
+constexpr uint64_t FX_P1 = 0xb8aa3b295bb827ull;    // 2^64
+constexpr uint32_t FX_P2 = 0x7b1c276bu;            // 2^48
+constexpr uint32_t FX_P3 = 0x5c54fcu;              // 2^48
+constexpr uint32_t FX_P4 = 0x4991u;                // 2^48
+
+__device__ __forceinline__ uint64_t fx_log2(double z, const FxLogTab &T, int *e)
+{
+  const uint64_t b = fx_bits(z);
+  *e = (int)(b >> 52) - 1023;
+  const int j = (int)(b >> 43) & (FX_TAB - 1);
+  const uint64_t m = (b << 11) | (1ull << 63);  // 2^63
+  const uint64_t u = fx_mul64(m, T.r[j]) + (m >> 32) - (1ull << 63);  // 2^63, below 2^-9 (1 + 2^-22)
+  const uint64_t rho = u << 9;  // 2^8 u, 2^64
+  const uint32_t r = (uint32_t)(rho >> 32), rl = (uint32_t)rho;
+  const uint32_t g3 = FX_P2 - fx_mulhi(r, FX_P3 - fx_mulhi(r, FX_P4));
+  const uint64_t g2 = FX_P1 - ((uint64_t)fx_mulhi(r, g3) << 16);
+  const uint64_t g1 = FX_P0 - ((fx_mul64(g2, r) + fx_mulhi((uint32_t)(g2 >> 32), rl)) >> 1);
+  const uint64_t y = fx_mul64(g1, r) + fx_mulhi((uint32_t)(g1 >> 32), rl);  // 2^63
+  return T.l[j] + (y >> 7);
+}
+
 __device__ __forceinline__ float pf_rcp(float a)
 {
   float r;

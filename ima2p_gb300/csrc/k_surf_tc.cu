@@ -28,7 +28,7 @@
 //              screen error of the point's lower bound, the values above that
 //              become candidates and go to a ring.
 //
-// 7.1 ms a call, 2.9 in the first pass and 3.7 in the second, against 20.3 with
+// 7.1 ms a call, 2.9 in the first pass and 3.6 in the second, against 20.3 with
 // bf16 operands split into two halves (three products), two 256-column
 // accumulators and one issuing thread; the first pass's products alone are 2.1.
 //

@@ -600,10 +600,12 @@ def edit_list_leg(ctx, api, wl, ci, li, u, par, steps):
     b64.run(use_graph=False)
     r64, _ = b64.results()
     b64.destroy()
+    if not np.array_equal(r_ff, r_full):
+        raise RuntimeError("edit-list and full HKY evaluations of the same genealogies differ")
     ms = statistics.median(tt)
     return {"value": round(len(ci) / (ms / 1e3), 1), "unit": "evals/s", "ms_per_step": round(ms, 5),
             "dirty_nodes_per_eval": 4, "recomputed_nodes_per_eval": round(nrec, 2),
-            "same_bits_as_full_evaluation": bool(np.array_equal(r_ff, r_full)),
+            "same_bits_as_full_evaluation": True,
             "error_vs_fp64_max_abs": float(np.abs(r_ff - r64).max())}
 
 

@@ -357,7 +357,9 @@ __host__ __device__ inline HkyLayout hky_layout_fast(int maxnl, bool ff)
 // recomputed node and entry) are listed in schedule order, x = (node - n) |
 // entry << 16, y = the daughters' entries (a tip's state), the internal
 // daughter first.  A full evaluation's list depends on the topology alone: it
-// is kept per item and read back while P.is_valid says so.  Loci whose masks
+// is kept per item and read back while P.is_valid says so.  The list of an
+// evaluation from edited edges is shorter; what of it does not fit in shared
+// memory goes to the same place, which ends the kept list.  Loci whose masks
 // pass HKY_MASK_WORDS, or whose patterns 16 bits, keep every pattern.
 constexpr int HKY_MASK_WORDS = 8192;
 __host__ __device__ inline bool hky_uniform(int n, int S)
@@ -664,7 +666,8 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
     if (full)
       for (int k = tid; k < n; k += BS) gtoff[k] = toff[k];
     __syncthreads();
-    if (full && tid == 0) P.is_valid[R.item] = 1;  // read by later launches only
+    // read by later launches only
+    if (tid == 0 && (full || tbase > 0)) P.is_valid[R.item] = full;
   }
 
   const size_t slot_stride = (size_t)nint * S4;

@@ -38,8 +38,8 @@ struct LocusHost {
   bool sumlogk_done = false;
 };
 
-// HKY requests of similar size, launched together (a launch's shared memory
-// is that of its largest chain-locus)
+// HKY requests launched together: of similar size (a launch's shared memory
+// is that of its largest chain-locus), a chain-locus once
 struct HkyBin {
   int off, n, maxn, maxs;
 };
@@ -1507,17 +1507,38 @@ static int build_batch(ima_ctx *c, Batch &b, int n, const int32_t *ci, const int
     const LocusDev &L = c->loci[li[k]].d;
     return L.model == IMA_MODEL_HKY ? (L.n + 31) / 32 : 0;
   };
+  // an HKY evaluation works in the chain-locus's own partials, so one that is
+  // listed again (with other parameters, say) takes a launch after the first
+  std::vector<int> again;  // earlier entries of a request's chain-locus; empty: none repeats
+  {
+    if ((int)c->pair_stamp.size() != c->nitems) c->pair_stamp.assign(c->nitems, -1);
+    const int gen = ++c->stamp_gen;
+    bool repeat = false;
+    for (int k : g[1]) {
+      int &stamp = c->pair_stamp[c->item_of(ci[k], li[k])];
+      repeat |= stamp == gen;
+      stamp = gen;
+    }
+    if (repeat) {
+      std::vector<int> seen(c->nitems, 0);
+      again.assign(n, 0);
+      for (int k : g[1]) again[k] = seen[c->item_of(ci[k], li[k])]++;
+    }
+  }
   for (int m = 1; m < 3; m++)
     std::stable_sort(g[m].begin(), g[m].end(), [&](int a, int b) {
+      if (m == 1 && !again.empty() && again[a] != again[b]) return again[a] < again[b];
       const int sa = size(a), sb = size(b);
       return sa != sb ? sa > sb : cost(a) > cost(b);
     });
-  // a launch per class, where it and the rest fill the device a few times
+  // and in the fast forms a launch per class, where it and the rest fill the
+  // device a few times
   b.bins.clear();
   for (size_t k = 0; k < g[1].size(); k++) {
     const LocusDev &L = c->loci[li[g[1][k]]].d;
-    if (k == 0 || (size(g[1][k]) != size(g[1][k - 1]) && b.bins.back().n >= 8 * c->nsm &&
-                   (int)(g[1].size() - k) >= 8 * c->nsm))
+    if (k == 0 || (!again.empty() && again[g[1][k]] != again[g[1][k - 1]]) ||
+        (prec != IMA_PREC_FP64 && size(g[1][k]) != size(g[1][k - 1]) && b.bins.back().n >= 8 * c->nsm &&
+         (int)(g[1].size() - k) >= 8 * c->nsm))
       b.bins.push_back({(int)k, 0, 0, 0});
     HkyBin &q = b.bins.back();
     q.n++;
@@ -1657,7 +1678,8 @@ static void hky_bins(const Pools &P, const Batch &b, int variant, cudaStream_t s
 {
   for (const HkyBin &q : b.bins) {
     const int o = b.nis + q.off;
-    if (b.prec == IMA_PREC_FP32) launch_hky_fp32(P, b.d_req + o, q.n, q.maxn, q.maxs, variant, b.d_res + o, b.d_st + o, st);
+    if (b.prec == IMA_PREC_FP64) launch_hky_fp64(P, b.d_req + o, q.n, q.maxn, b.d_res + o, b.d_st + o, st);
+    else if (b.prec == IMA_PREC_FP32) launch_hky_fp32(P, b.d_req + o, q.n, q.maxn, q.maxs, variant, b.d_res + o, b.d_st + o, st);
     else launch_hky_fast(P, b.d_req + o, q.n, q.maxn, q.maxs, variant, b.d_res + o, b.d_st + o, st);
   }
 }
@@ -1670,11 +1692,8 @@ static void enqueue(ima_ctx *c, Batch &b, cudaStream_t on = nullptr)
   if (b.nis)
     c->launch(IMA_K_IS, 0.0, [&] { launch_is(P, b.d_req, b.nis, b.maxn_is, b.maxs_is, b.d_res, b.d_st, nullptr, st); }, st);
   if (b.nhky) {
-    const ReqDev *r = b.d_req + b.nis;
-    if (b.prec == IMA_PREC_FP64)
-      c->launch(IMA_K_HKY_FP64, b.hky_bytes, [&] { launch_hky_fp64(P, r, b.nhky, b.maxn_hky, b.d_res + b.nis, b.d_st + b.nis, st); }, st);
-    else
-      c->launch(b.prec == IMA_PREC_FP32 ? IMA_K_HKY_FP32 : IMA_K_HKY_FAST, b.hky_bytes, [&] { hky_bins(P, b, b.hky_variant, st); }, st);
+    const int kind = b.prec == IMA_PREC_FP64 ? IMA_K_HKY_FP64 : b.prec == IMA_PREC_FP32 ? IMA_K_HKY_FP32 : IMA_K_HKY_FAST;
+    c->launch(kind, b.hky_bytes, [&] { hky_bins(P, b, b.hky_variant, st); }, st);
   }
   if (b.nsw) {
     const ReqDev *r = b.d_req + b.nis + b.nhky;

@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
     if (full)
       for (int k = tid; k < n; k += BS) gtoff[k] = toff[k];
     __syncthreads();
-    // read by later launches only
+    // read by later launches only (an item is in a launch once)
     if (tid == 0 && (full || tbase > 0)) P.is_valid[R.item] = full;
   }
 

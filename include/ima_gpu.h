@@ -162,7 +162,10 @@ int ima_gpu_get_dlikeA(ima_ctx *ctx, int ci, int li, int ai, double *dlikeA);
  * One launch over many chain-locus pairs of mixed models (the batched form
  * of the calls above, as changet_RY1 / updategenealogy make them,
  * update_t_RY.cpp:343-389, update_gtree.cpp:838-888).
- *   ci, li     : chain-locus pairs (may repeat loci and mix models)
+ *   ci, li     : chain-locus pairs (may repeat loci and mix models; an HKY
+ *                pair listed more than once, with other parameters say, is
+ *                evaluated in as many launches, and its last entry's partials
+ *                are the ones that a commit takes)
  *   u          : mutation rate scalar per pair
  *   kappa      : HKY kappa per pair; for SW pairs the branch-time scale tr
  *                of likelihoodSW (ignored for IS; NULL = 1.0)

@@ -1694,6 +1694,7 @@ static void enqueue(ima_ctx *c, Batch &b, cudaStream_t on = nullptr)
   if (b.nhky) {
     const int kind = b.prec == IMA_PREC_FP64 ? IMA_K_HKY_FP64 : b.prec == IMA_PREC_FP32 ? IMA_K_HKY_FP32 : IMA_K_HKY_FAST;
     c->launch(kind, b.hky_bytes, [&] { hky_bins(P, b, b.hky_variant, st); }, st);
+    c->launches += (long long)b.bins.size() - 1;
   }
   if (b.nsw) {
     const ReqDev *r = b.d_req + b.nis + b.nhky;
@@ -1906,7 +1907,7 @@ extern "C" int ima_gpu_batch_run(ima_ctx *c, int batch, int use_graph)
     c->launches -= nk;  // counted when replayed
   }
   r = c->cuda(cudaGraphLaunch(b.graph, c->st), "graph launch");
-  c->launches += (b.nis ? 1 : 0) + (b.nhky ? 1 : 0) + (b.nsw ? 1 : 0);
+  c->launches += (b.nis ? 1 : 0) + (int)b.bins.size() + (b.nsw ? 1 : 0);
   return r;
 }
 
@@ -1927,31 +1928,31 @@ extern "C" int ima_gpu_batch_autotune(ima_ctx *c, int batch, int reps, int *hky_
     Pools P = c->pools();
     cudaStream_t st = c->st;
     cudaEvent_t e0 = c->ev(), e1 = c->ev();
-    auto timed = [&](auto launch) -> float {
+    auto timed = [&](int kernels, auto launch) -> float {
       launch();
       cudaEventRecord(e0, st);
       for (int k = 0; k < reps; k++) launch();
       cudaEventRecord(e1, st);
       float ms = 0.f;
       if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) return -1.f;
-      c->launches += reps + 1;
+      c->launches += (reps + 1) * kernels;
       return ms / reps;
     };
-    auto pick = [&](int nvar, auto launch_v) -> int {
+    auto pick = [&](int nvar, int kernels, auto launch_v) -> int {
       std::vector<float> t(nvar);
-      for (int v = 0; v < nvar; v++) t[v] = timed([&] { launch_v(v); });
+      for (int v = 0; v < nvar; v++) t[v] = timed(kernels, [&] { launch_v(v); });
       int best = 0;
       for (int v = 1; v < nvar; v++)
         if (t[v] >= 0.f && t[v] < t[best]) best = v;
       return (t[0] >= 0.f && t[0] <= 1.02f * t[best]) ? 0 : best;
     };
     if (b.nhky) {
-      b.hky_variant = pick(HKY_FAST_VARIANTS, [&](int v) { hky_bins(P, b, v, st); });
+      b.hky_variant = pick(HKY_FAST_VARIANTS, (int)b.bins.size(), [&](int v) { hky_bins(P, b, v, st); });
     }
     if (b.nsw) {
       const ReqDev *rq = b.d_req + b.nis + b.nhky;
       const int off = b.nis + b.nhky;
-      b.sw_variant = pick(SW_FAST_VARIANTS, [&](int v) {
+      b.sw_variant = pick(SW_FAST_VARIANTS, 1, [&](int v) {
         launch_sw_fast(P, rq, b.nsw, b.maxn_sw, v, b.d_res + off, b.d_st + off, st);
       });
     }
@@ -2083,7 +2084,7 @@ extern "C" int ima_gpu_batch_sweep(ima_ctx *c, int batch, const uint8_t *accept,
     c->launches += 2;
     if (swap) enqueue_swap(c, swaptries, include_probg, seed);
   };
-  const int nk = (b.nis ? 1 : 0) + (b.nhky ? 1 : 0) + (b.nsw ? 1 : 0) + 2 + (swap ? 1 : 0);
+  const int nk = (b.nis ? 1 : 0) + (int)b.bins.size() + (b.nsw ? 1 : 0) + 2 + (swap ? 1 : 0);
   if (!use_graph || c->profiling) {
     body();
     return c->cuda(cudaGetLastError(), "sweep");

@@ -36,12 +36,14 @@ struct LocusHost {
   std::vector<int8_t> seq;
   std::vector<int32_t> mult;
   bool sumlogk_done = false;
+  bool uni = false;  // HKY: partials kept once per state (hky_uniform_entries)
 };
 
 // HKY requests launched together: of similar size (a launch's shared memory
-// is that of its largest chain-locus), a chain-locus once
+// is that of its largest chain-locus) and one kind of loci, a chain-locus once
 struct HkyBin {
   int off, n, maxn, maxs;
+  bool uni;  // as LocusHost
 };
 
 struct Batch {
@@ -575,6 +577,7 @@ static int add_locus(ima_ctx *c, int model, int n, int S, int tots, const int8_t
     }
   }
   if (mult) L.mult.assign(mult, mult + S);
+  if (model == IMA_MODEL_HKY) L.uni = hky_uniform_entries(n, S, seq);
   *li = (int)c->loci.size();
   c->loci.push_back(std::move(L));
   return IMA_OK;
@@ -1480,8 +1483,9 @@ static void batch_shape(const Batch &b, int *k)
   memcpy(k, v, sizeof(v));
 }
 
+// partial: the device fills in the HKY requests' edits
 static int build_batch(ima_ctx *c, Batch &b, int n, const int32_t *ci, const int32_t *li, const double *u,
-                       const double *kappa, const int32_t *edits, const int32_t *ai, int prec)
+                       const double *kappa, const int32_t *edits, const int32_t *ai, int prec, bool partial = false)
 {
   if (!c->nchains) return c->fail(IMA_ERR_STATE, "call ima_gpu_set_chains first");
   if (n < 1 || !ci || !li || !u) return c->fail(IMA_ERR_ARG, "empty or null request list");
@@ -1525,9 +1529,11 @@ static int build_batch(ima_ctx *c, Batch &b, int n, const int32_t *ci, const int
       for (int k : g[1]) again[k] = seen[c->item_of(ci[k], li[k])]++;
     }
   }
+  auto uni = [&](int k) { return (bool)c->loci[li[k]].uni; };
   for (int m = 1; m < 3; m++)
     std::stable_sort(g[m].begin(), g[m].end(), [&](int a, int b) {
       if (m == 1 && !again.empty() && again[a] != again[b]) return again[a] < again[b];
+      if (m == 1 && uni(a) != uni(b)) return uni(b);
       const int sa = size(a), sb = size(b);
       return sa != sb ? sa > sb : cost(a) > cost(b);
     });
@@ -1537,9 +1543,10 @@ static int build_batch(ima_ctx *c, Batch &b, int n, const int32_t *ci, const int
   for (size_t k = 0; k < g[1].size(); k++) {
     const LocusDev &L = c->loci[li[g[1][k]]].d;
     if (k == 0 || (!again.empty() && again[g[1][k]] != again[g[1][k - 1]]) ||
-        (prec != IMA_PREC_FP64 && size(g[1][k]) != size(g[1][k - 1]) && b.bins.back().n >= 8 * c->nsm &&
-         (int)(g[1].size() - k) >= 8 * c->nsm))
-      b.bins.push_back({(int)k, 0, 0, 0});
+        (prec != IMA_PREC_FP64 &&
+         (uni(g[1][k]) != uni(g[1][k - 1]) || (size(g[1][k]) != size(g[1][k - 1]) && b.bins.back().n >= 8 * c->nsm &&
+                                               (int)(g[1].size() - k) >= 8 * c->nsm))))
+      b.bins.push_back({(int)k, 0, 0, 0, uni(g[1][k])});
     HkyBin &q = b.bins.back();
     q.n++;
     q.maxn = std::max(q.maxn, L.n);
@@ -1550,10 +1557,34 @@ static int build_batch(ima_ctx *c, Batch &b, int n, const int32_t *ci, const int
   b.nis = (int)g[0].size();
   b.nhky = (int)g[1].size();
   b.nsw = (int)g[2].size();
-  // float-float HKY: 128-thread CTAs, 6 per SM, unless the batch is one wave
-  // of the 96-thread shape's 11 and more than one of 6 (1,600 chain-loci of 40
-  // genes: 41 us against 46; 12,800 of 12 to 180 genes: 861 against 741)
-  b.hky_variant = (prec == IMA_PREC_FAST && b.nhky > 6 * c->nsm && b.nhky <= 11 * c->nsm) ? 5 : 0;
+  // Launch shape of the fast HKY forms, for what a chain-locus's CTA has to do
+  // (partials of a full evaluation; of edited edges a quarter):
+  //  - 256 threads where one wave of such CTAs holds the launch (4 per SM,
+  //    FP32 6) and there is work for them: 64 chain-loci of 40 genes x 60
+  //    patterns 18 us and 19, x 100 19 and 20, x 150 25 and 22; of 100 genes x
+  //    300 patterns 300 take 102 and 73, 600 118 and 94; 800 of 40 x 200 47 and 53.
+  //    Where every pattern is kept, however little the work (64 of 40 x 60:
+  //    24 and 22; 128 of 200 x 2,000 3.58 and 2.02 ms).
+  //  - float-float, one wave of the 96-thread shape's 11 and more than one of
+  //    6: that shape (1,600 chain-loci of 40 genes: 41 us against 46; 12,800 of
+  //    12 to 180 genes: 861 against 741)
+  //  - else 128 threads, 6 CTAs per SM (FP32 12), float-float with every pattern
+  //    kept 8 (10,000 of 40 x 60: 407 and 374)
+  {
+    double work = 0.0;
+    int most = 0;
+    bool plain = false;
+    for (int k : g[1]) work += (double)cost(k);
+    for (const HkyBin &q : b.bins) {
+      most = std::max(most, q.n);
+      plain |= !q.uni;
+    }
+    work /= std::max(1, b.nhky) * (edits || partial ? 4.0 : 1.0);
+    b.hky_variant = 0;
+    if (most <= (prec == IMA_PREC_FP32 ? 6 : 4) * c->nsm && (plain || work >= 4000.0)) b.hky_variant = 2;
+    else if (prec == IMA_PREC_FAST && plain) b.hky_variant = 4;
+    else if (prec == IMA_PREC_FAST && b.nhky > 6 * c->nsm && b.nhky <= 11 * c->nsm) b.hky_variant = 5;
+  }
   b.order.clear();
   b.h_req.clear();
   b.maxn_is = b.maxs_is = b.maxn_hky = b.maxs_hky = b.maxn_sw = 0;
@@ -1679,8 +1710,8 @@ static void hky_bins(const Pools &P, const Batch &b, int variant, cudaStream_t s
   for (const HkyBin &q : b.bins) {
     const int o = b.nis + q.off;
     if (b.prec == IMA_PREC_FP64) launch_hky_fp64(P, b.d_req + o, q.n, q.maxn, b.d_res + o, b.d_st + o, st);
-    else if (b.prec == IMA_PREC_FP32) launch_hky_fp32(P, b.d_req + o, q.n, q.maxn, q.maxs, variant, b.d_res + o, b.d_st + o, st);
-    else launch_hky_fast(P, b.d_req + o, q.n, q.maxn, q.maxs, variant, b.d_res + o, b.d_st + o, st);
+    else if (b.prec == IMA_PREC_FP32) launch_hky_fp32(P, b.d_req + o, q.n, q.maxn, q.maxs, q.uni, variant, b.d_res + o, b.d_st + o, st);
+    else launch_hky_fast(P, b.d_req + o, q.n, q.maxn, q.maxs, q.uni, variant, b.d_res + o, b.d_st + o, st);
   }
 }
 
@@ -4454,7 +4485,7 @@ extern "C" int ima_gpu_updategenealogy_sweep(ima_ctx *c, int nch, const int32_t 
     }
     if (c->loci[l0].d.model == IMA_MODEL_SW) continue;  // its update runs in k_ug_sw
     Batch &b = c->ugb[s];
-    r = build_batch(c, b, nr, lci.data(), lli.data(), lu.data(), lk.data(), nullptr, nullptr, precision);
+    r = build_batch(c, b, nr, lci.data(), lli.data(), lu.data(), lk.data(), nullptr, nullptr, precision, true);
     r = r ? r : init_sumlogk(c, b);
     for (int k = 0; k < nr && !r; k++) reqof[(size_t)l0 * nch + b.order[k]] = k;
   }

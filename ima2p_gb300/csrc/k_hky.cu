@@ -29,6 +29,7 @@
 // log(max) accumulated into an FP64 scale factor.
 #include <algorithm>
 #include <cmath>
+#include <vector>
 
 #include "ff.cuh"
 #include "internal.h"
@@ -316,14 +317,14 @@ __device__ __forceinline__ void hky_apply_tip_ff(const float *K, float2 p, int s
 __device__ __forceinline__ ff ff_of(float2 v) { return ff_make(v.x, v.y); }
 
 // Shared-memory carve-up, identical on host (sizing) and device.
-// branch: bytes of one branch's coefficients; time: bytes of one node's time.
+// coef: bytes of the branches' coefficients; time: bytes of one node's time.
 struct HkyLayout {
   size_t nd, times, fresh, order, tip, off, total;
 };
-__host__ __device__ inline HkyLayout hky_layout(int maxnl, size_t branch, size_t time)
+__host__ __device__ inline HkyLayout hky_layout(int maxnl, size_t coef, size_t time)
 {
   HkyLayout l;
-  l.nd = branch * (size_t)maxnl;
+  l.nd = coef;
   l.times = l.nd + sizeof(NodeRec) * (size_t)maxnl;
   l.fresh = l.times + time * (size_t)maxnl;
   l.order = (l.fresh + 3 * (size_t)maxnl + 15) & ~size_t(15);
@@ -334,13 +335,17 @@ __host__ __device__ inline HkyLayout hky_layout(int maxnl, size_t branch, size_t
 }
 __host__ __device__ inline HkyLayout hky_layout64(int maxnl)  // k_hky_fp64: a 4 x 4 matrix per branch
 {
-  return hky_layout(maxnl, 16 * sizeof(double), 0);
+  return hky_layout(maxnl, 16 * sizeof(double) * (size_t)maxnl, 0);
 }
-// k_hky_fast: floats per branch (5 coefficients, as pairs in float-float)
+// k_hky_fast: floats per branch (5 coefficients, as pairs in float-float) and
+// per tip's branch (float-float with every pattern kept: the four columns of
+// P(b) as pairs)
 __host__ __device__ constexpr int hky_floats(bool ff) { return ff ? 12 : 8; }
-__host__ __device__ inline HkyLayout hky_layout_fast(int maxnl, bool ff)
+__host__ __device__ constexpr int hky_tip_floats(bool uni, bool ff) { return ff && !uni ? 32 : hky_floats(ff); }
+__host__ __device__ inline HkyLayout hky_layout_fast(int maxnl, bool uni, bool ff)
 {
-  return hky_layout(maxnl, 4 * hky_floats(ff), sizeof(float2));
+  const size_t maxn = (size_t)(maxnl + 1) / 2;
+  return hky_layout(maxnl, 4 * (maxn * hky_tip_floats(uni, ff) + (maxn - 1) * hky_floats(ff)), sizeof(float2));
 }
 
 // ----------------------------------------------------- uniform patterns
@@ -359,13 +364,11 @@ __host__ __device__ inline HkyLayout hky_layout_fast(int maxnl, bool ff)
 // daughter first.  A full evaluation's list depends on the topology alone: it
 // is kept per item and read back while P.is_valid says so.  The list of an
 // evaluation from edited edges is shorter; what of it does not fit in shared
-// memory goes to the same place, which ends the kept list.  Loci whose masks
-// pass HKY_MASK_WORDS, or whose patterns 16 bits, keep every pattern.
+// memory goes to the same place, which ends the kept list.
+// Loci whose masks pass HKY_MASK_WORDS, or whose patterns 16 bits, keep every
+// pattern and have no list (UNI false in the kernel), and so do those where
+// most tips differ (hky_uniform_entries).
 constexpr int HKY_MASK_WORDS = 8192;
-__host__ __device__ inline bool hky_uniform(int n, int S)
-{
-  return (long long)(n - 1) * ((S + 31) / 32) <= HKY_MASK_WORDS && S <= 65531 && n <= 32768;
-}
 __device__ __forceinline__ int2 hky_children(const NodeRec &nd, int n)  // the internal daughter first
 {
   return nd.up0 < n && nd.up1 >= n ? make_int2(nd.up1, nd.up0) : make_int2(nd.up0, nd.up1);
@@ -433,17 +436,16 @@ __device__ __forceinline__ int expo_of(float m)  // floor(log2(m)) for normal m 
 
 // ------------------------------------------------------------------ FP32
 // One CTA per chain-locus, internal nodes level by level.  Each branch gets
-// the five coefficients of hky_coef_fast (in place of a 4 x 4 matrix), and a
-// warp works on one node and 32 of its patterns at a time, so the children's
-// coefficients are warp-uniform and no warp mixes tip and internal children.
-// With CACHE, the partials this launch computes are also kept in shared
-// memory ([internal node][pattern]) and daughters are read from there instead
-// of making an L2 round trip per level.  BS threads per CTA, registers for
-// MINB resident CTAs per SM.  FF: every value a float-float pair (the lo
-// parts of the partials in P.partlo); otherwise FP32 (which clears the lo
-// parts of what it writes when they exist, so a later FF evaluation reads
-// its partials as exact pairs).
-template <bool FF, int BS, int MINB>
+// the five coefficients of hky_coef_fast (in place of a 4 x 4 matrix).  UNI: a
+// node's partials are those of its mixed patterns and of the four states, and
+// a thread takes a task of the list at a time.  Otherwise a node keeps every
+// pattern and a warp takes one node and 32 of its patterns at a time, so that
+// the children's coefficients are warp-uniform and no warp mixes tip and
+// internal children.  BS threads per CTA, registers for MINB resident CTAs per
+// SM.  FF: every value a float-float pair (the lo parts of the partials in
+// P.partlo); otherwise FP32 (which clears the lo parts of what it writes when
+// they exist, so a later FF evaluation reads its partials as exact pairs).
+template <bool UNI, bool FF, int BS, int MINB>
 __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *reqs,
                                                      double *result, int32_t *status, int maxnl,
                                                      int mcap, int pcap, int tcap)
@@ -453,9 +455,10 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
   // below wait on this one load only
   const ReqDev R = reqs[blockIdx.x];
   const int n = R.n, nl = 2 * n - 1, S = R.nsites, nint = n - 1;
-  constexpr int PB = hky_floats(FF);
-  const HkyLayout lay = hky_layout_fast(maxnl, FF);
-  float *Pm = reinterpret_cast<float *>(smem);                 // [branch][PB]
+  constexpr int PB = hky_floats(FF), PT = hky_tip_floats(UNI, FF);
+  const HkyLayout lay = hky_layout_fast(maxnl, UNI, FF);
+  float *Pt = reinterpret_cast<float *>(smem);  // [n][PT], a tip's branch
+  float *Pm = Pt + (PT - PB) * n;               // [2n - 1][PB], from n on: the other branches
   float2 *stm = reinterpret_cast<float2 *>(smem + lay.times);        // node times
   Tree T;
   T.nd = reinterpret_cast<NodeRec *>(smem + lay.nd);
@@ -492,17 +495,16 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
   for (int k = tid; k < 2 * n; k += BS) T.order[k] = P.sched[R.sched_off + k];
   const int nlev = P.nlev[R.item];
   T.lstart = T.order + nint;
-  const bool uni = hky_uniform(n, S);
   const int W = (S + 31) >> 5, S4 = S + 4;  // S4: partials stored per node
   const int lw = W > 1 ? 32 - __clz(W - 1) : 0;  // words per node rounded up to 2^lw
   const uint32_t *plane = P.planes + R.plane_off;
   uint2 *task = P.task + R.part_off / 2;
   int32_t *gtoff = P.toff + R.sched_off;
-  const bool listed = uni && full && P.is_valid[R.item];
+  const bool listed = UNI && full && P.is_valid[R.item];
   // the list's offsets are loaded beside the flag that says whether they hold
-  if (uni && full)
+  if (UNI && full)
     for (int k = tid; k < n; k += BS) toff[k] = gtoff[k];
-  if (uni && !listed && n * 2 * W <= pcap) {
+  if (UNI && !listed && n * 2 * W <= pcap) {
     for (int k = tid; k < n * 2 * W; k += BS) splane[k] = plane[k];
     plane = splane;
   }
@@ -552,7 +554,7 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
   if (!full) __syncthreads();
   // the masks and the nodes' task counts by the first warp, the branches'
   // coefficients by the others
-  const bool build = uni && !listed;
+  const bool build = UNI && !listed;
   if (listed) {  // the copies land during the coefficients
     const int tbase = max(0, toff[nint] - tcap);
     for (int k = tbase + tid; k < toff[nint]; k += BS)
@@ -609,10 +611,20 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
       const ff br = (u < 0) ? tc : ff_sub(tc, ff_of(stm[u]));
       float Kc[10];
       hky_coef_ff(sH, stab, ff_mul(ff_of(smu), br), Kc);
-      float4 *dst = reinterpret_cast<float4 *>(Pm + PB * c);
+      float4 *dst = reinterpret_cast<float4 *>(UNI || c >= n ? Pm + PB * c : Pt + PT * c);
       dst[0] = make_float4(Kc[0], Kc[0], Kc[2], Kc[4]);
       dst[1] = make_float4(Kc[6], Kc[8], Kc[1], Kc[1]);
       dst[2] = make_float4(Kc[3], Kc[5], Kc[7], Kc[9]);
+      if (!UNI && c < n) {  // the four columns, over the coefficients they come from
+        ff2 col[4][2];
+#pragma unroll
+        for (int st = 0; st < 4; st++) hky_apply_tip_ff(Pt + PT * c, spi[st], st, col[st]);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const float2 h = f2_un(col[k >> 1][k & 1].hi), l = f2_un(col[k >> 1][k & 1].lo);
+          dst[k] = make_float4(h.x, h.y, l.x, l.y);
+        }
+      }
     } else {
       float pil[4] = {spi[0].x, spi[1].x, spi[2].x, spi[3].x};
       hky_coef_fast(pil, skpa.x, smu.x * branch_ff(T.nd, stm, c), Pm + PB * c);
@@ -620,7 +632,7 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  const int tbase = uni ? max(0, toff[nint] - tcap) : 0;
+  const int tbase = UNI ? max(0, toff[nint] - tcap) : 0;
   if (build) {
     // a thread takes eight patterns of a node
     for (int q = tid; q < nint << (lw + 2); q += BS) {
@@ -678,26 +690,38 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
   const float pi4[4] = {spi[0].x, spi[1].x, spi[2].x, spi[3].x};
   const ff2 pi2[2] = {ff2_make(f2_pack(spi[0].x, spi[1].x), f2_pack(spi[0].y, spi[1].y)),
                       ff2_make(f2_pack(spi[2].x, spi[3].x), f2_pack(spi[2].y, spi[3].y))};
-  // a level's tasks are independent; the threads take them in turn
+  // A level's tasks are independent; the threads take them in turn.  Without a
+  // list the warps take (node, 32 patterns) in turn: warp w starts at node j0 of
+  // the level and chunk c0 and advances by NW chunks (no division in the loop).
+  constexpr int NW = BS / 32;
+  const int jstep = UNI ? 0 : NW / W, cstep = UNI ? 0 : NW - jstep * W, j0 = UNI ? 0 : (tid >> 5) / W,
+            c0 = UNI ? 0 : (tid >> 5) - j0 * W;
   for (int lv = 0; lv < nlev; lv++) {
-    const int beg = uni ? toff[T.lstart[lv]] : 0,
-              end = uni ? toff[T.lstart[lv + 1]] : (T.lstart[lv + 1] - T.lstart[lv]) * S;
-    for (int q = beg + tid; q < end; q += BS) {
+    const int beg = UNI ? toff[T.lstart[lv]] + tid : tid >> 5,
+              end = UNI ? toff[T.lstart[lv + 1]] : (T.lstart[lv + 1] - T.lstart[lv]) * W;
+    int jj = j0, chunk = c0;
+    for (int q = beg; q < end; q += UNI ? BS : NW) {
       int node, i, ic[2];  // the daughters' entries
-      if (uni) {
+      if (UNI) {
         const uint2 t = q >= tbase ? stask[q - tbase] : task[q];
         node = n + (int)(t.x & 0xffffu);
         i = (int)(t.x >> 16);
         ic[0] = (int)(t.y & 0xffffu);
         ic[1] = (int)(t.y >> 16);
       } else {
-        node = T.order[T.lstart[lv] + q / S];
-        i = q % S;
-        if (!T.fresh[node]) continue;
+        node = T.order[T.lstart[lv] + jj];
+        i = chunk * 32 + (tid & 31);
+        jj += jstep;
+        chunk += cstep;
+        if (chunk >= W) {
+          chunk -= W;
+          jj++;
+        }
+        if (!T.fresh[node] || i >= S) continue;
       }
       const int2 ch = hky_children(T.nd[node], n);
       const int cc[2] = {ch.x, ch.y};
-      if (!uni)
+      if (!UNI)
         for (int h = 0; h < 2; h++) ic[h] = cc[h] < n ? seq[(size_t)cc[h] * S + i] : i;
       int e = 0;
       float4 ov, ol = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -706,7 +730,12 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           const int c = cc[h];
-          if (c < n) {
+          if (!UNI && c < n) {
+            const float4 *col = reinterpret_cast<const float4 *>(Pt + PT * c) + 2 * ic[h];
+            const float4 a = col[0], b = col[1];
+            v[h][0] = ff2_make(f2_pack(a.x, a.y), f2_pack(a.z, a.w));
+            v[h][1] = ff2_make(f2_pack(b.x, b.y), f2_pack(b.z, b.w));
+          } else if (c < n) {
             hky_apply_tip_ff(Pm + PB * c, spi[ic[h]], ic[h], v[h]);
           } else {
             const int rs = T.fresh[c] ? 1 - T.slot[c] : T.slot[c];
@@ -967,46 +996,76 @@ __global__ void k_hky_commit(Pools P, const int32_t *items, const uint8_t *accep
 
 constexpr size_t HKY_TASK_CAP = 640, HKY_PLANE_CAP = 1024;  // tasks and words kept in shared memory
 
-template <bool FF, int BS, int MINB>
-static void hky_fast_bs(const Pools &P, const ReqDev *reqs, int nreq, int maxnl, int maxS, double *result,
-                        int32_t *status, cudaStream_t st)
+template <bool UNI, bool FF, int BS, int MINB>
+static void hky_fast_launch(const Pools &P, const ReqDev *reqs, int nreq, int maxnl, int maxS, double *result,
+                            int32_t *status, cudaStream_t st)
 {
   const size_t maxn = (size_t)(maxnl + 1) / 2, W = ((size_t)maxS + 31) / 32;
-  const size_t mcap = std::min((size_t)HKY_MASK_WORDS, (maxn - 1) * W);
-  const size_t pcap = std::min(HKY_PLANE_CAP, 2 * maxn * W), tcap = std::min(HKY_TASK_CAP, (maxn - 1) * (maxS + 4));
-  const size_t sm = hky_layout_fast(maxnl, FF).total + 4 * (mcap + pcap) + 2 * ((mcap + 1) & ~size_t(1)) + tcap * sizeof(uint2);
+  const size_t mcap = UNI ? std::min((size_t)HKY_MASK_WORDS, (maxn - 1) * W) : 0;
+  const size_t pcap = UNI ? std::min(HKY_PLANE_CAP, 2 * maxn * W) : 0;
+  const size_t tcap = UNI ? std::min(HKY_TASK_CAP, (maxn - 1) * (maxS + 4)) : 0;
+  const size_t sm = hky_layout_fast(maxnl, UNI, FF).total + 4 * (mcap + pcap) + 2 * ((mcap + 1) & ~size_t(1)) + tcap * sizeof(uint2);
   if (sm > 40 * 1024)  // (48 KB with the static part)
-    cudaFuncSetAttribute(k_hky_fast<FF, BS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_hky_fast<FF, BS, MINB><<<nreq, BS, sm, st>>>(P, reqs, result, status, maxnl, (int)mcap, (int)pcap, (int)tcap);
+    cudaFuncSetAttribute(k_hky_fast<UNI, FF, BS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_hky_fast<UNI, FF, BS, MINB><<<nreq, BS, sm, st>>>(P, reqs, result, status, maxnl, (int)mcap, (int)pcap, (int)tcap);
 }
 
-void launch_hky_fast(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, int variant,
+template <bool FF, int BS, int MINB>
+static void hky_fast_bs(const Pools &P, const ReqDev *reqs, int nreq, int maxnl, int maxS, bool uni, double *result,
+                        int32_t *status, cudaStream_t st)
+{
+  if (uni) hky_fast_launch<true, FF, BS, MINB>(P, reqs, nreq, maxnl, maxS, result, status, st);
+  else hky_fast_launch<false, FF, BS, MINB>(P, reqs, nreq, maxnl, maxS, result, status, st);
+}
+
+// One entry per state pays where the tips below a node often agree.  Where
+// few pairs of tips do, the list's loads and the mixed daughters of a warp
+// cost more than the entries save: with 44% of the pairs alike 1,280
+// chain-loci of 100 genes x 300 patterns take 389 us either way and 12,800 of
+// 96 x 80 836 and 806, with 25% (unrelated sequences) 433 and 374, 927 and 804;
+// with 57% 345 and 374, 757 and 804.  That is of states drawn tip by tip; along a
+// genealogy equal states lie together, and simulated sequences have 64-94%.
+constexpr double HKY_AGREE = 0.4;
+
+bool hky_uniform_entries(int n, int S, const int8_t *seq)
+{
+  if ((long long)(n - 1) * ((S + 31) / 32) > HKY_MASK_WORDS || S > 65531 || n > 32768) return false;
+  // pairs of tips with the same state, over the patterns
+  std::vector<int> f(4 * (size_t)S, 0);
+  for (int t = 0; t < n; t++)
+    for (int k = 0; k < S; k++) f[4 * (size_t)k + seq[(size_t)t * S + k]]++;
+  double same = 0.0;
+  for (int v : f) same += (double)v * (v - 1);
+  return same >= HKY_AGREE * S * (double)n * (n - 1);
+}
+
+void launch_hky_fast(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, bool uni, int variant,
                      double *result, int32_t *status, cudaStream_t st)
 {
   if (nreq <= 0) return;
   const int maxnl = 2 * maxn - 1;
   switch (variant) {
-    case 1: hky_fast_bs<true, 64, 16>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
-    case 2: hky_fast_bs<true, 256, 4>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
-    case 3: hky_fast_bs<true, 128, 10>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
-    case 4: hky_fast_bs<true, 128, 8>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
-    case 5: hky_fast_bs<true, 96, 11>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
-    default: hky_fast_bs<true, 128, 6>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
+    case 1: hky_fast_bs<true, 64, 16>(P, reqs, nreq, maxnl, maxS, uni, result, status, st); break;
+    case 2: hky_fast_bs<true, 256, 4>(P, reqs, nreq, maxnl, maxS, uni, result, status, st); break;
+    case 3: hky_fast_bs<true, 128, 10>(P, reqs, nreq, maxnl, maxS, uni, result, status, st); break;
+    case 4: hky_fast_bs<true, 128, 8>(P, reqs, nreq, maxnl, maxS, uni, result, status, st); break;
+    case 5: hky_fast_bs<true, 96, 11>(P, reqs, nreq, maxnl, maxS, uni, result, status, st); break;
+    default: hky_fast_bs<true, 128, 6>(P, reqs, nreq, maxnl, maxS, uni, result, status, st); break;
   }
 }
 
-void launch_hky_fp32(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, int variant,
+void launch_hky_fp32(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, bool uni, int variant,
                      double *result, int32_t *status, cudaStream_t st)
 {
   if (nreq <= 0) return;
   const int maxnl = 2 * maxn - 1;
   switch (variant) {
-    case 1: hky_fast_bs<false, 64, 24>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
-    case 2: hky_fast_bs<false, 256, 6>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
-    case 3: hky_fast_bs<false, 128, 6>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
-    case 4: hky_fast_bs<false, 128, 8>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
-    case 5: hky_fast_bs<false, 96, 16>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
-    default: hky_fast_bs<false, 128, 12>(P, reqs, nreq, maxnl, maxS, result, status, st); break;
+    case 1: hky_fast_bs<false, 64, 24>(P, reqs, nreq, maxnl, maxS, uni, result, status, st); break;
+    case 2: hky_fast_bs<false, 256, 6>(P, reqs, nreq, maxnl, maxS, uni, result, status, st); break;
+    case 3: hky_fast_bs<false, 128, 6>(P, reqs, nreq, maxnl, maxS, uni, result, status, st); break;
+    case 4: hky_fast_bs<false, 128, 8>(P, reqs, nreq, maxnl, maxS, uni, result, status, st); break;
+    case 5: hky_fast_bs<false, 96, 16>(P, reqs, nreq, maxnl, maxS, uni, result, status, st); break;
+    default: hky_fast_bs<false, 128, 12>(P, reqs, nreq, maxnl, maxS, uni, result, status, st); break;
   }
 }
 

@@ -317,25 +317,27 @@ __device__ __forceinline__ void hky_apply_tip_ff(const float *K, float2 p, int s
 __device__ __forceinline__ ff ff_of(float2 v) { return ff_make(v.x, v.y); }
 
 // Shared-memory carve-up, identical on host (sizing) and device.
-// coef: bytes of the branches' coefficients; time: bytes of one node's time.
+// coef: bytes of the branches' coefficients; fast: with the node times, the
+// tips and the list's offsets of k_hky_fast.
 struct HkyLayout {
   size_t nd, times, fresh, order, tip, off, total;
 };
-__host__ __device__ inline HkyLayout hky_layout(int maxnl, size_t coef, size_t time)
+__host__ __device__ inline HkyLayout hky_layout(int maxnl, size_t coef, bool fast)
 {
+  const size_t nl = (size_t)maxnl;
   HkyLayout l;
   l.nd = coef;
-  l.times = l.nd + sizeof(NodeRec) * (size_t)maxnl;
-  l.fresh = l.times + time * (size_t)maxnl;
-  l.order = (l.fresh + 3 * (size_t)maxnl + 15) & ~size_t(15);
-  l.tip = l.order + sizeof(int16_t) * (size_t)(maxnl + 3);
-  l.off = (l.tip + sizeof(int16_t) * (size_t)maxnl + 3) & ~size_t(3);
-  l.total = (l.off + sizeof(int32_t) * (size_t)(maxnl / 2 + 2) + 15) & ~size_t(15);
+  l.times = l.nd + sizeof(NodeRec) * nl;
+  l.fresh = l.times + (fast ? sizeof(float2) * nl : 0);
+  l.order = (l.fresh + 3 * nl + 15) & ~size_t(15);
+  l.tip = l.order + sizeof(int16_t) * (nl + 3);
+  l.off = fast ? (l.tip + sizeof(int16_t) * nl + 3) & ~size_t(3) : l.tip;
+  l.total = (l.off + (fast ? sizeof(int32_t) * (nl / 2 + 2) : 0) + 15) & ~size_t(15);
   return l;
 }
 __host__ __device__ inline HkyLayout hky_layout64(int maxnl)  // k_hky_fp64: a 4 x 4 matrix per branch
 {
-  return hky_layout(maxnl, 16 * sizeof(double) * (size_t)maxnl, 0);
+  return hky_layout(maxnl, 16 * sizeof(double) * (size_t)maxnl, false);
 }
 // k_hky_fast: floats per branch (5 coefficients, as pairs in float-float) and
 // per tip's branch (float-float with every pattern kept: the four columns of
@@ -345,7 +347,7 @@ __host__ __device__ constexpr int hky_tip_floats(bool uni, bool ff) { return ff 
 __host__ __device__ inline HkyLayout hky_layout_fast(int maxnl, bool uni, bool ff)
 {
   const size_t maxn = (size_t)(maxnl + 1) / 2;
-  return hky_layout(maxnl, 4 * (maxn * hky_tip_floats(uni, ff) + (maxn - 1) * hky_floats(ff)), sizeof(float2));
+  return hky_layout(maxnl, 4 * (maxn * hky_tip_floats(uni, ff) + (maxn - 1) * hky_floats(ff)), true);
 }
 
 // ----------------------------------------------------- uniform patterns

@@ -45,7 +45,7 @@ __device__ void rng_load(LocalRng &r, const ima_ug_rng *g, uint32_t *smt, int ti
   uint2 *dst = reinterpret_cast<uint2 *>(smt);
   for (int k = tid; k < RNG_N / 2; k += nt) dst[k] = src[k];
   r.mt = smt;
-  r.mti = g->mt.mti;
+  r.mti = (int)min((unsigned)g->mt.mti, (unsigned)RNG_N);  // a count outside the state: all words are drawn
   r.iset = g->iset;
   r.gset = g->gset;
   r.iseed = g->iseed;

@@ -301,6 +301,12 @@ struct ima_ctx {
   const void *twin_dev = nullptr;
   std::vector<int32_t> twin_perm;
   std::vector<long long> twin_evoff;
+  // sources of copies that a split-time update queues and does not wait for
+  // before it returns to them: the band's parameters, the chains' groups.  (An
+  // asynchronous copy from pageable memory may read it when the stream gets
+  // there.)  Every call that queues such copies waits before it returns.
+  std::vector<double> band_prm;
+  std::vector<int32_t> tp_off, tp_end;
   void *d_twin = nullptr, *d_twout = nullptr, *d_tpbuf = nullptr;
   size_t twin_cap = 0, twout_cap = 0, tpbuf_cap = 0;
   int tw_ngen = 0, tw_ntv = 0;
@@ -3895,6 +3901,13 @@ static void* rsel(ima_ctx *c, size_t bytes)
   return c->d_rsel;
 }
 
+// a failed call's queued copies may still read its host buffers
+static int settled(ima_ctx *c, int r)
+{
+  if (r) cudaStreamSynchronize(c->st);
+  return r;
+}
+
 static void dev_newer(ima_ctx *c, int nch, const int32_t *chains)
 {
   for (int k = 0; k < nch; k++) {
@@ -3904,14 +3917,16 @@ static void dev_newer(ima_ctx *c, int nch, const int32_t *chains)
 }
 
 // the band on the device; counts stay in d_bcnt, the chain list in
-// *d_chains (the caller's chains, device copy) when asked for
+// *d_chains (the caller's chains, device copy) when asked for.  Without sync the
+// caller waits for the stream before it calls again or gives up chains.
 static int band_run(ima_ctx *c, int nch, const int32_t *chains, const int32_t *period, const double *oldt,
                     const double *newt, const double *t_u, const double *t_d, int inverse, int32_t *counts,
                     bool sync, int32_t **d_chains = nullptr)
 {
   int r = IMA_OK;
   const int last = c->h_tw.npops - 1;
-  std::vector<double> prm(5 * (size_t)nch);
+  std::vector<double> &prm = c->band_prm;
+  prm.resize(5 * (size_t)nch);
   for (int k = 0; k < nch; k++) {
     if (period[k] < 0 || period[k] >= last) return c->fail(IMA_ERR_ARG, "period %d out of range", period[k]);
     if (!(oldt[k] > t_u[k]) || !(newt[k] > t_u[k]) || !(oldt[k] < t_d[k]) || !(newt[k] < t_d[k]))
@@ -3957,7 +3972,6 @@ static int band_run(ima_ctx *c, int nch, const int32_t *chains, const int32_t *p
   c->launches += nk - 1;
   r = c->cuda(cudaGetLastError(), "band launch");
   if (!r && counts && !inverse) r = c->cuda(cudaMemcpyAsync(counts, c->d_bcnt, 16ul * nch, cudaMemcpyDeviceToHost, c->st), "band counts");
-  // (the parameter block is pageable host memory: its copy has been staged)
   if (sync) r = r ? r : c->cuda(cudaStreamSynchronize(c->st), "band");
   if (!r) dev_newer(c, nch, chains);
   if (d_chains) *d_chains = d_ch;
@@ -3972,7 +3986,7 @@ extern "C" int ima_gpu_rubber_band(ima_ctx *c, int nch, const int32_t *chains, c
   if (!c->tw_ready) return c->fail(IMA_ERR_STATE, "call ima_gpu_set_popmodel first");
   int r = chains_ready(c, nch, chains);
   if (r) return r;
-  return band_run(c, nch, chains, period, oldt, newt, t_u, t_d, inverse, counts, true);
+  return settled(c, band_run(c, nch, chains, period, oldt, newt, t_u, t_d, inverse, counts, true));
 }
 
 static int chain_weights_run(ima_ctx *c, int nch, const int32_t *chains, const double *tvals, double *probg,
@@ -4052,12 +4066,12 @@ static int chain_weights_run(ima_ctx *c, int nch, const int32_t *chains, const d
   // this size from pageable memory waits for the work before it)
   if (c->twin_dev != c->d_twin || c->twin_perm != perm || c->twin_evoff != evoff) {
     c->twin_dev = nullptr;
-    r = c->cuda(cudaMemcpyAsync(d_perm, perm.data(), ns * 4, cudaMemcpyHostToDevice, c->st), "weights");
-    r = r ? r : c->cuda(cudaMemcpyAsync(d_evoff, evoff.data(), (ni + 1) * 8ul, cudaMemcpyHostToDevice, c->st), "weights");
-    if (r) return r;
-    c->twin_dev = c->d_twin;
     c->twin_perm = std::move(perm);
     c->twin_evoff = std::move(evoff);
+    r = c->cuda(cudaMemcpyAsync(d_perm, c->twin_perm.data(), ns * 4, cudaMemcpyHostToDevice, c->st), "weights");
+    r = r ? r : c->cuda(cudaMemcpyAsync(d_evoff, c->twin_evoff.data(), (ni + 1) * 8ul, cudaMemcpyHostToDevice, c->st), "weights");
+    if (r) return r;
+    c->twin_dev = c->d_twin;
   }
   r = c->cuda(cudaMemcpyAsync(c->d_tvr, c->h_tvr.data(), c->h_tvr.size() * 8, cudaMemcpyHostToDevice, c->st), "weights");
   r = r ? r : c->cuda(cudaMemsetAsync(c->d_twerr, 0, 8, c->st), "weights");
@@ -4081,7 +4095,9 @@ static int chain_weights_run(ima_ctx *c, int nch, const int32_t *chains, const d
   c->tw_fc = a.fc;
   c->tw_fm = a.fm;
   c->tw_tvals = c->d_tvr;
-  std::vector<int32_t> goff(nch), gend(nch);
+  std::vector<int32_t> &goff = c->tp_off, &gend = c->tp_end;
+  goff.resize(nch);
+  gend.resize(nch);
   for (int k = 0; k < nch; k++) {
     goff[k] = chains[k] * nl;
     gend[k] = chains[k] * nl + nl;
@@ -4098,7 +4114,7 @@ extern "C" int ima_gpu_chain_weights(ima_ctx *c, int nch, const int32_t *chains,
   if (!c->tw_ready) return c->fail(IMA_ERR_STATE, "call ima_gpu_set_popmodel first");
   int r = chains_ready(c, nch, chains);
   if (r) return r;
-  return chain_weights_run(c, nch, chains, tvals, probg, q, m, nullptr);
+  return settled(c, chain_weights_run(c, nch, chains, tvals, probg, q, m, nullptr));
 }
 
 extern "C" int ima_gpu_changet_ry1_sweep(ima_ctx *c, int nch, const int32_t *chains, const int32_t *period,
@@ -4120,7 +4136,7 @@ extern "C" int ima_gpu_changet_ry1_sweep(ima_ctx *c, int nch, const int32_t *cha
   // weights and p(G) run on while the host stages the likelihood requests;
   // their error word is read once the likelihoods have synchronised
   r = r ? r : chain_weights_run(c, nch, chains, tvals, nullptr, nullptr, nullptr, &d_pgnew, true);
-  if (r) return r;
+  if (r) return settled(c, r);
   // the chains' likelihoods (writes the per-item pdg_new pool)
   std::vector<int32_t> ci((size_t)nch * nl), li((size_t)nch * nl), st((size_t)nch * nl);
   std::vector<double> kap((size_t)nch * nl, 1.0), res((size_t)nch * nl);
@@ -4132,13 +4148,13 @@ extern "C" int ima_gpu_changet_ry1_sweep(ima_ctx *c, int nch, const int32_t *cha
     }
   r = ima_gpu_eval(c, nch * nl, ci.data(), li.data(), u, kap.data(), nullptr, nullptr, precision, res.data(), st.data());
   r = r ? r : tw_check_err(c, "chain weights / p(G)");
-  if (r) return r;
+  if (r) return settled(c, r);
   for (size_t k = 0; k < st.size(); k++)
     if (st[k] == IMA_EVAL_IS_FAIL)
       return c->fail(IMA_ERR_DATA, "chain %d locus %d: data incompatible with the genealogy", ci[k], li[k]);
   // the decisions, on the device
   char *buf = static_cast<char *>(rsel(c, carve_size({nch * 4ul, 40ul * nch, 24ul * nch, 8ul * nch, nch * 1ul, 8ul * nch})));
-  if (!buf) return c->fail(IMA_ERR_NOMEM, "decision buffers");
+  if (!buf) return settled(c, c->fail(IMA_ERR_NOMEM, "decision buffers"));
   Carve cv{buf};
   int32_t *d_ch2 = cv.take<int32_t>(nch);
   cv.take<double>(5 * (size_t)nch);  // the band's parameter block (same buffer)
@@ -4154,7 +4170,7 @@ extern "C" int ima_gpu_changet_ry1_sweep(ima_ctx *c, int nch, const int32_t *cha
   }
   r = c->cuda(cudaMemcpyAsync(d_ch2, chains, nch * 4ul, cudaMemcpyHostToDevice, c->st), "decide");
   r = r ? r : c->cuda(cudaMemcpyAsync(d_logs, logs.data(), logs.size() * 8, cudaMemcpyHostToDevice, c->st), "decide");
-  if (r) return r;
+  if (r) return settled(c, r);
   RyArgs a{};
   a.nch = nch;
   a.nloci = nl;
@@ -4177,7 +4193,7 @@ extern "C" int ima_gpu_changet_ry1_sweep(ima_ctx *c, int nch, const int32_t *cha
   r = r ? r : c->cuda(cudaMemcpyAsync(accept, d_acc, nch, cudaMemcpyDeviceToHost, c->st), "decisions");
   if (pdgsum) r = r ? r : c->cuda(cudaMemcpyAsync(pdgsum, d_sum, nch * 8ul, cudaMemcpyDeviceToHost, c->st), "decisions");
   r = r ? r : c->cuda(cudaStreamSynchronize(c->st), "decisions");
-  if (r) return r;
+  if (r) return settled(c, r);
   // commit the accepted chains' evaluations, move the others back
   std::vector<uint8_t> acc_items((size_t)nch * nl);
   std::vector<int32_t> rc, rp;
@@ -4201,7 +4217,7 @@ extern "C" int ima_gpu_changet_ry1_sweep(ima_ctx *c, int nch, const int32_t *cha
     r = c->cuda(cudaMemcpyAsync(all.data(), c->d_probg, c->nchains * 8ul, cudaMemcpyDeviceToHost, c->st), "probg");
   r = r ? r : c->cuda(cudaStreamSynchronize(c->st), "split-time update");
   for (int k = 0; !r && probg && k < nch; k++) probg[k] = all[chains[k]];
-  return r;
+  return settled(c, r);
 }
 
 // changet_RY1's draws in the library: for each chain in order, getnewt

@@ -102,10 +102,13 @@ __global__ void __launch_bounds__(256) k_prep_tiles(SurfPrep S)
       f[j] = k < S.K ? v : 0.f;
       const __half x = __float2half_rn(v * exp2i(-e));
       const float d = v - __half2float(x) * exp2i(e);
+      // no weight, or no bound: infinite, so that every other term passes the
+      // screen (a value that is not a number leaves none, its own or a point's)
+      const float r = isinf(k == S.K + 1 ? bias.x : v) ? INFINITY : d;
       if (k == S.K) left = d;
       if (j & 1) h[j >> 1] = __halves2half2(__low2half(h[j >> 1]), x);
       else h[j >> 1] = __halves2half2(x, x);
-      const unsigned m = k == S.K ? 0u : __reduce_max_sync(0xffffffffu, g < S.G ? __float_as_uint(fabsf(d)) : 0u);
+      const unsigned m = k == S.K ? 0u : __reduce_max_sync(0xffffffffu, g < S.G ? __float_as_uint(fabsf(r)) : 0u);
       if ((threadIdx.x & 31) == k) top = m;
     }
     if (q == SURF_KP / 8 - 1) {

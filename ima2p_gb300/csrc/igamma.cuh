@@ -1,12 +1,16 @@
 // igamma.cuh -- the reference's incomplete gamma functions on the device
 // (uppergamma, lowergamma, gser/gserlog, gcf/gcflog, expint(1, x) and
 // LogDiff; utilities.cpp:808-1130, imamp.hpp:257-262), shared by the p(G)
-// integrals (k_treeweight.cu) and the 2NM densities (k_popmig.cu).  Both
-// files are compiled with -fmad=false so that these add and multiply in the
-// reference's order; log and exp are the device's.
+// integrals (k_treeweight.cu, k_updgen.cu) and the 2NM densities
+// (k_popmig.cu).  All FP64; log and exp are the device's.  The series takes
+// one division for four terms and gcf's fraction runs on numerators and
+// denominators, so their roundings are not the reference's one by one: both
+// stop at its term, and the sums are within 5e-15 of the same sums in quad
+// precision, as its own are (60,000 random (a, x) in each of ten ranges of a up
+// to 12,000; the logarithms' errors are equal in mean and maximum).  The other
+// expressions keep its order of operations (-fmad=false).
 #pragma once
 
-#include "ff.cuh"
 #include "internal.h"
 
 namespace {
@@ -14,114 +18,23 @@ namespace {
 enum { IG_E_TERM = 4, IG_E_LF = 5 };  // a series or fraction that did not converge; a count past logfact
 
 // The reference's incomplete gamma functions, restated from the published
-// Numerical Recipes methods it uses (series, Lentz continued fraction, E1
-// series / continued fraction) with its constants: EPS 3e-7, ITMAX 1000,
+// Numerical Recipes methods it uses (series, continued fraction, E1 series /
+// continued fraction by Lentz's method) with its constants: EPS 3e-7, ITMAX 1000,
 // FPMIN 1e-30, expint's MAXIT 100 and Euler constant 0.5772156649.
 constexpr double IG_EPS = 3.0e-7, IG_FPMIN = 1.0e-30, EI_EULER = 0.5772156649;
 constexpr int IG_ITMAX = 1000, EI_MAXIT = 100;
 constexpr double LD_CUT = 7.0978271289338397e+02, MPRIORMIN = 0.000001;
 constexpr double LOG2 = 0.69314718055994530941723212146;
 
-// From IGF_AMIN on the series and the fraction run on the FP32 pipe in
-// float-float (2^-46; FP64's exponent a ln x - x - gln, by which they are
-// multiplied or to whose logarithm they are added, is off by more from a = 32
-// on): its operations take a tenth of the time, and there are 64 of them for
-// one of FP64.  One pass each, the sum or the convergents growing until the
-// reference's rule stops them, which FP32 decides unless the ratio lies
-// within IGF_TOL of EPS; that bounds what IGF_NMAX steps of a few roundings
-// each can be off.  A stop that cannot be told is left to the FP64 loops.
-constexpr int IGF_AMIN = 32, IGF_NMAX = 512;
-constexpr float IGF_EPS = 3.0e-7f, IGF_TOL = 2e-4f, IGF_XMAX = 1e6f;
-
-__device__ __forceinline__ ff igf_rcp(float a)  // 1 / a, 1 <= a < 2^24
-{
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
-  r = __fmaf_rn(r, __fmaf_rn(-a, r, 1.f), r);
-  return ff_make(r, __fmul_rn(__fmaf_rn(-a, r, 1.f), r));
-}
-
-// the sum of gser's series over its first term 1 / a: false where the number
-// of terms cannot be told
-__device__ __forceinline__ bool igf_series(float a, double x, double *s)
-{
-  const ff xf = ff_split(x);
-  if (!(xf.hi < IGF_XMAX)) return false;
-  float ap = a, sum = 1.f, rest = 0.f;
-  ff del = ff_from(1.f);
-  for (int n = 0; n < IGF_NMAX; n++) {
-    ap = __fadd_rn(ap, 1.f);
-    const ff r = igf_rcp(ap);
-    const float q = __fmul_rn(xf.hi, r.hi);
-    const float qe = __fmaf_rn(xf.hi, r.lo, __fmaf_rn(xf.lo, r.hi, __fmaf_rn(xf.hi, r.hi, -q)));
-    const float p = __fmul_rn(del.hi, q);
-    del.lo = __fmaf_rn(del.hi, qe, __fmaf_rn(del.lo, q, __fmaf_rn(del.hi, q, -p)));
-    del.hi = p;
-    const ff t = two_sum(sum, p);
-    sum = t.hi;
-    rest = __fadd_rn(rest, __fadd_rn(t.lo, del.lo));
-    const float stop = __fmul_rn(sum, IGF_EPS);
-    if (p < stop * (1.f + IGF_TOL)) {
-      *s = (double)sum + (double)rest;
-      return p < stop * (1.f - IGF_TOL);
-    }
-  }
-  return false;
-}
-
-// gcf's fraction, A / B of the convergents A_n = b_n A_(n-1) + a_n A_(n-2) (B
-// alike) in units that keep B near 1; b0 = x + 1 - a.  Convergents n and n - 1
-// differ by D / (B B'), D the product of the -a_i.
-__device__ __forceinline__ bool igf_fraction(float a, double b0, double *h)
-{
-  const ff bf = ff_split(b0);
-  if (!(bf.hi < IGF_XMAX) || !(bf.hi >= 1.f)) return false;
-  ff A = ff_from(1.f), Ap = ff_from(0.f), B = bf, Bp = ff_from(1.f);
-  float D = 1.f;
-  for (int n = 1; n <= IGF_NMAX; n++) {
-    const float fn = (float)n;
-    ff b = two_sum(bf.hi, __fadd_rn(fn, fn));
-    b.lo = __fadd_rn(b.lo, bf.lo);
-    const ff an = two_prod(fn, __fsub_rn(a, fn));
-    auto next = [&](ff c, ff cp) {
-      const float u = __fmul_rn(b.hi, c.hi), v = __fmul_rn(an.hi, cp.hi);
-      const float ue = __fmaf_rn(b.hi, c.lo, __fmaf_rn(b.lo, c.hi, __fmaf_rn(b.hi, c.hi, -u)));
-      const float ve = __fmaf_rn(an.hi, cp.lo, __fmaf_rn(an.lo, cp.hi, __fmaf_rn(an.hi, cp.hi, -v)));
-      const ff t = two_sum(u, v);
-      return ff_make(t.hi, __fadd_rn(t.lo, __fadd_rn(ue, ve)));
-    };
-    const ff An = next(A, Ap), Bn = next(B, Bp);
-    D = __fmul_rn(D, an.hi);
-    // |h / h_before - 1| = |D| / |A_before B|
-    const float stop = fabsf(__fmul_rn(A.hi, Bn.hi)) * IGF_EPS;
-    Ap = A;
-    Bp = B;
-    A = An;
-    B = Bn;
-    if (fabsf(D) < stop * (1.f + IGF_TOL)) {
-      const ff r = ff_div(fast_two_sum(A.hi, A.lo), fast_two_sum(B.hi, B.lo));
-      *h = (double)r.hi + (double)r.lo;
-      return fabsf(D) < stop * (1.f - IGF_TOL);
-    }
-    if (fabsf(B.hi) > 1e6f) {  // by 1 / B's power of two
-      const float q = __int_as_float((254 - ((__float_as_int(B.hi) >> 23) & 0xff)) << 23);
-      auto scale = [&](ff &v) { v = ff_make(__fmul_rn(v.hi, q), __fmul_rn(v.lo, q)); };
-      scale(A);
-      scale(Ap);
-      scale(B);
-      scale(Bp);
-      D = __fmul_rn(D, __fmul_rn(q, q));
-    }
-  }
-  return false;
-}
-
 // The series and the fraction follow one another term by term, each at the
 // latency of FP64 operations (the pipe issues at 1/64 of the FP32 rate), and
 // a division is a dozen of them.  So the series divides once for four terms
 // and the fraction not at all: it runs on numerators and denominators,
 // h = A / B, and compares successive convergents crosswise.  Both stop at the
-// term where the reference does.
+// term where the reference does.  (In float-float from a = 32 on, 2^-46, a
+// genealogy update of 50 HKY loci x 32 chains took 1.24 ms where it takes 1.69,
+// 128 chains' split times 0.85 and 0.96; but the logarithm was then off by
+// 1.5e-14 on average and 4e-13 at most at a = 32 to 40, against 6e-15 and 3e-14.)
 struct IgBase {
   const double *lft;
   int st;
@@ -139,11 +52,6 @@ struct IgBase {
     if (x <= 0.0) {
       if (x < 0.0) st = IG_E_TERM;
       return 0.0;
-    }
-    double sf;
-    if (a >= IGF_AMIN && igf_series((float)a, x, &sf)) {
-      sf /= a;
-      return lg ? log(sf) + (-x + a * log(x) - (*gln)) : sf * exp(-x + a * log(x) - (*gln));
     }
     double ap = a, del = 1.0 / a, sum = del;
     static_assert(IG_ITMAX % 4 == 0, "four terms at a time");
@@ -167,9 +75,6 @@ struct IgBase {
   __device__ double gcf(double a, double x, double *gln, bool lg)
   {
     *gln = lf((int)a - 1);
-    double hf;
-    if (a >= IGF_AMIN && igf_fraction((float)a, x + 1.0 - a, &hf))
-      return lg ? (-x + a * log(x) - (*gln)) + log(hf) : exp(-x + a * log(x) - (*gln)) * hf;
     // convergents: A / B of this term and of the one before
     double b = x + 1.0 - a, A = 1.0, Am = 0.0, B = b, Bm = 1.0;
     int i;

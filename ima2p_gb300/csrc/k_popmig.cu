@@ -10,7 +10,8 @@
 // exponentials in fixed point, some 17 FP64 operations a term where the
 // logarithmic form took about 760 (GB300 issues 1.6 per cycle and SM).  The
 // terms popfast.cuh leaves out, and the exponential prior (k_popmig), take the
-// FP64 form below, written in the reference's operation order.
+// FP64 form below, written in the reference's operation order but for the
+// sums inside igamma.cuh.
 //
 // k_popmig_fast: a warp takes a block of 2^lognx points of one term and a
 // chunk of genealogies, 32 at a time staged in its shared memory by the warp's

@@ -34,6 +34,7 @@
 #include <algorithm>
 #include <cfloat>
 
+#include "ff.cuh"
 #include "igamma.cuh"
 
 namespace {

@@ -511,26 +511,22 @@ __global__ void __launch_bounds__(BS, MINB) k_hky_fast(Pools P, const ReqDev *re
     plane = splane;
   }
   if (tid == 0) {
-    // mu = u / (totsites standfactor): 2 kappa (pA pG + pC pT) + 2 (pA + pG)
-    // (pC + pT), in float-float (in FP64 one thread's fifty operations held up
-    // the CTA for some 3,000 cycles)
+    // mu = u / (totsites standfactor) in FP64, the standard factor as 2 kappa
+    // (pA pG + pC pT) + 2 (pA + pG) (pC + pT): its sum of twelve products held
+    // up the CTA for some 3,000 cycles
+    const double *pid = P.pi + 4 * (size_t)R.item;
+    const double p0 = pid[0], p1 = pid[1], p2 = pid[2], p3 = pid[3];
+    smu = ff_round(R.u / (2.0 * R.totsites * fma(R.par, fma(p0, p2, p1 * p3), (p0 + p2) * (p1 + p3))));
+  } else if (tid == 32) {
     const double *pid = P.pi + 4 * (size_t)R.item;
     ff pj[4];
     for (int j = 0; j < 4; j++) {
-      pj[j] = ff_split(pid[j]);
-      spi[j] = make_float2(pj[j].hi, pj[j].lo);
+      spi[j] = ff_round(pid[j]);
+      pj[j] = ff_of(spi[j]);
     }
-    const ff kap = ff_split(R.par);
-    ff sf = ff_mul(kap, ff_add(ff_mul(pj[0], pj[2]), ff_mul(pj[1], pj[3])));
-    sf = ff_add(sf, ff_mul(ff_add(pj[0], pj[2]), ff_add(pj[1], pj[3])));
-    const ff mu = ff_div(ff_split(R.u), ff_mul(ff_make(2.f * sf.hi, 2.f * sf.lo), ff_split((double)R.totsites)));
-    smu = make_float2(mu.hi, mu.lo);
-  } else if (tid == 32) {
-    const double *pid = P.pi + 4 * (size_t)R.item;
-    const ff PR = ff_add(ff_split(pid[0]), ff_split(pid[2])), PY = ff_add(ff_split(pid[1]), ff_split(pid[3]));
-    const ff kp = ff_add_f(ff_split(R.par), -1.0f), one = ff_from(1.0f);
+    skpa = ff_round(R.par - 1.0);
+    const ff PR = ff_add(pj[0], pj[2]), PY = ff_add(pj[1], pj[3]), kp = ff_of(skpa), one = ff_from(1.0f);
     auto put = [](ff v) { return make_float2(v.hi, v.lo); };
-    skpa = put(kp);
     sH.AR = put(ff_add_f(ff_mul(PR, kp), 1.0f));
     sH.AY = put(ff_add_f(ff_mul(PY, kp), 1.0f));
     sH.iR = put(ff_div(one, PR));

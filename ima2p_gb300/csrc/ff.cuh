@@ -167,46 +167,12 @@ __device__ __forceinline__ ff ff_horner(const float2 *c, int m, ff y)
 
 __device__ __forceinline__ double ff_to_double(ff a) { return (double)a.hi + (double)a.lo; }
 
-// ln 2 = LN2_A + LN2_B + LN2_C: LN2_A = 355/512 (9 significant bits, so k
-// LN2_A is exact for |k| < 2^15), LN2_B and LN2_C the next two float parts
-constexpr float LN2_A = 0.693359375f;
-constexpr float LN2_B = -2.121944417e-04f;
-constexpr float LN2_C = 1.646571768e-12f;
 // ln 2 as a normalised float-float pair
 constexpr float LN2_HI = 6.931471825e-01f;
 constexpr float LN2_LO = -1.904654212e-09f;
 
-// e^x and e^x - 1 for -86 < x < 88 in float-float.  x = k ln2 + r with
-// |r| <= ln2 / 2, y = expm1(r / 16) from its Taylor series (degree 7,
-// |r / 16| <= 0.022), four doublings expm1(2z) = expm1(z) (expm1(z) + 2),
-// then e^x = 2^k (1 + y) and e^x - 1 = y (k = 0) or 2^k (1 + y) - 1.  No
-// step cancels: e^x - 1 of a short branch keeps its relative accuracy
-// (about 1e-14).
-__device__ __forceinline__ void ff_exp_expm1(ff x, ff *ex, ff *em1)
-{
-  if (x.hi < -86.0f) {
-    *ex = ff_from(0.0f);
-    *em1 = ff_from(-1.0f);
-    return;
-  }
-  const float kf = rintf(x.hi * 1.44269504f);
-  ff r = ff_sub(x, ff_from(kf * LN2_A));
-  r = ff_sub(r, two_prod(kf, LN2_B));
-  r = ff_add_f(r, -kf * LN2_C);
-  const ff s = ff_make(r.hi * 0.0625f, r.lo * 0.0625f);
-  // the coefficients from 1/120 on in float (their terms weigh < 2e-9 of
-  // the sum), the rest in float-float
-  const float tail = __fmaf_rn(s.hi, __fmaf_rn(s.hi, 1.0f / 5040.0f, 1.0f / 720.0f), 1.0f / 120.0f);
-  ff u = ff_add(ff_make(0.041666668f, -1.2417635e-09f), ff_mul_f(s, tail));  // 1/24 + s tail
-  u = ff_add(ff_make(0.16666667f, -4.967054e-09f), ff_mul(s, u));          // 1/6 + s u
-  u = ff_add_f(ff_mul(s, u), 0.5f);
-  u = ff_add_f(ff_mul(s, u), 1.0f);
-  ff y = ff_mul(s, u);
-#pragma unroll
-  for (int i = 0; i < 4; i++) y = ff_mul(y, ff_add_f(y, 2.0f));
-  const int k = (int)kf;
-  const float p2 = __int_as_float((127 + k) << 23);  // 2^k, -125 <= k <= 127
-  const ff one_y = ff_add_f(y, 1.0f);
-  *ex = ff_make(one_y.hi * p2, one_y.lo * p2);
-  *em1 = (k == 0) ? y : ff_add_f(*ex, -1.0f);
-}
+// ln 2 / 64 = L64_A + L64_B + L64_C: the first two of 11 significant bits, so
+// k times them is exact for |k| < 2^13
+constexpr float L64_A = 0.01082611083984375f;
+constexpr float L64_B = 4.3101608753204346e-06f;
+constexpr float L64_C = 3.695530104153022e-09f;

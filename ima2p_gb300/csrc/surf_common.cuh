@@ -9,7 +9,7 @@
 #include "internal.h"
 
 constexpr int SURF_K = 30;          // exact terms: 2 (theta + migration parameters)
-constexpr int SURF_KP = 32;         // screened columns: the terms, the bias, zero padding
+constexpr int SURF_KP = 32;         // screened columns: the terms, the bias (tensor-core screen: in two), zero padding
 constexpr int SURF_MAX_CHUNKS = 64;
 constexpr float SURF_MARGIN = 32.0f;  // nats below the running max that still count
 constexpr int SURF_SEED = 256;      // genealogies sampled per point for the seed maximum (FP32 screen)
@@ -103,12 +103,6 @@ __device__ __forceinline__ ff surf_exact_row(const SurfPrep &S, int g, const flo
   }
   return fast_two_sum(sum, comp);
 }
-
-// ln 2 / 64 = L64_A + L64_B + L64_C: the first two of 11 significant bits, so
-// k times them is exact for |k| < 2^13
-constexpr float L64_A = 0.01082611083984375f;
-constexpr float L64_B = 4.3101608753204346e-06f;
-constexpr float L64_C = 3.695530104153022e-09f;
 
 // e^(dh + dl) for |dh| <= 86: d = k ln2 / 64 + r, |r| <= ln2 / 128, e^r from
 // its series (r and r^2/2 in float-float, r^3 .. r^5 in FP32), times tab[k &

@@ -90,6 +90,11 @@ void launch_is_sumlogk(const Pools &P, int item, int locus, int maxn, int maxS, 
                        cudaStream_t st);
 void launch_is(const Pools &P, const ReqDev *reqs, int nreq, int maxn, int maxS, double *result,
                int32_t *status, int32_t *site_node, cudaStream_t st);
+// Shared memory that a CTA can have.  A kernel whose need varies is allowed all
+// that its static part leaves, the same at every launch: the limit belongs to
+// the kernel, and a smaller one set by another context's thread between this
+// one's call and its launch would refuse the launch.
+constexpr int SMEM_MAX = 227 * 1024;
 // variant: launch shape, by the batch's size and work or by the autotuner
 constexpr int HKY_FAST_VARIANTS = 6;  // float-float: 128 threads with registers for 6 CTAs per SM, 64 threads
                                       // (16 CTAs), 256 (4), 128 at 10 CTAs, 128 at 8, 96 at 11;

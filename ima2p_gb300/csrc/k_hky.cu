@@ -1001,7 +1001,7 @@ static void hky_fast_launch(const Pools &P, const ReqDev *reqs, int nreq, int ma
   const size_t tcap = UNI ? std::min(HKY_TASK_CAP, (maxn - 1) * (maxS + 4)) : 0;
   const size_t sm = hky_layout_fast(maxnl, UNI, FF).total + 4 * (mcap + pcap) + 2 * ((mcap + 1) & ~size_t(1)) + tcap * sizeof(uint2);
   if (sm > 40 * 1024)  // (48 KB with the static part)
-    cudaFuncSetAttribute(k_hky_fast<UNI, FF, BS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_hky_fast<UNI, FF, BS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024);
   k_hky_fast<UNI, FF, BS, MINB><<<nreq, BS, sm, st>>>(P, reqs, result, status, maxnl, (int)mcap, (int)pcap, (int)tcap);
 }
 
@@ -1093,7 +1093,7 @@ void launch_hky_fp64(const Pools &P, const ReqDev *reqs, int nreq, int maxn, dou
   if (nreq <= 0) return;
   size_t sm = hky_layout64(2 * maxn - 1).total;
   if (sm > 48 * 1024)
-    cudaFuncSetAttribute(k_hky_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_hky_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 128);
   k_hky_fp64<<<nreq, HKY_BS, sm, st>>>(P, reqs, result, status, 2 * maxn - 1);
 }
 

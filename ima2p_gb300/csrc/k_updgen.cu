@@ -839,8 +839,8 @@ void launch_ug_propose(const UgArgs &a, cudaStream_t st)
 {
   const size_t bytes = UG_RNG_SMEM + a.k * ug_locus_smem(a.maxn);
   cudaFuncSetAttribute(k_ug_propose, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  if (bytes > 36 * 1024)
-    cudaFuncSetAttribute(k_ug_propose, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (bytes > 36 * 1024)  // (48 KB with the static part)
+    cudaFuncSetAttribute(k_ug_propose, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 12 * 1024);
   k_ug_propose<<<a.nch, 32 * (a.k + UG_RNG_WARPS), bytes, st>>>(a);
 }
 

@@ -20,13 +20,16 @@
 // issues about 1.6 FP64 operations or conversions per cycle and SM: the
 // former kernel (conversions, six operations and an FP64 exponential per
 // term) spent 20 cycles a term, 83.5 ms for 13,000 points x 100,000
-// genealogies; now 6.8 ms, 5.2 of them the two FMAs of each term.  Adding the
-// doubles instead (a third FP64 operation) measured 14.6 ms against 11.9 for
+// genealogies; now 6.9 ms, 5.2 of them the two FMAs of each term.  (6.8 while
+// the products with log2 e were left rounded: on the rows of a run the
+// densities were off by 3.2e-16 to 4.2e-16 of their mean from an FP64
+// evaluation, now by 1.4e-16, with FP64 exponentials by 2.0e-16 to 2.8e-16.)
+// Adding the doubles instead (a third FP64 operation) measured 14.6 ms against 11.9 for
 // the integer sums before the last two steps (integer compare, shorter tail).
 //
 // Threads: `nx` requests by MG_BS / nx genealogy strides, nx the power of two
 // that holds the largest parameter's requests, so a search's few points
-// still use every lane.  Partial sums per chunk are added in chunk order by
+// still use every lane.  Partial sums per chunk are added in a fixed order by
 // the merge kernel.
 #include <cfloat>
 #include <cmath>
@@ -39,7 +42,8 @@ namespace {
 constexpr int MG_BS = 128;  // threads per CTA
 constexpr int MG_TG = 128;  // genealogies per shared-memory tile
 constexpr double LOG2 = 0.69314718055994530942;
-constexpr double LOG2E = 1.4426950408889634074;
+constexpr double LOG2E = 1.4426950408889634074, LOG2E_LO = 2.0355273740931033e-17;  // log2 e, and the rest of it
+constexpr double FX_ONE = 9007199254740992.0;  // 2^53: fx_fix's fraction bits
 constexpr int FX_LIMIT_HI = 0x408f4000;  // high word of 1000.0, the bound of the fixed-point form's argument
 
 __constant__ uint64_t c_fxtab[FX_TAB];
@@ -54,6 +58,7 @@ __global__ void __launch_bounds__(MG_BS) k_margin(MarginArgs a, int lognx, int c
 {
   __shared__ uint64_t tab[FX_TAB];
   __shared__ double sc[MG_TG], sf[MG_TG], sb[MG_TG];
+  __shared__ float4 sl[MG_TG];  // c and f in FP32, and what the rounding of base leaves (2^-53)
   const int tid = threadIdx.x, nx = 1 << lognx;
   const int k = blockIdx.x * nx + (tid & (nx - 1));  // this thread's request
   const int sub = tid >> lognx, nsub = MG_BS >> lognx;
@@ -61,9 +66,14 @@ __global__ void __launch_bounds__(MG_BS) k_margin(MarginArgs a, int lognx, int c
   const int pi = a.param[blockIdx.x * nx];
   const double x = a.x[k];
   const bool theta = pi < a.np;
-  // the term's coefficients in units of ln 2
-  const double A = (theta ? LOG2 - log(x) : log(x)) * LOG2E;
-  const double B = (theta ? 1.0 / x : x) * LOG2E;
+  // The term's coefficients, as the reference rounds them, in units of ln 2;
+  // and in units of 2^-53 what that product's rounding leaves.  (That is the
+  // same for every genealogy, or of base for every x, and where few
+  // genealogies make the sum neither averages out.)
+  const double a_ = theta ? LOG2 - log(x) : log(x), b_ = theta ? 1.0 / x : x;
+  const double A = a_ * LOG2E, B = b_ * LOG2E;
+  const float Al = (float)((__fma_rn(a_, LOG2E, -A) + a_ * LOG2E_LO) * FX_ONE);
+  const float Bl = (float)((__fma_rn(b_, LOG2E, -B) + b_ * LOG2E_LO) * FX_ONE);
   double cst = 0.0;
   if (EXPO && !theta) {
     const double meani = 1.0 / a.expo_mean[pi - a.np];
@@ -84,16 +94,20 @@ __global__ void __launch_bounds__(MG_BS) k_margin(MarginArgs a, int lognx, int c
       const float r0 = r[c0], r1 = r[c1], r2 = r[c2], r3 = r[c3];
       sc[tid] = theta && a.raw_cc ? (double)r1 : intround(r1);
       sf[tid] = theta ? -2.0 * (double)r3 : -(double)r2;
-      sb[tid] = theta ? (-(double)r0 - (double)r2) * LOG2E : -(double)r0 * LOG2E;
+      const double base = theta ? -(double)r0 - (double)r2 : -(double)r0;
+      sb[tid] = base * LOG2E;
+      sl[tid] = make_float4((float)sc[tid], (float)sf[tid],
+                            (float)((__fma_rn(base, LOG2E, -sb[tid]) + base * LOG2E_LO) * FX_ONE), 0.f);
     }
     __syncthreads();
     for (int j = sub; j < nt; j += nsub) {
-      double v = __fma_rn(sc[j], A, __fma_rn(sf[j], B, sb[j]));
+      double v = __fma_rn(sf[j], B, __fma_rn(sc[j], A, sb[j]));
       if (EXPO) v += cst;
       // |v| < 1000, compared as bits: a DSETP would be a third FP64 operation
       if ((__double2hiint(v) & 0x7fffffff) < FX_LIMIT_HI) {
         int i;
-        const uint64_t m = fx_exp2(fx_fix(v), tab, &i);
+        const float4 l = sl[j];
+        const uint64_t m = fx_exp2(fx_fix(v) + __float2int_rn(__fmaf_rn(l.x, Al, __fmaf_rn(l.y, Bl, l.z))), tab, &i);
         sum.add(m, i);
       } else {  // beyond it, infinite or NaN
         sum.total += exp2(v);
@@ -107,22 +121,27 @@ __global__ void __launch_bounds__(MG_BS) k_margin(MarginArgs a, int lognx, int c
   }
   sum.flush();
   double s = sum.total;
-  if (nsub > 1) {  // the strides of a request, in order
+  if (nsub > 1) {  // the strides of a request, pairwise
     __shared__ double red[MG_BS];
     red[tid] = s;
-    __syncthreads();
-    if (sub == 0)
-      for (int w = 1; w < nsub; w++) s += red[(w << lognx) + tid];
+    for (int o = nsub >> 1; o; o >>= 1) {
+      __syncthreads();
+      if (sub < o) red[tid] = s += red[tid + (o << lognx)];
+    }
   }
   if (sub == 0) part[(size_t)k * gridDim.y + blockIdx.y] = s;
 }
 
-__global__ void k_margin_merge(MarginArgs a, int nchunks, const double *part, double *out)
+// a warp per request: its chunks by lane, then the lanes pairwise (fewer
+// roundings follow one another than chunk by chunk)
+__global__ void __launch_bounds__(128) k_margin_merge(MarginArgs a, int nchunks, const double *part, double *out)
 {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int k = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (k >= a.n) return;
   double s = 0.0;
-  for (int c = 0; c < nchunks; c++) s += part[(size_t)k * nchunks + c];
+  for (int c = lane; c < nchunks; c += 32) s += part[(size_t)k * nchunks + c];
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane) return;
   s /= a.div;
   if (a.logi) s = (s <= 0.0) ? -1e200 : log(s);  // LOWLOG
   out[k] = s - a.yadjust;
@@ -170,6 +189,6 @@ int launch_margin(const MarginArgs &a, int lognx, double *part, int nchunks, dou
   const dim3 grid(a.n >> lognx, nchunks);
   if (a.expo_mean) k_margin<true><<<grid, MG_BS, 0, st>>>(a, lognx, chunk, part);
   else k_margin<false><<<grid, MG_BS, 0, st>>>(a, lognx, chunk, part);
-  k_margin_merge<<<(a.n + 127) / 128, 128, 0, st>>>(a, nchunks, part, out);
+  k_margin_merge<<<(a.n + 3) / 4, 128, 0, st>>>(a, nchunks, part, out);
   return 0;
 }

@@ -75,9 +75,11 @@ __global__ void __launch_bounds__(MG_BS) k_margin(MarginArgs a, int lognx, int c
   const float Al = (float)((__fma_rn(a_, LOG2E, -A) + a_ * LOG2E_LO) * FX_ONE);
   const float Bl = (float)((__fma_rn(b_, LOG2E, -B) + b_ * LOG2E_LO) * FX_ONE);
   double cst = 0.0;
+  float cl = 0.f;
   if (EXPO && !theta) {
-    const double meani = 1.0 / a.expo_mean[pi - a.np];
-    cst = (log(meani) - x * meani) * LOG2E;
+    const double meani = 1.0 / a.expo_mean[pi - a.np], c_ = log(meani) - x * meani;
+    cst = c_ * LOG2E;
+    cl = (float)((__fma_rn(c_, LOG2E, -cst) + c_ * LOG2E_LO) * FX_ONE);
   }
   const int p = pi - a.np;  // columns: (qi, cc, hcc, fc) or (mi, mc, fm)
   const int c0 = theta ? a.qip + pi : a.mip + p, c1 = theta ? a.ccp + pi : a.mcp + p,
@@ -107,7 +109,7 @@ __global__ void __launch_bounds__(MG_BS) k_margin(MarginArgs a, int lognx, int c
       if ((__double2hiint(v) & 0x7fffffff) < FX_LIMIT_HI) {
         int i;
         const float4 l = sl[j];
-        const uint64_t m = fx_exp2(fx_fix(v) + __float2int_rn(__fmaf_rn(l.x, Al, __fmaf_rn(l.y, Bl, l.z))), tab, &i);
+        const uint64_t m = fx_exp2(fx_fix(v) + __float2int_rn(__fmaf_rn(l.x, Al, __fmaf_rn(l.y, Bl, EXPO ? l.z + cl : l.z))), tab, &i);
         sum.add(m, i);
       } else {  // beyond it, infinite or NaN
         sum.total += exp2(v);

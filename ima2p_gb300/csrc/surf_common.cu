@@ -130,7 +130,7 @@ constexpr float TC_ACC_ERR = 2e-5f;
 // phi(x) of every point, a warp per two points: half a warp for the
 // parameters of each (FP64 logarithms and reciprocals), then a lane per
 // column of one and of the other; terms outside the model type get
-// coefficient 0.  Then, a lane per genealogy, the exact maximum over nseed
+// coefficient 0.  Then, a lane per genealogy, the exact maximum over nseed <= 32
 // evenly spaced ones, the starting value of the maximum shared by chunks.
 __global__ void __launch_bounds__(256) k_prep_points(SurfArgs a, SurfPrep S, int npad, int nseed, SurfZero z)
 {
@@ -208,6 +208,31 @@ __global__ void __launch_bounds__(256) k_prep_points(SurfArgs a, SurfPrep S, int
         S.xmax[p] = f2ord(best);
       }
     }
+  }
+}
+
+// the same maximum from more genealogies than a lane each, a warp per point
+// (256 of them by the kernel above, two points a warp, took 190 us more for
+// 16,384 points)
+__global__ void __launch_bounds__(256) k_surf_seed(SurfPrep S, int npoints, int nseed)
+{
+  const int p = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (p >= npoints) return;  // warp-uniform
+  float2 phi[SURF_K];
+#pragma unroll
+  for (int k = 0; k < SURF_K; k++) phi[k] = S.phiff[(size_t)p * SURF_K + k];
+  float best = -INFINITY;
+  const int n = min(nseed, S.G);
+  for (int i = lane; i < n; i += 32) {
+    const int g = (int)(((long long)i * S.G) / n);
+    best = fmaxf(best, surf_exact(S, g, S.sT + g, S.Gpad, phi).hi);
+  }
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+  if (lane == 0) {
+    S.seed[p] = best;
+    S.best[p] = f2ord(best);
+    S.xmax[p] = f2ord(best);
   }
 }
 
@@ -304,7 +329,11 @@ int surf_prep(const SurfArgs &a, SurfPrep &S, bool tc, bool rows_ready, int nsee
     }
   }
   const int npad = (a.npoints + 255) / 256 * 256;
-  k_prep_points<<<npad / 16, 256, 0, st>>>(a, S, npad, nseed, z);
+  k_prep_points<<<npad / 16, 256, 0, st>>>(a, S, npad, nseed > 32 ? 0 : nseed, z);
+  if (nseed > 32) {
+    k_surf_seed<<<(a.npoints + 7) / 8, 256, 0, st>>>(S, a.npoints, nseed);
+    nk++;
+  }
   return nk;
 }
 

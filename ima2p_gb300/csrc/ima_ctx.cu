@@ -1564,7 +1564,8 @@ static int build_batch(ima_ctx *c, Batch &b, int n, const int32_t *ci, const int
   b.nhky = (int)g[1].size();
   b.nsw = (int)g[2].size();
   // Launch shape of the fast HKY forms, for what a chain-locus's CTA has to do
-  // (partials of a full evaluation; of edited edges a quarter):
+  // (partials of a full evaluation; of edited edges half as many, for the
+  // masks and the list are made of all):
   //  - 256 threads where one wave of such CTAs holds the launch (4 per SM,
   //    FP32 6) and there is work for them: 64 chain-loci of 40 genes x 60
   //    patterns 18 us and 19, x 100 19 and 20, x 150 25 and 22; of 100 genes x
@@ -1585,7 +1586,7 @@ static int build_batch(ima_ctx *c, Batch &b, int n, const int32_t *ci, const int
       most = std::max(most, q.n);
       plain |= !q.uni;
     }
-    work /= std::max(1, b.nhky) * (edits || partial ? 4.0 : 1.0);
+    work /= std::max(1, b.nhky) * (edits || partial ? 2.0 : 1.0);
     b.hky_variant = 0;
     if (most <= (prec == IMA_PREC_FP32 ? 6 : 4) * c->nsm && (plain || work >= 4000.0)) b.hky_variant = 2;
     else if (prec == IMA_PREC_FAST && plain) b.hky_variant = 4;

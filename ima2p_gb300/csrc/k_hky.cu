@@ -990,6 +990,8 @@ __global__ void k_hky_commit(Pools P, const int32_t *items, const uint8_t *accep
 }  // namespace
 
 constexpr size_t HKY_TASK_CAP = 640, HKY_PLANE_CAP = 1024;  // tasks and words kept in shared memory
+constexpr int HKY_FEW = 4 * 152;
+constexpr size_t HKY_FEW_SMEM = 56 * 1024;  // so that four CTAs fit an SM
 
 template <bool UNI, bool FF, int BS, int MINB>
 static void hky_fast_launch(const Pools &P, const ReqDev *reqs, int nreq, int maxnl, int maxS, double *result,
@@ -997,9 +999,12 @@ static void hky_fast_launch(const Pools &P, const ReqDev *reqs, int nreq, int ma
 {
   const size_t maxn = (size_t)(maxnl + 1) / 2, W = ((size_t)maxS + 31) / 32;
   const size_t mcap = UNI ? std::min((size_t)HKY_MASK_WORDS, (maxn - 1) * W) : 0;
-  const size_t pcap = UNI ? std::min(HKY_PLANE_CAP, 2 * maxn * W) : 0;
   const size_t tcap = UNI ? std::min(HKY_TASK_CAP, (maxn - 1) * (maxS + 4)) : 0;
-  const size_t sm = hky_layout_fast(maxnl, UNI, FF).total + 4 * (mcap + pcap) + 2 * ((mcap + 1) & ~size_t(1)) + tcap * sizeof(uint2);
+  const size_t base = hky_layout_fast(maxnl, UNI, FF).total + 4 * mcap + 2 * ((mcap + 1) & ~size_t(1)) + tcap * sizeof(uint2);
+  // few CTAs take all of the tips' planes, which one warp reads for the masks
+  const size_t planes = UNI ? 2 * maxn * W : 0;
+  const size_t pcap = nreq <= HKY_FEW && base + 4 * planes <= HKY_FEW_SMEM ? planes : std::min(HKY_PLANE_CAP, planes);
+  const size_t sm = base + 4 * pcap;
   if (sm > 40 * 1024)  // (48 KB with the static part)
     cudaFuncSetAttribute(k_hky_fast<UNI, FF, BS, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 1024);
   k_hky_fast<UNI, FF, BS, MINB><<<nreq, BS, sm, st>>>(P, reqs, result, status, maxnl, (int)mcap, (int)pcap, (int)tcap);

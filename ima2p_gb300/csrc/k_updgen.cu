@@ -34,9 +34,10 @@
 // launch per locus a decision took 43 us (an incomplete gamma function a
 // lane, 10 to 20 us, and chains of dependent loads) and a proposal 26, 50 us
 // a step with the launches.  Measured (2 sweeps of 50 HKY loci x 32 chains /
-// 100 stepwise ones x 64): 5.0 -> 1.1 ms and 10.1 -> 2.4 ms, of which 0.7 and
-// 1.2 ms are set-up; after 400 such calls, when the heated chains have lengths
-// that need the gamma functions' series, 1.3 and 3.9 ms.  A proposal and a
+// 100 stepwise ones x 64): 5.3 -> 1.5 (1.0 some calls on) and 10.0 -> 2.3
+// ms, of which 0.7 and 1.2 ms are set-up; after 300 such calls, when the heated
+// chains have lengths that need the gamma functions' series, 6.5 -> 1.6 and
+// 21.4 -> 5.6 ms.  A proposal and a
 // decision of a launch take 25 to 35 us each, whatever its number of loci.
 // The file is compiled with -fmad=false: the reference's adds and
 // multiplies round as written; log, exp and sqrt are the device's.
